@@ -252,28 +252,27 @@ unsigned long long *bad_counter(dream_das_plan *p) {
 int launch_plain(dream_das_plan *p, PlainLaunch &L, cudaStream_t st) {
   L.ny = p->K * num_columns(p);
   L.bad = bad_counter(p);
-  // 2-D warp patches for RCA volumes with a grid hint (das_uni: its own
-  // grid). On the 128x128-element RCA volume (128x128x256 points) they take
-  // plain FP32 from 194.8 to 180.7 ms; on the 64x64-element TFM frame
-  // (512x512 points) they cost 4 % (FP64 2.43 -> 2.52 ms), so TFM and SAFT
-  // keep warps of consecutive points.
+  // TFM and RCA images on a grid (the plan's hint, or das_uni's own grid) are
+  // cut into 2-D tiles, unless the grid is so narrow that most of their points
+  // would lie outside it.
   L.n_fast = 0;
-  if (L.method == DREAM_DAS_RCA_COLTX || L.method == DREAM_DAS_RCA_ROWTX) {
-    if (L.uni) {
-      const int64_t nf = L.Ny > 1 ? L.Ny : L.Ny * L.Nz;
-      if (nf >= 8 && L.No % nf == 0 && nf < L.No) L.n_fast = nf;
-    } else if (p->n_fast >= 8 && p->n_fast < L.No) {
-      L.n_fast = p->n_fast;
-    }
+  const int bd = L.method == DREAM_DAS_SAFT ? 0 : plain_tile_threads(L.method == DREAM_DAS_RCA_ROWTX ? L.Nt : L.Nr,
+                                                                      p->precision == DREAM_PREC_F64 ? 8 : 4);
+  const int64_t nf = L.uni ? (L.Ny > 1 ? L.Ny : L.Ny * L.Nz) : p->n_fast;
+  int64_t rows = 0;
+  if (bd > 0 && nf > 0 && nf < L.No && L.No % nf == 0) {
+    const int64_t tf = plain_tile_f(L.method, bd), ts = plain_tile_s(L.method, bd);
+    rows = (L.No / nf + ts - 1) / ts;
+    if ((nf + tf - 1) / tf * tf * rows * ts <= 2 * L.No) L.n_fast = nf;
   }
   // Pixel chunks keep a cancellation request observable between launches.
   const int64_t tpp = std::max<int64_t>(terms_per_pixel(p), 1);
   int64_t chunk = std::max<int64_t>(int64_t(1) << 16, (int64_t(1) << 33) / tpp);
   chunk = (chunk + 255) / 256 * 256;
   int64_t total = L.No;
-  if (L.n_fast > 0) {  // the range is over rows of warp patches (at most 65535 per launch: the grid's y extent)
-    total = (L.No / L.n_fast + PLAIN_PATCH_S - 1) / PLAIN_PATCH_S;
-    chunk = std::min<int64_t>(65535, std::max<int64_t>(1, chunk / (PLAIN_PATCH_S * L.n_fast)));
+  if (L.n_fast > 0) {  // the range is over rows of tiles (at most 65535 per launch: the grid's y extent)
+    total = rows;
+    chunk = std::min<int64_t>(65535, std::max<int64_t>(1, chunk / (plain_tile_s(L.method, bd) * L.n_fast)));
   }
   for (int64_t s = 0; s < total; s += chunk) {
     if (p->cancelled.load()) return fail(DREAM_ERR_CANCELLED, "DAS cancelled");

@@ -18,10 +18,34 @@ struct Consts32 {
   float Fs, ocp, delay_ms;
 };
 
-// Warp patch of the plain kernels under a grid hint: PLAIN_PATCH_F points
-// along the grid's fast axis x (32 / PLAIN_PATCH_F) along the slow one.
-constexpr int PLAIN_PATCH_F = 8;
-constexpr int PLAIN_PATCH_S = 32 / PLAIN_PATCH_F;
+// Warp patch of the plain TFM / RCA kernel on a hinted grid: points along the
+// fast axis (depth, on the usual grids), the rest of the 32 along the slow one.
+// The fewer different samples a patch reads from one A-scan, the fewer
+// wavefronts its gather takes: in depth a point moves by the sum of both legs'
+// cosines, across by sines of opposite signs, so TFM patches are 4 deep and 8
+// wide (64x64 elements, 512x512 points, FP64: 0.69 ms; 8 x 4: 0.80). Both
+// sideways axes of an RCA volume move its legs alike: 8 x 4 (128x128 elements,
+// 131072 points, FP64 3.1 ms; 4 x 8: 3.6, 2 x 16: 4.9).
+constexpr int plain_patch_f(int method) { return method == 1 /* TFM */ ? 4 : 8; }
+
+// Terms whose gathers are issued together.
+constexpr int PLAIN_U = 16;
+
+// Leg table of a block of the plain TFM / RCA kernel: n_in legs per thread, in
+// whole pairs of gather groups.
+constexpr size_t plain_table_bytes(int64_t n_in, size_t elem, int threads) {
+  return (size_t)((n_in + 2 * PLAIN_U - 1) / (2 * PLAIN_U) * (2 * PLAIN_U)) * elem * threads;
+}
+// Threads per block: the largest block whose table leaves room for three on
+// an SM; a table that does not fit one warp in shared memory: 0 (no table).
+constexpr int plain_tile_threads(int64_t n_in, size_t elem) {
+  int bd = 128;
+  while (bd > 32 && plain_table_bytes(n_in, elem, bd) > 72 * 1024) bd >>= 1;
+  return plain_table_bytes(n_in, elem, bd) <= 200 * 1024 ? bd : 0;
+}
+// Tile of image points of such a block on a hinted grid.
+constexpr int plain_tile_f(int method, int threads) { return (threads >= 128 ? 2 : 1) * plain_patch_f(method); }
+constexpr int plain_tile_s(int method, int threads) { return threads / plain_tile_f(method, threads); }
 
 struct PlainLaunch {
   int method;  // 0 SAFT, 1 TFM, 2 RCA col-tx, 3 RCA row-tx
@@ -30,7 +54,7 @@ struct PlainLaunch {
   int64_t K;
   const void *Ro;
   int64_t No;
-  int64_t no0, no1;  // pixel range of this launch (patch-row range when n_fast > 0)
+  int64_t no0, no1;  // pixel range of this launch (tile-row range when n_fast > 0)
   int64_t n_fast;    // grid hint: points along the grid's fast axis (0: none)
   const void *Gt;
   int64_t Nt;

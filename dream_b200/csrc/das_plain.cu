@@ -9,16 +9,16 @@
 //   RCA row-tx  extra_src/das.cc:533-626, opencl/das_uni_double.cl:283-394
 // Each thread owns one image point and sums its terms in the reference order
 // (outer element loop, inner element loop), so the image is bit-identical to
-// the reference CPU code, not merely close to it. With a grid hint the warps
-// take 8 x 4 patches of the image grid (PLAIN_PATCH_F x PLAIN_PATCH_S) instead
-// of 32 consecutive points, which changes only which thread owns which point.
+// the reference CPU code, not merely close to it. With a grid hint TFM and RCA
+// blocks take 2-D tiles of the image grid instead of consecutive points, which
+// changes only which thread owns which point.
 //
 // What differs from the reference is where the work goes. The inner-loop
 // element leg (receive leg for TFM/col-tx, column leg for row-tx) depends
 // only on (pixel, inner element), so it is computed once per pixel into a
-// per-thread shared-memory table instead of once per term; every term then
-// costs one add, one multiply, the bounds test, the truncation and one
-// gather from Y. Hoisting is exact: the leg is the same rounded value.
+// per-thread shared-memory table instead of once per term. Hoisting is exact:
+// the leg is the same rounded value. So is the bounds test: rounding is
+// monotone, so the extreme legs decide it for all terms of an outer element.
 #include "das_common.cuh"
 #include "das_kernels.h"
 
@@ -34,7 +34,7 @@ struct PlainParams {
   int Nt;
   const T *Gr;
   int Nr;
-  int64_t no0, no1;  // pixel range [no0, no1) of this launch, or patch-row range when n_fast > 0
+  int64_t no0, no1;  // pixel range [no0, no1) of this launch, or tile-row range when n_fast > 0
   int64_t n_fast, n_slow;  // grid hint: warps take patches of (fast, slow) points
   const T *delay;  // das: device delays in us (1 value, or No when delay_multi)
   int delay_multi;
@@ -45,7 +45,7 @@ struct PlainParams {
   int64_t ny;               // elements in Y (bounds-checked builds)
   unsigned long long *bad;  // gather index violations (bounds-checked builds)
   int64_t *idx;             // index mode: idx[col * No + no] = sample index or -1
-  int bigk;  // K >= 2^22 (FP32): use the conversion unit for truncation
+  int bigk;  // K >= 2^22 (FP32: truncation needs the conversion unit) or 2^28 (FP64): no grouped sample numbers
   // uniform grids
   T tri[15];
   int64_t Nx, Ny, Nz;
@@ -55,7 +55,7 @@ struct PlainParams {
 // conversion unit; every other case uses the exact add-based form.
 template <class T, bool BIGK>
 __device__ __forceinline__ int to_index(T p) {
-  if (BIGK) return __float2int_rz((float)p);
+  if constexpr (BIGK && sizeof(T) == 4) return __float2int_rz(p);
   return trunc_index(p);
 }
 
@@ -66,74 +66,79 @@ __device__ __forceinline__ float delay_to_ms(float d) {
   return __double2float_rn((double)d / 1000.0);
 }
 
-constexpr int UNROLL = 8;  // gathers in flight per thread before their in-order adds
-
 // Sample ycol[off] of Y. The bounds-checked build tests the element index
 // against the extent of Y first (a violation is counted and reads 0); the
 // normal build is the plain load.
-// FP64 addresses the sample from the base of Y with a 64-bit element index,
-// FP32 from the column pointer: on a 64x64-element TFM frame (K 3000, 512x512
-// points) each form is the faster one for its type (FP64 2.46 vs 2.86 ms,
-// FP32 1.19 vs 1.36 ms).
 template <class T>
 __device__ __forceinline__ T load_y(const PlainParams<T> &P, const T *ycol, int64_t off) {
 #ifdef DREAM_DAS_CHECKED
   const int64_t gi = (ycol - P.Y) + off;
   return gather_ok<T>(gi, P.ny, P.bad) ? __ldg(P.Y + gi) : (T)0;
 #else
-  if constexpr (sizeof(T) == 8) return __ldg(P.Y + ((ycol - P.Y) + off));
-  else return __ldg(ycol + off);
+  return __ldg(ycol + off);
 #endif
 }
 
-// IDX: instead of gathering and summing, write every term's sample index
-// (the one the gather would read; -1 for an out-of-bounds term) to P.idx.
-// PATCH: warps take 2-D patches of the grid (P.n_fast > 0); a template
-// parameter, so the consecutive-point kernel compiles as if it did not exist.
-template <class T, int M, bool UNI, bool TAB, bool BIGK, bool IDX = false, bool PATCH = false>
-__global__ void __launch_bounds__(256) das_plain_kernel(const PlainParams<T> P) {
+// The sample k places after y, for a 32-bit k.
+template <class T>
+__device__ __forceinline__ T load_at(const PlainParams<T> &P, const T *y, uint32_t k) {
+  const T *a;  // one multiply-add of the 32-bit number: as y + k it takes two more instructions
+  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(a) : "r"(k), "n"((int)sizeof(T)), "l"(y));
+  return gather_ok<T>((y - P.Y) + k, P.ny, P.bad) ? __ldg(a) : (T)0;
+}
+
+// The image point of one thread and its legs, for method M on arbitrary
+// (UNI = false) or uniform geometry. TFM: outer = transmit, inner = receive;
+// col-tx: columns, rows; row-tx: rows, columns.
+template <class T, int M, bool UNI>
+struct PlainPoint {
   using A = Ar<T>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *tab = reinterpret_cast<T *>(smem_raw);
-  const int tid = threadIdx.x;
-  const int bd = blockDim.x;
-  int64_t no_raw;
-  bool active;
-  if constexpr (PATCH) {
-    // 2-D patches: warp w of block (x, y) covers PLAIN_PATCH_F points along
-    // the grid's fast axis (patch x * warps + w) x PLAIN_PATCH_S along the
-    // slow one (patch row no0 + y)
-    const int lane = tid & 31;
-    const int64_t f = ((int64_t)blockIdx.x * (bd >> 5) + (tid >> 5)) * PLAIN_PATCH_F + lane % PLAIN_PATCH_F;
-    const int64_t s = (P.no0 + blockIdx.y) * PLAIN_PATCH_S + lane / PLAIN_PATCH_F;
-    active = f < P.n_fast && s < P.n_slow;
-    no_raw = s * P.n_fast + f;
-  } else {
-    no_raw = P.no0 + (int64_t)blockIdx.x * bd + tid;
-    active = no_raw < P.no1;
-  }
-  const int64_t no = active ? no_raw : (PATCH ? 0 : P.no0);  // inactive lanes read a valid point and write nothing
+  T xo, yo, zo, delay_ms, gy_c, gx_r;
 
-  // ---- image point ----
-  T xo, yo, zo;
-  if (UNI) {
-    // linear index -> (ny fastest, nz, nx)   (opencl/das_uni_double.cl:32-43)
-    int64_t yq = no / P.Ny, ny = no - yq * P.Ny;
-    int64_t zq = yq / P.Nz, nz = yq - zq * P.Nz;
-    int64_t xq = zq / P.Nx, nx = zq - xq * P.Nx;
-    xo = A::add(P.tri[6], A::mul((T)nx, P.tri[7]));
-    yo = A::add(P.tri[9], A::mul((T)ny, P.tri[10]));
-    zo = A::add(P.tri[12], A::mul((T)nz, P.tri[13]));
-  } else {
-    xo = P.Ro[no];
-    yo = P.Ro[no + P.No];
-    zo = P.Ro[no + 2 * P.No];
+  __device__ __forceinline__ void init(const PlainParams<T> &P, int64_t no) {
+    if (UNI) {
+      // linear index -> (ny fastest, nz, nx)   (opencl/das_uni_double.cl:32-43)
+      int64_t yq = no / P.Ny, ny = no - yq * P.Ny;
+      int64_t zq = yq / P.Nz, nz = yq - zq * P.Nz;
+      int64_t xq = zq / P.Nx, nx = zq - xq * P.Nx;
+      xo = A::add(P.tri[6], A::mul((T)nx, P.tri[7]));
+      yo = A::add(P.tri[9], A::mul((T)ny, P.tri[10]));
+      zo = A::add(P.tri[12], A::mul((T)nz, P.tri[13]));
+    } else {
+      xo = P.Ro[no];
+      yo = P.Ro[no + P.No];
+      zo = P.Ro[no + 2 * P.No];
+    }
+    delay_ms = UNI ? P.delay_ms : delay_to_ms(P.delay[P.delay_multi ? no : 0]);
+    // RCA stripe clamps (extra_src/das.cc:464-467,475-486,493-503)
+    gy_c = (T)0;
+    gx_r = (T)0;
+    if (M == RCA_COLTX || M == RCA_ROWTX) {
+      T gc_y_min, gc_y_max, gr_x_min, gr_x_max;
+      if (UNI) {  // opencl/das_uni_double.cl:213-216
+        gc_y_min = P.tri[3]; gc_y_max = P.tri[5];
+        gr_x_min = P.tri[0]; gr_x_max = P.tri[2];
+      } else {  // literal (num_cols/num_rows mixed) reads of the reference
+        gc_y_min = P.Gr[0 + 1 * P.Nt];
+        gc_y_max = P.Gr[P.Nt - 1 + 1 * P.Nt];
+        gr_x_min = P.Gt[0];
+        gr_x_max = P.Gt[P.Nr - 1];
+      }
+      if (yo >= gc_y_min && yo <= gc_y_max) gy_c = (T)0;
+      else if (yo < gc_y_min) gy_c = A::sub(gc_y_min, yo);
+      else gy_c = A::sub(gc_y_max, yo);
+      if (UNI) {
+        if (xo < gr_x_min || xo > gr_x_max) gx_r = (xo < gr_x_min) ? A::sub(gr_x_min, xo) : A::sub(gr_x_max, xo);
+      } else {
+        if (xo >= gr_x_min && xo <= gr_x_max) gx_r = (T)0;
+        else if (xo < gr_x_min) gx_r = A::sub(gr_x_min, xo);
+        else gx_r = A::sub(gr_x_max, xo);
+      }
+    }
   }
-  const T delay_ms = UNI ? P.delay_ms : delay_to_ms(P.delay[P.delay_multi ? no : 0]);
 
-  // ---- element coordinates ----
   // transmit / column elements
-  auto elem_t = [&](int n, T &ex, T &ey, T &ez) {
+  __device__ __forceinline__ void elem_t(const PlainParams<T> &P, int n, T &ex, T &ey, T &ez) const {
     if (UNI) {
       ex = A::add(P.tri[0], A::mul((T)n, P.tri[1]));
       ey = (T)0;
@@ -143,9 +148,9 @@ __global__ void __launch_bounds__(256) das_plain_kernel(const PlainParams<T> P) 
       ey = P.Gt[n + P.Nt];
       ez = P.Gt[n + 2 * P.Nt];
     }
-  };
+  }
   // receive / row elements (uniform RCA rows lie along y)
-  auto elem_r = [&](int n, T &ex, T &ey, T &ez) {
+  __device__ __forceinline__ void elem_r(const PlainParams<T> &P, int n, T &ex, T &ey, T &ez) const {
     if (UNI) {
       T c = A::add(P.tri[3], A::mul((T)n, P.tri[4]));
       if (M == RCA_COLTX || M == RCA_ROWTX) {
@@ -159,139 +164,261 @@ __global__ void __launch_bounds__(256) das_plain_kernel(const PlainParams<T> P) 
       ey = P.Gr[n + P.Nr];
       ez = P.Gr[n + 2 * P.Nr];
     }
-  };
+  }
+  // leg of a transmit (TFM, SAFT) or column (RCA) element, of a receive or row element
+  __device__ __forceinline__ T leg_t(const PlainParams<T> &P, int n) const {
+    T ex, ey, ez;
+    elem_t(P, n, ex, ey, ez);
+    return leg_time(A::sub(ex, xo), (M == TFM || M == SAFT) ? A::sub(ey, yo) : gy_c, A::sub(ez, zo), P.ocp);
+  }
+  __device__ __forceinline__ T leg_r(const PlainParams<T> &P, int n) const {
+    T ex, ey, ez;
+    elem_r(P, n, ex, ey, ez);
+    return leg_time((M == TFM || M == SAFT) ? A::sub(ex, xo) : gx_r, A::sub(ey, yo), A::sub(ez, zo), P.ocp);
+  }
+  // das row-tx: delay on the (inner) column leg; das_uni row-tx: on the
+  // (outer) row leg (opencl/das_uni_double.cl:358-360).
+  static constexpr bool DELAY_OUTER = (M != RCA_ROWTX) || UNI;
+  __device__ __forceinline__ T outer_leg(const PlainParams<T> &P, int o) const {
+    const T l = (M == RCA_ROWTX) ? leg_r(P, o) : leg_t(P, o);
+    return DELAY_OUTER ? A::add(l, delay_ms) : l;
+  }
+  __device__ __forceinline__ T inner_leg(const PlainParams<T> &P, int i) const {
+    const T l = (M == RCA_ROWTX) ? leg_t(P, i) : leg_r(P, i);
+    return DELAY_OUTER ? l : A::add(l, delay_ms);
+  }
+};
 
-  // ---- RCA stripe clamps (extra_src/das.cc:464-467,475-486,493-503) ----
-  T gy_c = (T)0, gx_r = (T)0;
-  if (M == RCA_COLTX || M == RCA_ROWTX) {
-    T gc_y_min, gc_y_max, gr_x_min, gr_x_max;
-    if (UNI) {  // opencl/das_uni_double.cl:213-216
-      gc_y_min = P.tri[3]; gc_y_max = P.tri[5];
-      gr_x_min = P.tri[0]; gr_x_max = P.tri[2];
-    } else {  // literal (num_cols/num_rows mixed) reads of the reference
-      gc_y_min = P.Gr[0 + 1 * P.Nt];
-      gc_y_max = P.Gr[P.Nt - 1 + 1 * P.Nt];
-      gr_x_min = P.Gt[0];
-      gr_x_max = P.Gt[P.Nr - 1];
-    }
-    if (yo >= gc_y_min && yo <= gc_y_max) gy_c = (T)0;
-    else if (yo < gc_y_min) gy_c = A::sub(gc_y_min, yo);
-    else gy_c = A::sub(gc_y_max, yo);
-    if (UNI) {
-      if (xo < gr_x_min || xo > gr_x_max) gx_r = (xo < gr_x_min) ? A::sub(gr_x_min, xo) : A::sub(gr_x_max, xo);
-    } else {
-      if (xo >= gr_x_min && xo <= gr_x_max) gx_r = (T)0;
-      else if (xo < gr_x_min) gx_r = A::sub(gr_x_min, xo);
-      else gx_r = A::sub(gr_x_max, xo);
+// One thread per point, every term tested on its own: SAFT images (IDX =
+// false), the index table of any method (IDX = true: every term's sample
+// index, -1 out of bounds, goes to P.idx instead of being gathered), and
+// TFM / RCA images whose inner elements are too many for the leg table of
+// das_plain_tile_kernel.
+template <class T, int M, bool UNI, bool BIGK, bool IDX>
+__global__ void __launch_bounds__(256) das_plain_kernel(const PlainParams<T> P) {
+  using A = Ar<T>;
+  const int64_t no_raw = P.no0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool active = no_raw < P.no1;
+  const int64_t no = active ? no_raw : P.no0;  // inactive lanes read a valid point and write nothing
+  PlainPoint<T, M, UNI> pt;
+  pt.init(P, no);
+  T im = (T)0;
+  unsigned int oob = 0;
+  const T *ycol = P.Y;
+  const int n_out = (M == RCA_ROWTX) ? P.Nr : P.Nt;
+  const int n_in = (M == SAFT) ? 1 : (M == RCA_ROWTX ? P.Nt : P.Nr);
+  for (int o = 0; o < n_out; o++) {
+    T lo = (M == SAFT) ? (T)0 : pt.outer_leg(P, o);
+    for (int i = 0; i < n_in; i++) {
+      // SAFT: exact doubling of one leg, as 2.0*t_tr
+      const T t = (M == SAFT) ? A::mul((T)2, pt.outer_leg(P, o)) : A::add(lo, pt.inner_leg(P, i));
+      const T p = A::mul(t, P.Fs);
+      const bool v = p > (T)-1 && p < P.Kf;
+      if constexpr (IDX) {
+        if (active) P.idx[((int64_t)o * n_in + i) * P.No + no] = v ? (int64_t)to_index<T, BIGK>(p) : -1;
+      } else if (v) {
+        im = A::add(im, load_y(P, ycol, to_index<T, BIGK>(p)));
+      }
+      oob += v ? 0 : 1;
+      ycol += P.K;
     }
   }
+  if (!IDX && active) P.Im[no] = im;
+  add_count(P.oob, active ? oob : 0u);
+}
 
-  // leg of a column stripe / row stripe / point element
-  auto leg_col = [&](int n) {
-    T ex, ey, ez;
-    elem_t(n, ex, ey, ez);
-    return leg_time(A::sub(ex, xo), gy_c, A::sub(ez, zo), P.ocp);
-  };
-  auto leg_row = [&](int n) {
-    T ex, ey, ez;
-    elem_r(n, ex, ey, ez);
-    return leg_time(gx_r, A::sub(ey, yo), A::sub(ez, zo), P.ocp);
-  };
-  auto leg_tx = [&](int n) {
-    T ex, ey, ez;
-    elem_t(n, ex, ey, ez);
-    return leg_time(A::sub(ex, xo), A::sub(ey, yo), A::sub(ez, zo), P.ocp);
-  };
-  auto leg_rx = [&](int n) {
-    T ex, ey, ez;
-    elem_r(n, ex, ey, ez);
-    return leg_time(A::sub(ex, xo), A::sub(ey, yo), A::sub(ez, zo), P.ocp);
-  };
+// Sample numbers of U terms with in-bounds times p = RN(RN(lo + li) * Fs) >= 0,
+// plus u * K for the u-th column of the group. FP64 adds 2^52 + u * K toward
+// zero, which leaves u * K + floor(p) in the low mantissa word; FP32 adds 2^23
+// and takes the bits from there (cofs = u * K - bits(2^23)).
+template <int U>
+__device__ __forceinline__ void sample_numbers(double lo, const double (&li)[U], double Fs, const double (&mag)[U],
+                                               uint32_t (&k)[U]) {
+#pragma unroll
+  for (int u = 0; u < U; u++)
+    k[u] = (uint32_t)__double2loint(__dadd_rz(__dmul_rn(__dadd_rn(lo, li[u]), Fs), mag[u]));
+}
+__device__ __forceinline__ uint64_t pair(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+template <int U>
+__device__ __forceinline__ void sample_numbers(float lo, const float (&li)[U], float Fs, const uint32_t (&cofs)[U],
+                                               uint32_t (&k)[U]) {
+  // two terms per instruction (each half rounds as the scalar operation)
+  const uint64_t lo2 = pair(lo, lo), fs2 = pair(Fs, Fs), mag2 = pair(8388608.0f, 8388608.0f);
+#pragma unroll
+  for (int u = 0; u < U; u += 2) {
+    uint64_t v = pair(li[u], li[u + 1]);
+    asm("add.rn.f32x2 %0, %1, %0;" : "+l"(v) : "l"(lo2));
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(fs2));
+    asm("add.rz.f32x2 %0, %0, %1;" : "+l"(v) : "l"(mag2));
+    k[u] = (uint32_t)v + cofs[u];
+    k[u + 1] = (uint32_t)(v >> 32) + cofs[u + 1];
+  }
+}
+template <class T>
+struct ColStep;
+template <>
+struct ColStep<double> {
+  using type = double;
+  static __device__ __forceinline__ double of(int u, int64_t K) { return 4503599627370496.0 + (double)(u * K); }
+};
+template <>
+struct ColStep<float> {
+  using type = uint32_t;
+  static __device__ __forceinline__ uint32_t of(int u, int64_t K) { return (uint32_t)(u * K) - 0x4B000000u; }
+};
+
+// TFM and RCA images (or, IDX, their index tables) with the inner legs of
+// every thread in shared memory.
+//
+// Bound and layout (64x64 elements, K = 3000, 512x512 points on B200; the same
+// frame with one branch per term and warps of 32 consecutive points took 2.43
+// ms in FP64 and 0.98 in FP32). FP64: 0.69 ms, 0.77 of the shared-memory / L1
+// data pipe (2 wavefronts per term for the leg, 2.3 for the 8-byte sample),
+// the FP64 pipe (two-leg add, scale, truncation, accumulate) at 0.42. FP32:
+// 0.36 ms, 8.6 instructions per term, 0.73 of the issue slots. What got it there:
+//  - no test per term. The shortest and the longest inner leg bound every time
+//    of an outer element exactly (rounded sums and products are monotone), so
+//    one vote per outer element shows that all its terms are in bounds.
+//  - sample numbers by adding a power of two toward zero, the column offset
+//    inside a group in the same addend (FP64) or one 32-bit add (FP32, whose
+//    leg sum, scale and truncation run two terms per instruction).
+//  - addresses by one 32x32+64-bit multiply-add (three moves per term fewer
+//    than pointer + index).
+//  - U = 16 gathers issued before the adds of the 16 before them: with 3 or 4
+//    blocks of 4 warps on an SM the gathers' latency is what is left (U = 8:
+//    0.82 and 0.42 ms).
+// MINB: resident blocks the registers must allow; 3 (170 registers), or 4
+// where the table lets a fourth in (32x32 elements, 256x256 points, FP64: less
+// than one wave of blocks, 0.065 against 0.094 ms).
+template <class T, int M, bool UNI, bool BIGK, bool IDX, int BD, int MINB>
+__global__ void __launch_bounds__(BD, MINB * 128 / BD) das_plain_tile_kernel(const PlainParams<T> P) {
+  using A = Ar<T>;
+  constexpr int U = MINB == 4 ? PLAIN_U / 2 : PLAIN_U;  // 16 FP64 samples, twice, do not fit 128 registers
+  constexpr int V = 16 / sizeof(T);  // legs per 16-byte table read
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T *tab = reinterpret_cast<T *>(smem_raw);  // leg i of thread t: tab[(i / V) * V * BD + t * V + i % V]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int64_t no_raw, first;
+  bool active;
+  if (P.n_fast > 0) {
+    constexpr int PF = plain_patch_f(M), TF = plain_tile_f(M, BD), WF = TF / PF;  // lanes, points, warps along the fast axis
+    const int64_t f0 = (int64_t)blockIdx.x * TF, s0 = (P.no0 + blockIdx.y) * plain_tile_s(M, BD);
+    const int64_t f = f0 + (warp % WF) * PF + lane % PF;
+    const int64_t s = s0 + (warp / WF) * (32 / PF) + lane / PF;
+    active = f < P.n_fast && s < P.n_slow;
+    no_raw = s * P.n_fast + f;
+    first = s0 * P.n_fast + f0;
+  } else {
+    no_raw = P.no0 + (int64_t)blockIdx.x * BD + tid;
+    active = no_raw < P.no1;
+    first = P.no0 + (int64_t)blockIdx.x * BD;
+  }
+  const int64_t no = active ? no_raw : first;  // inactive lanes repeat the tile's first point and write nothing
+  PlainPoint<T, M, UNI> pt;
+  pt.init(P, no);
+  const int n_out = (M == RCA_ROWTX) ? P.Nr : P.Nt;
+  const int n_in = (M == RCA_ROWTX) ? P.Nt : P.Nr;
+  T mn = (T)INFINITY, mx = -(T)INFINITY;
+  bool fin = P.Fs > (T)0;
+  for (int i = 0; i < n_in; i++) {
+    const T l = pt.inner_leg(P, i);
+    tab[(i / V) * V * BD + tid * V + i % V] = l;
+    mn = l < mn ? l : mn;
+    mx = l > mx ? l : mx;
+    fin = fin && l == l;  // a NaN leg leaves every group to the tested form
+  }
+  typename ColStep<T>::type step[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) step[u] = ColStep<T>::of(u, P.K);
 
   T im = (T)0;
   unsigned int oob = 0;
   const T *ycol = P.Y;
-
-  if (M == SAFT) {
-    for (int n = 0; n < P.Nt; n++) {
-      T t = A::add(leg_tx(n), delay_ms);
-      T tdp = A::mul((T)2, t);  // exact doubling, as 2.0*t_tr
-      T p = A::mul(tdp, P.Fs);
-      if constexpr (IDX) {
+  int64_t *idx = IDX ? P.idx + no : nullptr;
+  auto legs = [&](int i, T(&li)[U]) {
+#pragma unroll
+    for (int v = 0; v < U / V; v++)
+#pragma unroll
+      for (int q = 0; q < V; q++) li[v * V + q] = tab[(i / V + v) * V * BD + tid * V + q];
+  };
+  // samples of terms (o, i .. i+U-1); terms past n_in and out-of-bounds ones
+  // are +0, which the sum (never -0: it starts from +0) takes unchanged
+  auto gather = [&](T lo, int i, T(&y)[U], bool full) {
+    T li[U];
+    uint32_t k[U];
+    legs(i, li);
+    sample_numbers<U>(lo, li, P.Fs, step, k);
+    const T *yb = ycol + (int64_t)i * P.K;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      y[u] = (T)0;
+      if (full || i + u < n_in) y[u] = load_at(P, yb, k[u]);
+    }
+  };
+  auto gather_tested = [&](T lo, int i, T(&y)[U]) {
+    T li[U];
+    legs(i, li);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      y[u] = (T)0;
+      if (i + u < n_in) {
+        const T p = A::mul(A::add(lo, li[u]), P.Fs);
         const bool v = p > (T)-1 && p < P.Kf;
-        if (active) P.idx[(int64_t)n * P.No + no] = v ? (int64_t)to_index<T, BIGK>(p) : -1;
-        oob += v ? 0 : 1;
-      } else if (p > (T)-1 && p < P.Kf) {
-        im = A::add(im, load_y(P, ycol, to_index<T, BIGK>(p)));
-      } else {
-        oob++;
-      }
-      ycol += P.K;
-    }
-  } else {
-    // outer / inner element roles and which leg carries the delay
-    const int n_out = (M == RCA_ROWTX) ? P.Nr : P.Nt;
-    const int n_in = (M == RCA_ROWTX) ? P.Nt : P.Nr;
-    // das row-tx: delay on the (inner) column leg; das_uni row-tx: on the
-    // (outer) row leg (opencl/das_uni_double.cl:358-360).
-    const bool delay_outer = (M != RCA_ROWTX) || UNI;
-    auto inner_leg = [&](int i) -> T {
-      T l;
-      if (M == TFM) l = leg_rx(i);
-      else if (M == RCA_COLTX) l = leg_row(i);
-      else l = leg_col(i);
-      return delay_outer ? l : A::add(l, delay_ms);
-    };
-    if (TAB) {
-      for (int i = 0; i < n_in; i++) tab[i * bd + tid] = inner_leg(i);
-    }
-    for (int o = 0; o < n_out; o++) {
-      T lo;
-      if (M == TFM) lo = leg_tx(o);
-      else if (M == RCA_COLTX) lo = leg_col(o);
-      else lo = leg_row(o);
-      if (delay_outer) lo = A::add(lo, delay_ms);
-      int i = 0;
-      // UNROLL terms at a time: all gathers are issued before the adds, which
-      // then run in the reference order (the sum is unchanged bit for bit).
-      for (; i + UNROLL <= n_in; i += UNROLL) {
-        T y[UNROLL];
-        bool v[UNROLL];
-#pragma unroll
-        for (int u = 0; u < UNROLL; u++) {
-          T li = TAB ? tab[(i + u) * bd + tid] : inner_leg(i + u);
-          T p = A::mul(A::add(lo, li), P.Fs);
-          v[u] = p > (T)-1 && p < P.Kf;
-          if constexpr (IDX) {
-            if (active) P.idx[((int64_t)o * n_in + i + u) * P.No + no] = v[u] ? (int64_t)to_index<T, BIGK>(p) : -1;
-            y[u] = (T)0;
-          } else {
-            y[u] = v[u] ? load_y(P, ycol, (int64_t)u * P.K + to_index<T, BIGK>(p)) : (T)0;
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < UNROLL; u++) {
-          if (v[u]) im = A::add(im, y[u]);
-          else oob++;
-        }
-        ycol += UNROLL * P.K;
-      }
-      for (; i < n_in; i++) {
-        T li = TAB ? tab[i * bd + tid] : inner_leg(i);
-        T p = A::mul(A::add(lo, li), P.Fs);
         if constexpr (IDX) {
-          const bool v = p > (T)-1 && p < P.Kf;
-          if (active) P.idx[((int64_t)o * n_in + i) * P.No + no] = v ? (int64_t)to_index<T, BIGK>(p) : -1;
-          oob += v ? 0 : 1;
-        } else if (p > (T)-1 && p < P.Kf) {
-          im = A::add(im, load_y(P, ycol, to_index<T, BIGK>(p)));
-        } else {
-          oob++;
+          if (active) *idx = v ? (int64_t)to_index<T, BIGK>(p) : -1;
+          idx += P.No;
+        } else if (v) {
+          const int k = to_index<T, BIGK>(p);
+          y[u] = BIGK ? load_y(P, ycol + (int64_t)(i + u) * P.K, k)
+                      : load_at(P, ycol + (int64_t)i * P.K, (uint32_t)u * (uint32_t)P.K + (uint32_t)k);
         }
-        ycol += P.K;
+        oob += v ? 0 : 1;
       }
     }
+  };
+  auto accumulate = [&](const T(&y)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; u++) im = A::add(im, y[u]);
+  };
+  // Two groups alternate: the gathers of one are issued before the in-order
+  // adds of the other, so the sum's serial adds overlap the gathers' latency.
+  T ya[U], yb[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) yb[u] = (T)0;
+  for (int o = 0; o < n_out; o++) {
+    const T lo = pt.outer_leg(P, o);
+    // Rounded sums and products are monotone, so every time of this outer
+    // element lies between those of the shortest and the longest inner leg.
+    const bool in = fin && A::mul(A::add(lo, mn), P.Fs) >= (T)0 && A::mul(A::add(lo, mx), P.Fs) < P.Kf;
+    if (!BIGK && !IDX && __all_sync(0xffffffffu, in)) {
+      int i = 0;
+      for (; i + 2 * U <= n_in; i += 2 * U) {
+        gather(lo, i, ya, true);
+        accumulate(yb);
+        gather(lo, i + U, yb, true);
+        accumulate(ya);
+      }
+      if (i < n_in) {
+        gather(lo, i, ya, false);
+        accumulate(yb);
+        gather(lo, i + U, yb, false);
+        accumulate(ya);
+      }
+    } else {
+      for (int i = 0; i < n_in; i += 2 * U) {
+        gather_tested(lo, i, ya);
+        accumulate(yb);
+        gather_tested(lo, i + U, yb);
+        accumulate(ya);
+      }
+    }
+    ycol += (int64_t)n_in * P.K;
   }
+  accumulate(yb);
   if (!IDX && active) P.Im[no] = im;
   add_count(P.oob, active ? oob : 0u);
 }
@@ -300,47 +427,57 @@ __global__ void __launch_bounds__(256) das_plain_kernel(const PlainParams<T> P) 
 // launcher
 // ---------------------------------------------------------------------------
 
-template <class T, int M, bool UNI, bool TAB, bool IDX = false>
-static cudaError_t launch_one(const PlainParams<T> &P, int bd, size_t smem, cudaStream_t st) {
-  const bool patch = P.n_fast > 0, bigk = sizeof(T) == 4 && P.bigk;
-  auto kern = patch ? (bigk ? das_plain_kernel<T, M, UNI, TAB, true, IDX, true>
-                            : das_plain_kernel<T, M, UNI, TAB, false, IDX, true>)
-                    : (bigk ? das_plain_kernel<T, M, UNI, TAB, true, IDX, false>
-                            : das_plain_kernel<T, M, UNI, TAB, false, IDX, false>);
-  cudaError_t e = ensure_smem(kern, smem);
-  if (e != cudaSuccess) return e;
-  dim3 grid;
-  if (patch) {  // [no0, no1) are patch rows; a block holds bd / 32 patches of a row
-    const int64_t wpb = bd >> 5;
-    grid = dim3((unsigned)(((P.n_fast + PLAIN_PATCH_F - 1) / PLAIN_PATCH_F + wpb - 1) / wpb), (unsigned)(P.no1 - P.no0));
-  } else {
-    grid = dim3((unsigned)((P.no1 - P.no0 + bd - 1) / bd));
-  }
-  kern<<<grid, bd, smem, st>>>(P);
+template <class T, int M, bool UNI, bool IDX>
+static cudaError_t launch_terms(const PlainParams<T> &P, cudaStream_t st) {
+  const bool bigk = sizeof(T) == 4 && P.bigk;
+  auto kern = bigk ? das_plain_kernel<T, M, UNI, true, IDX> : das_plain_kernel<T, M, UNI, false, IDX>;
+  kern<<<(unsigned)((P.no1 - P.no0 + 255) / 256), 256, 0, st>>>(P);
   return cudaGetLastError();
 }
 
+template <class T, int M, bool UNI, bool IDX, int BD, int MINB = 3>
+static cudaError_t launch_tile(const PlainParams<T> &P, int n_in, cudaStream_t st) {
+  const size_t smem = plain_table_bytes(n_in, sizeof(T), BD);
+  auto kern = P.bigk ? das_plain_tile_kernel<T, M, UNI, true, IDX, BD, MINB>
+                     : das_plain_tile_kernel<T, M, UNI, false, IDX, BD, MINB>;
+  cudaError_t e = ensure_smem(kern, smem);
+  if (e != cudaSuccess) return e;
+  dim3 grid;
+  if (P.n_fast > 0) {  // [no0, no1) are tile rows
+    constexpr int tf = plain_tile_f(M, BD);
+    grid = dim3((unsigned)((P.n_fast + tf - 1) / tf), (unsigned)(P.no1 - P.no0));
+  } else {
+    grid = dim3((unsigned)((P.no1 - P.no0 + BD - 1) / BD));
+  }
+  kern<<<grid, BD, smem, st>>>(P);
+  return cudaGetLastError();
+}
+
+template <class T, int M, bool UNI, bool IDX>
+static cudaError_t launch_method(const PlainParams<T> &P, cudaStream_t st) {
+  if constexpr (M == SAFT) {
+    return launch_terms<T, M, UNI, IDX>(P, st);
+  } else {
+    const int n_in = M == RCA_ROWTX ? P.Nt : P.Nr;
+    switch (plain_tile_threads(n_in, sizeof(T))) {
+      case 128:
+        if constexpr (sizeof(T) == 8 && !IDX)  // FP32 blocks need few enough registers for a fourth anyway
+          if (plain_table_bytes(n_in, sizeof(T), 128) <= 54 * 1024) return launch_tile<T, M, UNI, IDX, 128, 4>(P, n_in, st);
+        return launch_tile<T, M, UNI, IDX, 128>(P, n_in, st);
+      case 64: return launch_tile<T, M, UNI, IDX, 64>(P, n_in, st);
+      case 32: return launch_tile<T, M, UNI, IDX, 32>(P, n_in, st);
+      default: return launch_terms<T, M, UNI, IDX>(P, st);
+    }
+  }
+}
+
 template <class T, bool UNI, bool IDX = false>
-static cudaError_t launch_method(int method, const PlainParams<T> &P, cudaStream_t st) {
-  const int n_in = (method == SAFT) ? 0 : (method == RCA_ROWTX ? P.Nt : P.Nr);
-  // Largest block whose per-thread inner-leg table fits in 64 KB (three
-  // blocks per SM); very long inner loops fall back to recomputing the leg.
-  int bd = 256;
-  while (bd > 32 && (size_t)n_in * bd * sizeof(T) > 64 * 1024) bd >>= 1;
-  bool tab = (size_t)n_in * bd * sizeof(T) <= 200 * 1024;
-  if (!tab) bd = 128;
-  size_t smem = tab ? (size_t)n_in * bd * sizeof(T) : 0;
+static cudaError_t launch_any(int method, const PlainParams<T> &P, cudaStream_t st) {
   switch (method) {
-    case SAFT: return launch_one<T, SAFT, UNI, false, IDX>(P, 256, 0, st);
-    case TFM:
-      return tab ? launch_one<T, TFM, UNI, true, IDX>(P, bd, smem, st)
-                 : launch_one<T, TFM, UNI, false, IDX>(P, bd, 0, st);
-    case RCA_COLTX:
-      return tab ? launch_one<T, RCA_COLTX, UNI, true, IDX>(P, bd, smem, st)
-                 : launch_one<T, RCA_COLTX, UNI, false, IDX>(P, bd, 0, st);
-    case RCA_ROWTX:
-      return tab ? launch_one<T, RCA_ROWTX, UNI, true, IDX>(P, bd, smem, st)
-                 : launch_one<T, RCA_ROWTX, UNI, false, IDX>(P, bd, 0, st);
+    case SAFT: return launch_method<T, SAFT, UNI, IDX>(P, st);
+    case TFM: return launch_method<T, TFM, UNI, IDX>(P, st);
+    case RCA_COLTX: return launch_method<T, RCA_COLTX, UNI, IDX>(P, st);
+    case RCA_ROWTX: return launch_method<T, RCA_ROWTX, UNI, IDX>(P, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -367,7 +504,7 @@ static PlainParams<T> make_params(const PlainLaunch &L) {
   P.ny = L.ny;
   P.bad = L.bad;
   P.idx = L.idx;
-  P.bigk = L.K >= (int64_t(1) << 22);
+  P.bigk = L.K >= (int64_t(1) << (sizeof(T) == 4 ? 22 : 28));
   P.Nx = L.Nx;
   P.Ny = L.Ny;
   P.Nz = L.Nz;
@@ -382,9 +519,9 @@ cudaError_t launch_plain_f64(const PlainLaunch &L, cudaStream_t st) {
   P.Kf = (double)L.K;
   for (int i = 0; i < 15; i++) P.tri[i] = L.tri64[i];
   if (L.idx)
-    return L.uni ? launch_method<double, true, true>(L.method, P, st)
-                 : launch_method<double, false, true>(L.method, P, st);
-  return L.uni ? launch_method<double, true>(L.method, P, st) : launch_method<double, false>(L.method, P, st);
+    return L.uni ? launch_any<double, true, true>(L.method, P, st)
+                 : launch_any<double, false, true>(L.method, P, st);
+  return L.uni ? launch_any<double, true>(L.method, P, st) : launch_any<double, false>(L.method, P, st);
 }
 
 cudaError_t launch_plain_f32(const PlainLaunch &L, cudaStream_t st) {
@@ -395,9 +532,9 @@ cudaError_t launch_plain_f32(const PlainLaunch &L, cudaStream_t st) {
   P.Kf = (float)L.K;
   for (int i = 0; i < 15; i++) P.tri[i] = L.tri32[i];
   if (L.idx)
-    return L.uni ? launch_method<float, true, true>(L.method, P, st)
-                 : launch_method<float, false, true>(L.method, P, st);
-  return L.uni ? launch_method<float, true>(L.method, P, st) : launch_method<float, false>(L.method, P, st);
+    return L.uni ? launch_any<float, true, true>(L.method, P, st)
+                 : launch_any<float, false, true>(L.method, P, st);
+  return L.uni ? launch_any<float, true>(L.method, P, st) : launch_any<float, false>(L.method, P, st);
 }
 
 }  // namespace dream
