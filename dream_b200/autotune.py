@@ -1,8 +1,7 @@
 """Autotuner for the FP32/BF16-storage DAS kernels.
 
-Picks, per shape bucket, the CTA tile of image points (tile_f x tile_s) and
-the inner-chunk length (8 or 16 register-resident legs) by timing each
-candidate on the actual frame with CUDA events (median of a few runs after a
+Picks, per shape bucket, the CTA tile of image points (tile_f x tile_s) by
+timing each candidate on the actual frame with CUDA events (median of a few runs after a
 warm-up, the L2 cache flushed before each timed run: a frame that arrives from
 the host or from another kernel is not L2-resident, and shapes that win with
 warm caches can lose without them). Results are cached in a JSON file keyed by GPU name, method,
@@ -65,20 +64,20 @@ def _p2(n: int) -> int:
 def bucket_key(method, storage, Nt, Nr, K, n_fast, No, nthr, device) -> str:
     name = torch.cuda.get_device_name(device).replace(" ", "_")
     n_slow = No // n_fast if n_fast else 1
-    return (f"v2|{name}|{method}|{storage}|nthr={nthr}|Nt={Nt}|Nr={Nr}|K={_p2(K)}|"
+    return (f"v3|{name}|{method}|{storage}|nthr={nthr}|Nt={Nt}|Nr={Nr}|K={_p2(K)}|"
             f"grid={_p2(n_fast) if n_fast else 0}x{_p2(n_slow)}")
 
 
 def candidates(hinted: bool, nthr: int):
-    """(tile_f, tile_s, jc) shapes with tile_f*tile_s == nthr."""
+    """(tile_f, tile_s, jc) shapes with tile_f*tile_s == nthr (the gathers have one chunk length)."""
     out = []
     if hinted:
         for tf in (8, 16, 32, 64):
             ts = nthr // tf
             if ts >= 4 and ts % 4 == 0 and tf * ts == nthr:
-                out += [(tf, ts, 16), (tf, ts, 8)]
+                out.append((tf, ts, 16))
     else:
-        out += [(nthr, 1, 16), (nthr, 1, 8)]
+        out.append((nthr, 1, 16))
     return out
 
 

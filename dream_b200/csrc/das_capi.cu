@@ -338,39 +338,53 @@ int zero_length_ascans(dream_das_plan *p, void *dIm, unsigned long long *doob, c
   return 0;
 }
 
-// Tile of the FP32/BF16-storage kernels: the user's, or the largest CTA
-// whose outer-leg table (n_out x threads x 4 B) fits in 96 KB, at most 128
-// points on a hinted grid (16 x 8: on the 64x64-element TFM frame 0.532 ms
-// against 0.565 ms for 32 x 8) and 256 consecutive points otherwise.
-void fast_tile(const dream_das_plan *p, int n_out, int &tf, int &ts, int &wf) {
+// Tile of the operator's adjoint: the user's, or the largest CTA whose
+// outer-leg table (n_out x threads x 4 B) fits in 96 KB, 16 x 8 points on a
+// hinted grid (8 x 32 for frames of fewer points than two waves of 128-point
+// tiles, whose set-up then serves twice the points) and 256 consecutive points
+// otherwise. TFM on a hinted grid: 8 x 32 points, long along the slow axis,
+// where a column's sample window grows slowest relative to the tile's terms
+// (64x64-element TFM frame 1.25 -> 1.20 ms, 32x32-element CG configuration
+// 0.130 -> 0.120 ms, against 16 x 8). RCA volumes keep the short tile: 32
+// points along their slow axis spread a stripe's leg beyond the window
+// (128x128 frame: 108.7 against 81.7 ms).
+void scatter_tile(const dream_das_plan *p, FastParams &F) {
+  const int n_out = (F.method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt;
+  const bool hint = p->n_fast > 0;
+  F.wf = hint ? 8 : 32;
   if (p->tile_f > 0) {
-    tf = p->tile_f;
-    ts = p->tile_s;
-    wf = p->n_fast > 0 ? 8 : 32;
+    F.tile_f = p->tile_f;
+    F.tile_s = p->tile_s;
     return;
   }
-  // frames of fewer points than two waves of 128-point tiles (the CG
-  // configuration's 256x256): 8 x 32-point tiles, whose per-tile set-up serves
-  // twice the points (0.091 against 0.096 ms for that frame's forward)
-  const bool small = p->n_fast > 0 && p->No < (int64_t)p->sm_count * 8 * 128;
-  int nthr = (p->n_fast > 0 && !small) ? 128 : 256;
+  const bool small = hint && p->No < (int64_t)p->sm_count * 8 * 128;
+  int nthr = (hint && !small) ? 128 : 256;
   while (nthr > 32 && (size_t)n_out * nthr * 4 > 96 * 1024) nthr >>= 1;
-  if (p->n_fast > 0) {
-    wf = 8;
-    tf = small ? 8 : (nthr >= 256 ? 32 : (nthr >= 64 ? 16 : 8));
-    ts = nthr / tf;
-  } else {
-    wf = 32;
-    tf = nthr;
-    ts = 1;
+  F.tile_f = !hint ? nthr : (small ? 8 : (nthr >= 64 ? 16 : 8));
+  F.tile_s = nthr / F.tile_f;
+  if (hint && F.method == DREAM_DAS_TFM && (size_t)n_out * 256 * 4 <= 96 * 1024) {
+    F.tile_f = 8;
+    F.tile_s = 32;
   }
 }
 
-// Tiling of the FP32/BF16-storage kernels for plan p: tile shape, warp
-// layout, register chunk and grid axes (F.method, Nt, Nr, No must be set).
+// Tile of the gathers: the user's, or 128 points, 8 x 16 on a TFM grid and 16 x
+// 8 on an RCA's (64 and 256 points measure within 3 % of these; see gather_patch_f).
+void gather_tile(const dream_das_plan *p, int method, int &tf, int &ts, int &wf) {
+  const bool hint = p->n_fast > 0;
+  if (p->tile_f > 0) {
+    tf = p->tile_f;
+    ts = p->tile_s;
+  } else {
+    tf = !hint ? 128 : (method == DREAM_DAS_TFM ? 8 : 16);
+    ts = 128 / tf;
+  }
+  wf = gather_patch_f(method, hint, ts);
+}
+
+// Grid axes, chunk and adjoint tile of the FP32/BF16-storage kernels for plan p
+// (F.method, Nt, Nr, No must be set).
 int tile_params(const dream_das_plan *p, FastParams &F, int jc) {
-  const int n_out = (F.method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt;
-  fast_tile(p, n_out, F.tile_f, F.tile_s, F.wf);
   F.jc = jc ? jc : (p->jc ? p->jc : 16);
   if (p->n_fast > 0) {
     F.n_fast = p->n_fast;
@@ -379,8 +393,17 @@ int tile_params(const dream_das_plan *p, FastParams &F, int jc) {
     F.n_fast = p->No;
     F.n_slow = 1;
   }
+  scatter_tile(p, F);
   if (fast_smem_bytes(F, F.tile_f * F.tile_s) > 220 * 1024)
     return fail(DREAM_ERR_UNSUPPORTED, "too many elements on the outer loop for the FP32/BF16 storage kernels");
+  return 0;
+}
+// The same with the gathers' tile.
+int gather_params(const dream_das_plan *p, FastParams &F) {
+  int r = tile_params(p, F, 0);
+  if (r) return r;
+  gather_tile(p, F.method, F.tile_f, F.tile_s, F.wf);
+  F.out_block = gather_out_block((F.method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt, F.w == nullptr);
   return 0;
 }
 
@@ -418,8 +441,7 @@ int64_t slow_tile_chunk(const FastParams &F, int64_t terms_per_pixel) {
 
 int launch_fast_plan(dream_das_plan *p, const void *dY, const void *dRo, const void *dGt, const void *dGr,
                      double dt, int delay_type, const void *ddelay, double cp, const float *dW, float *dIm,
-                     unsigned long long *doob, cudaStream_t st, int in_lo = 0, int in_hi = 0, int accumulate = 0,
-                     int jc = 0) {
+                     unsigned long long *doob, cudaStream_t st, int in_lo = 0, int in_hi = 0, int accumulate = 0) {
   if (delay_type != DREAM_DELAY_SINGLE && delay_type != DREAM_DELAY_MULTIPLE)
     return fail(DREAM_ERR_ARGUMENT, "unknown delay type");
   if (ddelay == nullptr) return fail(DREAM_ERR_ARGUMENT, "delay pointer is NULL");
@@ -472,7 +494,7 @@ int launch_fast_plan(dream_das_plan *p, const void *dY, const void *dRo, const v
     return 0;
   }
   const int n_out = (method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt;
-  int r = tile_params(p, F, jc);
+  int r = gather_params(p, F);
   if (r) return r;
   const int64_t slow_tiles = (F.n_slow + F.tile_s - 1) / F.tile_s;
   const int64_t chunk = slow_tile_chunk(F, tpp);
@@ -699,8 +721,7 @@ int dream_das_get_tile(const dream_das_plan *p, int *tile_f, int *tile_s) {
   DREAM_API_TRY
   if (p == nullptr || tile_f == nullptr || tile_s == nullptr) return fail(DREAM_ERR_ARGUMENT, "NULL argument");
   int wf = 0;
-  const int n_out = (effective_method(p) == DREAM_DAS_RCA_ROWTX) ? (int)p->Nr : (int)p->Nt;
-  fast_tile(p, n_out, *tile_f, *tile_s, wf);
+  gather_tile(p, effective_method(p), *tile_f, *tile_s, wf);
   return 0;
   DREAM_API_CATCH
 }
@@ -754,7 +775,7 @@ static int op_gather(dream_das_plan *p, const float *dY, const float *dW, float 
   F.oob = d_oob;
   F.ny = p->K * num_columns(p);
   F.bad = bad_counter(p);
-  int r = tile_params(p, F, 0);
+  int r = gather_params(p, F);
   if (r) return r;
   if (!apply_shard(p, F)) return 0;
   const int64_t slow_tiles = (F.n_slow + F.tile_s - 1) / F.tile_s;
@@ -778,18 +799,6 @@ static int op_scatter(dream_das_plan *p, const float *X, const float *dW, float 
   F.w = dW;
   int r = tile_params(p, F, 0);
   if (r) return r;
-  // The scatter's own automatic tile on a hinted TFM grid: 8 x 32 points,
-  // long along the slow axis, where a column's sample window grows slowest
-  // relative to the tile's terms (64x64-element TFM frame 1.25 -> 1.20 ms,
-  // 32x32-element CG configuration 0.130 -> 0.120 ms, against 16 x 8). RCA
-  // volumes keep the forward's tile: 32 points along their slow axis spread a
-  // stripe's leg beyond the window (128x128 frame: 108.7 against 81.7 ms).
-  const int n_out = (F.method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt;
-  if (p->tile_f == 0 && p->n_fast > 0 && F.method == DREAM_DAS_TFM && (size_t)n_out * 256 * 4 <= 96 * 1024) {
-    F.tile_f = 8;
-    F.tile_s = 32;
-    F.wf = 8;
-  }
   if (!apply_shard(p, F)) return 0;
   const int64_t slow_tiles = (F.n_slow + F.tile_s - 1) / F.tile_s;
   const int64_t chunk = slow_tile_chunk(F, terms_per_pixel(p));
@@ -911,17 +920,17 @@ int batch_frame_params(const dream_das_frame &d, FastParams &F) {
   if (d.n_fast > 0) {
     F.n_fast = d.n_fast;
     F.n_slow = d.No / d.n_fast;
-    F.wf = 8;
-    F.tile_f = d.tile_f ? d.tile_f : 16;
-    F.tile_s = d.tile_s ? d.tile_s : 8;
+    F.tile_f = d.tile_f ? d.tile_f : (F.method == DREAM_DAS_TFM ? 8 : 16);
+    F.tile_s = d.tile_s ? d.tile_s : 128 / F.tile_f;
   } else {
     F.n_fast = d.No;
     F.n_slow = 1;
-    F.wf = 32;
     F.tile_f = 128;
     F.tile_s = 1;
   }
+  F.wf = gather_patch_f(F.method, d.n_fast > 0, F.tile_s);
   F.jc = d.jc ? d.jc : 16;
+  F.out_block = gather_out_block((F.method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt, false);
   return 0;
 }
 }  // namespace dream
@@ -970,16 +979,16 @@ int dream_das_batch_create(dream_das_batch **out, const dream_das_frame *fr, int
       dream_das_batch_destroy(b);
       return r;
     }
-    b->smem = std::max(b->smem, fast_smem_bytes(F, 128));
+    if (fast_smem_bytes(F, 128) > 220 * 1024) {
+      dream_das_batch_destroy(b);
+      return fail(DREAM_ERR_UNSUPPORTED, "a frame has too many outer elements for the batch kernel");
+    }
+    b->smem = std::max(b->smem, gather_smem_bytes(F, 128));
     b->frames.push_back(F);
     if (d.No > 0 && d.a_scan_len > 0) {
       const int64_t tf = (F.n_fast + F.tile_f - 1) / F.tile_f, ts = (F.n_slow + F.tile_s - 1) / F.tile_s;
       groups.push_back({(double)d.num_t_elements * d.num_r_elements, f, tf, ts});
     }
-  }
-  if (b->smem > 220 * 1024) {
-    dream_das_batch_destroy(b);
-    return fail(DREAM_ERR_UNSUPPORTED, "a frame has too many outer elements for the batch kernel");
   }
   // largest per-tile cost first: the queue drains big tiles before small ones
   std::stable_sort(groups.begin(), groups.end(), [](const Group &a, const Group &c) { return a.cost > c.cost; });
@@ -1301,10 +1310,8 @@ int dream_das_run(dream_das_plan *p, const void *Y, const void *Ro, const void *
       }
       CU(cudaEventRecord(p->chunk_ev[c], p->copy_stream));
       CU(cudaStreamWaitEvent(st, p->chunk_ev[c], 0));
-      // a register chunk that divides the range keeps every chunk full
-      const int jc = ((hi - lo) % 16 == 0) ? 16 : (((hi - lo) % 8 == 0) ? 8 : 0);
       r = launch_fast_plan(p, bf16 ? p->bY16.p : p->bY.p, p->bRo.p, p->bGt.p, p->bGr.p, dt, delay_type, p->bDelay.p,
-                           cp, nullptr, (float *)p->bIm.p, doob, st, lo, hi, c > 0 ? 1 : 0, jc);
+                           cp, nullptr, (float *)p->bIm.p, doob, st, lo, hi, c > 0 ? 1 : 0);
       if (r) return r;
     }
     void *staged = nullptr;

@@ -1,14 +1,19 @@
 // das_fast.cu -- DAS with FP32- or BF16-stored A-scans, FP32 compensated
 // accumulation and FP64-exact sample indices (precision upgrade of the
 // reference's das_double/das_float forms; optional per-column weights for
-// the differentiable operator).
+// the differentiable operator), and the operator's adjoint.
 //
-// Index exactness. A term's sample index is trunc(RN(RN(a + b) * Fs)) with
-// a, b the two FP64 leg times of the reference (extra_src/das.cc:392-404 and
-// its RCA/SAFT counterparts). Each leg is computed exactly once per (pixel,
-// element) in FP64, scaled by Fs in FP64 (A = RN(a*Fs), B = RN(b*Fs)) and
-// stored as fixed point relative to a tile-wide integer base, in one of two
-// formats chosen per tile:
+// Gather: every index by the reference's own FP64 chain (below, at
+// gather_issue). Tiles: a CTA owns a 2-D tile of image points (tile_f along the
+// fastest grid axis x tile_s along the next one, when the caller gives the
+// grid's fastest extent n_fast; otherwise consecutive points), so the 32
+// gathers of one warp fall on one or two 128-byte lines of the A-scan.
+//
+// Scatter (adjoint): the same indices from fixed-point legs. A term's sample
+// index is trunc(RN(RN(a + b) * Fs)) with a, b the two FP64 leg times of the
+// reference (extra_src/das.cc:392-404 and its RCA/SAFT counterparts). Each leg
+// is computed once per (pixel, element), scaled by Fs and stored as fixed point
+// relative to a tile-wide integer base, in one of two formats chosen per tile:
 //   fine: 24 fraction bits, legs spreading over < 127 samples in the tile;
 //         rounding <= 2^-25 per leg, delta = 2^-22, band 2*delta = 2^-21;
 //   wide: 20 fraction bits (coarse grids, spreads up to 4000 samples);
@@ -20,18 +25,9 @@
 // at least 2*delta. Terms inside the band (about 1 in 2 million with the
 // fine format) take an exact FP64 recomputation. The finer format matters
 // for speed: a warp with one ambiguous lane runs the serial FP64 path. The
-// selected indices are identical to the FP64 plain kernel's.
-//
-// Hot loop. The fixed-point leg carries the A-scan column offset in its high
-// word: with A64 = (offset_t + baseA) << 32 | fraction and the same for B, one
-// 64-bit add gives the sample's element offset in the high word and the
-// fraction in the low word, so a term costs: 64-bit add, one compare, address,
-// load, add.
-//
-// Tiles. A CTA owns a 2-D tile of image points (tile_f along the fastest grid
-// axis x tile_s along the next one, when the caller gives the grid's fastest
-// extent n_fast; otherwise consecutive points). Warps are 8 x 4 points so the
-// 32 gathers of one warp fall on one or two 128-byte lines of the A-scan.
+// selected indices are identical to the FP64 plain kernel's. The fixed-point
+// leg's 64-bit sum has the term's window cell in its high word and the fraction
+// in its low word.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -67,12 +63,11 @@ __device__ __forceinline__ float load_sample<__nv_bfloat16>(const __nv_bfloat16 
   return __uint_as_float(((unsigned int)u) << 16);
 }
 
-// base + off elements as one 32x32->64 multiply-add, which runs on the FMA
-// pipe and leaves the integer ALU to the index arithmetic.
+// base (bytes) + off elements as one 32x32+64-bit multiply-add: as pointer + index it takes three moves more.
 template <class YT>
-__device__ __forceinline__ const YT *elem_addr(const YT *base, uint32_t off) {
+__device__ __forceinline__ const YT *elem_addr(const char *base, uint32_t off) {
   const YT *r;
-  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(off), "r"((uint32_t)sizeof(YT)), "l"(base));
+  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(off), "n"((int)sizeof(YT)), "l"(base));
   return r;
 }
 
@@ -90,6 +85,11 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
 __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
 __device__ __forceinline__ float lo_f32(uint64_t v) { return __uint_as_float((uint32_t)v); }
@@ -134,38 +134,42 @@ __device__ __forceinline__ void pixel_of(const FastParams &P, int64_t no, Pixel 
   }
 }
 
-// Exact FP64 leg of outer element o / inner element i, including the delay on
-// the leg that carries it (TFM and col-tx: outer; row-tx: inner, the column).
-__device__ __forceinline__ double outer_leg(const FastParams &P, const Pixel &px, int o) {
-  using A = Ar<double>;
-  double l;
+// Coordinate differences between image point px and element e (outer or
+// inner), as the reference forms them for each method: TFM uses the element's
+// position; an RCA column (Gt) its x and z with the clamped y offset of the
+// column stripe, an RCA row (Gr) its y and z with the clamped x offset.
+__device__ __forceinline__ void leg_diffs(const FastParams &P, const Pixel &px, bool outer, int e, double &dx,
+                                          double &dy, double &dz) {
   if (P.method == TFM) {
-    l = leg_time(A::sub(P.Gt[o], px.xo), A::sub(P.Gt[o + P.Nt], px.yo), A::sub(P.Gt[o + 2 * P.Nt], px.zo), P.ocp);
-  } else if (P.method == RCA_COLTX) {
-    l = leg_time(A::sub(P.Gt[o], px.xo), px.gy_c, A::sub(P.Gt[o + 2 * P.Nt], px.zo), P.ocp);
-  } else {  // row-tx: outer = rows
-    l = leg_time(px.gx_r, A::sub(P.Gr[o + P.Nr], px.yo), A::sub(P.Gr[o + 2 * P.Nr], px.zo), P.ocp);
+    const double *G = outer ? P.Gt : P.Gr;
+    const int N = outer ? P.Nt : P.Nr;
+    dx = __dsub_rn(__ldg(G + e), px.xo);
+    dy = __dsub_rn(__ldg(G + e + N), px.yo);
+    dz = __dsub_rn(__ldg(G + e + 2 * N), px.zo);
+  } else if ((P.method == RCA_COLTX) == outer) {  // a column
+    dx = __dsub_rn(__ldg(P.Gt + e), px.xo);
+    dy = px.gy_c;
+    dz = __dsub_rn(__ldg(P.Gt + e + 2 * P.Nt), px.zo);
+  } else {  // a row
+    dx = px.gx_r;
+    dy = __dsub_rn(__ldg(P.Gr + e + P.Nr), px.yo);
+    dz = __dsub_rn(__ldg(P.Gr + e + 2 * P.Nr), px.zo);
   }
-  return (P.method == RCA_ROWTX) ? l : A::add(l, px.delay_ms);
 }
 
-__device__ __forceinline__ double inner_leg(const FastParams &P, const Pixel &px, int i) {
-  using A = Ar<double>;
-  double l;
-  if (P.method == TFM) {
-    l = leg_time(A::sub(P.Gr[i], px.xo), A::sub(P.Gr[i + P.Nr], px.yo), A::sub(P.Gr[i + 2 * P.Nr], px.zo), P.ocp);
-  } else if (P.method == RCA_COLTX) {
-    l = leg_time(px.gx_r, A::sub(P.Gr[i + P.Nr], px.yo), A::sub(P.Gr[i + 2 * P.Nr], px.zo), P.ocp);
-  } else {  // row-tx: inner = columns, carrying the delay
-    l = A::add(leg_time(A::sub(P.Gt[i], px.xo), px.gy_c, A::sub(P.Gt[i + 2 * P.Nt], px.zo), P.ocp), px.delay_ms);
-  }
-  return l;
+// Exact FP64 leg of outer or inner element e, including the delay on the leg
+// that carries it (TFM and col-tx: outer; row-tx: inner, the column).
+__device__ __forceinline__ double exact_leg(const FastParams &P, const Pixel &px, bool outer, int e) {
+  double dx, dy, dz;
+  leg_diffs(P, px, outer, e, dx, dy, dz);
+  const double l = leg_time(dx, dy, dz, P.ocp);
+  return (P.method == RCA_ROWTX) != outer ? __dadd_rn(l, px.delay_ms) : l;
 }
 
 // The reference's exact index of term (o, i): returns false when out of bounds.
 __device__ __noinline__ bool exact_index(const FastParams &P, const Pixel &px, int o, int i, int &k) {
   using A = Ar<double>;
-  double p = A::mul(A::add(outer_leg(P, px, o), inner_leg(P, px, i)), P.Fs);
+  double p = A::mul(A::add(exact_leg(P, px, true, o), exact_leg(P, px, false, i)), P.Fs);
   if (P.K > 0 && p > -1.0 && p < (double)P.K) {
     k = trunc_index(p);
     return true;
@@ -197,29 +201,6 @@ __device__ __forceinline__ int64_t ycol_outer(const FastParams &P, int n_in, int
 __device__ __forceinline__ int64_t ycol_inner(const FastParams &P, int i) { return (int64_t)i - P.ycol_i0; }
 __device__ __forceinline__ int64_t ycol(const FastParams &P, int n_in, int o, int i) {
   return ycol_outer(P, n_in, o) + ycol_inner(P, i);
-}
-
-// Coordinate differences between image point px and element e (outer or
-// inner), as the reference forms them for each method: TFM uses the element's
-// position; an RCA column (Gt) its x and z with the clamped y offset of the
-// column stripe, an RCA row (Gr) its y and z with the clamped x offset.
-__device__ __forceinline__ void leg_diffs(const FastParams &P, const Pixel &px, bool outer, int e, double &dx,
-                                          double &dy, double &dz) {
-  if (P.method == TFM) {
-    const double *G = outer ? P.Gt : P.Gr;
-    const int N = outer ? P.Nt : P.Nr;
-    dx = __ldg(G + e) - px.xo;
-    dy = __ldg(G + e + N) - px.yo;
-    dz = __ldg(G + e + 2 * N) - px.zo;
-  } else if ((P.method == RCA_COLTX) == outer) {  // a column
-    dx = __ldg(P.Gt + e) - px.xo;
-    dy = px.gy_c;
-    dz = __ldg(P.Gt + e + 2 * P.Nt) - px.zo;
-  } else {  // a row
-    dx = px.gx_r;
-    dy = __ldg(P.Gr + e + P.Nr) - px.yo;
-    dz = __ldg(P.Gr + e + 2 * P.Nr) - px.zo;
-  }
 }
 
 // Fixed-point leg: round(L * 2^fb) modulo 2^32, L = |d| * ocp * Fs + delay * Fs
@@ -290,20 +271,115 @@ struct TileShared {
   uint32_t *brel;  // [JC][nthreads]: the current chunk's inner legs, relative to base
 };
 
-// Exact partial sum of terms (o, i0 .. i0+jn-1): every index through the FP64
-// recomputation. Taken for the rare chunks holding an ambiguous or
-// out-of-range term, so the hot loop below stays free of calls.
+// ---------------------------------------------------------------------------
+// Gather: one tile of image points, every sample index by the reference's own
+// FP64 chain.
+//
+// trunc(RN(RN(a + b) * Fs)) costs three FP64 instructions per term (leg sum,
+// scale, truncation by adding 2^52 toward zero), which the FP64 pipe executes
+// beside the integer unit's addresses; in the low mantissa word the last one
+// leaves the sample number plus the column offset j * K inside the chunk. The
+// bounds test is one vote per chunk: rounded sums and products are monotone, so
+// the shortest and the longest legs decide exactly whether every term of the
+// chunk is in bounds.
+//
+// Bound (64x64 elements, K = 3000, 512x512 points, FP32 storage): 0.42 ms at 10
+// instructions per term and 0.71 of the issue slots; 6.5 of them are the three
+// FP64 operations, the 64-bit address, the load and half a packed add, about 2.5
+// the legs. The FP64 pipe is at 0.54 (its own limit for the terms alone would be
+// 0.17 ms), the L1 data pipe at 0.46. Fixed-point legs with an ambiguity test
+// and an FP64 fallback, the form this replaces, took 0.505 ms there, 0.069
+// against 0.037 for 32x32 elements and 256x256 points (no per-tile set-up with
+// block barriers here), 38.0 against 27.3 for the 128x128-element RCA volume.
+//
+// Layout: 8 inner legs and the 8 addends of the truncation in registers, the
+// outer legs in shared memory (a thread reads only its own: no barrier), two
+// groups of 4 outer x 8 inner gathers alternating. 16 inner legs with one or two
+// outer elements per group: 0.47 - 0.57 ms; 2 outer elements per group 0.48; one
+// group at a time 0.55; 96 registers (five blocks) 0.47 - 0.51.
+// ---------------------------------------------------------------------------
+
+constexpr int GATHER_JC = 8;  // inner elements per register chunk
+constexpr int GATHER_NO = 4;  // outer elements whose gathers are issued together
+
+// Raw bits of a gathered sample, and their value: the conversion waits for the
+// sample, so it belongs to the sum.
+__device__ __forceinline__ uint32_t load_bits(const float *p) { return __float_as_uint(__ldg(p)); }
+__device__ __forceinline__ uint32_t load_bits(const __nv_bfloat16 *p) {
+  return __ldg(reinterpret_cast<const unsigned short *>(p));
+}
+template <class YT>
+__device__ __forceinline__ float sample_of(uint32_t bits) {
+  return __uint_as_float(sizeof(YT) == 2 ? bits << 16 : bits);
+}
+
+// Issues the gathers of NO outer elements (legs a) x the chunk's inner elements
+// (FULL: all of them, else the first jn), all in bounds. yc: address of the
+// first term's column; the next outer element's is ystep bytes further.
+template <class YT, bool FULL, int NO>
+__device__ __forceinline__ void gather_issue(const FastParams &P, const double (&a)[NO], const double (&B)[GATHER_JC],
+                                             const double (&mag)[GATHER_JC], double Fs, const char *yc, int64_t ystep,
+                                             int jn, uint32_t (&y)[NO][GATHER_JC]) {
+#pragma unroll
+  for (int q = 0; q < NO; q++, yc += ystep) {
+#pragma unroll
+    for (int j = 0; j < GATHER_JC; j++) {
+      y[q][j] = 0;
+      const uint32_t k = (uint32_t)__double2loint(__dadd_rz(__dmul_rn(__dadd_rn(a[q], B[j]), Fs), mag[j]));
+      if ((FULL || j < jn) && gather_ok<float>(elem_addr<YT>(yc, k) - reinterpret_cast<const YT *>(P.Y), y_count(P), P.bad))
+        y[q][j] = load_bits(elem_addr<YT>(yc, k));
+    }
+  }
+}
+
+// Their sum, as a tree of packed pairs; weighted, w holds the chunk's
+// weights of the first outer element (shared memory, GATHER_JC per element).
+template <class YT, bool WEIGHTED, int NO>
+__device__ __forceinline__ float gather_sum(const uint32_t (&y)[NO][GATHER_JC], const float *w) {
+  constexpr int JP = GATHER_JC / 2;
+  uint64_t v[NO * JP];
+  auto pair = [&](int q, int j) { return pack_f32x2(sample_of<YT>(y[q][2 * j]), sample_of<YT>(y[q][2 * j + 1])); };
+#pragma unroll
+  for (int q = 0; q < NO; q++)
+#pragma unroll
+    for (int j = 0; j < JP; j += 2) {
+      uint64_t w0 = 0, w1 = 0;
+      if (WEIGHTED) {
+        const float4 w4 = *reinterpret_cast<const float4 *>(w + q * GATHER_JC + 2 * j);
+        w0 = pack_f32x2(w4.x, w4.y);
+        w1 = pack_f32x2(w4.z, w4.w);
+      }
+      if (!WEIGHTED) {
+        v[q * JP + j] = pair(q, j);
+        v[q * JP + j + 1] = pair(q, j + 1);
+      } else if (q == 0) {
+        v[j] = mul_f32x2(pair(q, j), w0);
+        v[j + 1] = mul_f32x2(pair(q, j + 1), w1);
+      } else {
+        v[j] = fma_f32x2(pair(q, j), w0, v[j]);
+        v[j + 1] = fma_f32x2(pair(q, j + 1), w1, v[j + 1]);
+      }
+    }
+#pragma unroll
+  for (int n = (WEIGHTED ? JP : NO * JP) / 2; n >= 1; n /= 2)
+#pragma unroll
+    for (int j = 0; j < n; j++) v[j] = add_f32x2(v[j], v[j + n]);
+  return lo_f32(v[0]) + hi_f32(v[0]);
+}
+
+// One outer element against a chunk, every term tested.
 template <class YT, bool WEIGHTED>
-__device__ __noinline__ float exact_partial(const FastParams &P, const Pixel &px, int o, int i0, int jn, int n_in,
-                                            unsigned int &oob) {
-  const YT *__restrict__ Y = reinterpret_cast<const YT *>(P.Y);
+__device__ __forceinline__ float gather_tested(const FastParams &P, double a, const double (&B)[GATHER_JC], double Fs,
+                                               double Kf, const char *yc, const float *w, int jn, unsigned int &oob) {
   float part = 0.0f;
-  for (int j = 0; j < jn; j++) {
-    int k;
-    const int64_t col = ycol(P, n_in, o, i0 + j);
-    if (exact_index(P, px, o, i0 + j, k)) {
-      const float y = gather_ok<float>(col * P.K + k, y_count(P), P.bad) ? load_sample(Y + col * P.K + k) : 0.0f;
-      part = WEIGHTED ? fmaf(__ldg(P.w + col), y, part) : part + y;
+#pragma unroll
+  for (int j = 0; j < GATHER_JC; j++) {
+    if (j >= jn) break;
+    const double p = __dmul_rn(__dadd_rn(a, B[j]), Fs);
+    if (p > -1.0 && p < Kf) {
+      const YT *e = reinterpret_cast<const YT *>(yc) + (j * P.K + trunc_index(p));
+      const float y = gather_ok<float>(e - reinterpret_cast<const YT *>(P.Y), y_count(P), P.bad) ? load_sample(e) : 0.0f;
+      part = WEIGHTED ? fmaf(w[j], y, part) : part + y;
     } else {
       oob++;
     }
@@ -311,185 +387,197 @@ __device__ __noinline__ float exact_partial(const FastParams &P, const Pixel &px
   return part;
 }
 
-// One outer element against a chunk of JN inner elements (JN = JC for full
-// chunks, so the unrolled body carries no per-term predicates). Gathers are
-// issued unconditionally: in an in-bounds tile every floor index, ambiguous
-// or not, lies inside its A-scan. Ambiguity is tracked as the minimum
-// fraction word; a chunk whose minimum falls in the band is recomputed. The
-// minimum runs as four interleaved chains, two terms per step (one
-// three-input minimum), and the packed sums as a tree, so no long dependency
-// chain holds the warp; one branch tests all NO outer elements.
-template <class YT, bool WEIGHTED, bool CHECKED, bool FULL, int JC, int NO>
-__device__ __forceinline__ float chunk_terms(const FastParams &P, const Pixel &px, const uint64_t (&B64)[JC],
-                                             const uint64_t (&A64)[NO], int o0, int i0, int jn, int n_in,
-                                             uint32_t amb_lo, unsigned int &oob) {
-  // NO outer elements x JC inner elements: all NO*JC gathers are issued before
-  // any (rare) call to the exact path, so they are in flight together.
-  const YT *__restrict__ Y = reinterpret_cast<const YT *>(P.Y);
-  const int64_t K = P.K;
-  constexpr int NM = JC < 4 ? JC : 4;  // independent minimum chains per outer element
-  float y[NO][JC];
-  uint32_t mlo[NO][NM];
-  unsigned int oob_chunk[NO];
-#pragma unroll
-  for (int q = 0; q < NO; q++) {
-    oob_chunk[q] = 0;
-#pragma unroll
-    for (int c = 0; c < NM; c++) mlo[q][c] = 0xffffffffu;
-#pragma unroll
-    for (int j = 0; j < JC; j++) {
-      y[q][j] = 0.0f;
-      if (FULL || j < jn) {
-        const uint64_t s = A64[q] + B64[j];
-        if (FULL && (j & 1)) {  // pairs: one three-input minimum per two terms
-          const uint32_t prev = (uint32_t)(A64[q] + B64[j - 1]);
-          mlo[q][(j >> 1) % NM] = min(mlo[q][(j >> 1) % NM], min(prev, (uint32_t)s));
-        } else if (!FULL) {
-          mlo[q][j % NM] = min(mlo[q][j % NM], (uint32_t)s);
-        }
-        const uint32_t off = (uint32_t)(s >> 32);
-        if (CHECKED) {
-          // Outside the ambiguity band the floor index is exact: [0, K) is in
-          // bounds, -1 means p in (-1, 0), i.e. sample 0 after truncation, and
-          // anything else is out of bounds.
-          const int64_t col0 = ycol(P, n_in, o0 + q, i0 + j) * K;
-          const int32_t kk = (int32_t)(off - (uint32_t)col0);  // floor index, exact modulo 2^32
-          if (kk >= 0 && kk < K) {
-            if (gather_ok<float>(col0 + kk, y_count(P), P.bad)) y[q][j] = load_sample(Y + col0 + kk);
-          } else if (kk == -1) {
-            y[q][j] = load_sample(Y + col0);
-          } else {
-            oob_chunk[q]++;
-          }
-        } else {
-          if (gather_ok<float>((int64_t)off, y_count(P), P.bad)) y[q][j] = load_sample(elem_addr(Y, off));
-        }
-      }
-    }
+// Bounds of a set of legs from their high words: the words as integers in the
+// legs' order (NaN above everything), widened to whole high words, so a set
+// costs four integer instructions per leg instead of FP64 comparisons.
+struct LegBounds {
+  int lo = INT_MAX, hi = INT_MIN;
+  __device__ __forceinline__ void add(double l) {
+    const int h = __double2hiint(l), key = h ^ ((h >> 31) & 0x7fffffff);
+    lo = min(lo, key);
+    hi = max(hi, key);
   }
-  float total = 0.0f;
-  float partq[NO];
-  uint32_t minlo[NO];
-#pragma unroll
-  for (int q = 0; q < NO; q++) {
-    minlo[q] = mlo[q][0];
-#pragma unroll
-    for (int c = 1; c < NM; c++) minlo[q] = min(minlo[q], mlo[q][c]);
-    float part = 0.0f;
-    if (WEIGHTED) {
-      const float *w = P.w + ycol(P, n_in, o0 + q, i0);
-      if (FULL && ((reinterpret_cast<uintptr_t>(w) & 15) == 0)) {
-        uint64_t acc2 = 0;  // (+0, +0)
-#pragma unroll
-        for (int j = 0; j < JC; j += 4) {
-          float4 w4 = __ldg(reinterpret_cast<const float4 *>(w + j));
-          acc2 = fma_f32x2(pack_f32x2(w4.x, w4.y), pack_f32x2(y[q][j], y[q][j + 1]), acc2);
-          acc2 = fma_f32x2(pack_f32x2(w4.z, w4.w), pack_f32x2(y[q][j + 2], y[q][j + 3]), acc2);
-        }
-        part = lo_f32(acc2) + hi_f32(acc2);
-      } else {
-#pragma unroll
-        for (int j = 0; j < JC; j++)
-          if (FULL || j < jn) part = fmaf(__ldg(w + j), y[q][j], part);
-      }
-    } else {
-      // packed FP32x2 adds: half the instructions; summed as a tree
-      uint64_t v[JC / 2];
-#pragma unroll
-      for (int j = 0; j < JC / 2; j++) v[j] = pack_f32x2(y[q][2 * j], y[q][2 * j + 1]);
-#pragma unroll
-      for (int w = JC / 4; w >= 1; w /= 2)
-#pragma unroll
-        for (int j = 0; j < w; j++) v[j] = add_f32x2(v[j], v[j + w]);
-      part = lo_f32(v[0]) + hi_f32(v[0]);
-    }
-    partq[q] = part;
-  }
-  uint32_t mm = minlo[0];
-#pragma unroll
-  for (int q = 1; q < NO; q++) mm = min(mm, minlo[q]);
-  if (mm < amb_lo) {
-#pragma unroll
-    for (int q = 0; q < NO; q++) {
-      if (minlo[q] < amb_lo) {
-        // this outer element's partial is replaced by the exact one (which counts its own OOB)
-        partq[q] = exact_partial<YT, WEIGHTED>(P, px, o0 + q, i0, jn, n_in, oob);
-      } else {
-        oob += oob_chunk[q];
-      }
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < NO; q++) oob += oob_chunk[q];
-  }
-#pragma unroll
-  for (int q = 0; q < NO; q++) total += partq[q];
-  return total;
+  __device__ __forceinline__ bool finite() const { return hi < 0x7ff00000 && lo > (int)0x800fffff; }
+  static __device__ __forceinline__ int word(int key) { return key ^ ((key >> 31) & 0x7fffffff); }
+  __device__ __forceinline__ double min_leg() const { return __hiloint2double(word(lo), lo < 0 ? -1 : 0); }
+  __device__ __forceinline__ double max_leg() const { return __hiloint2double(word(hi), hi < 0 ? 0 : -1); }
+};
+
+// The image point of this thread (inactive lanes repeat the tile's first point).
+__device__ __forceinline__ int64_t tile_point(const FastParams &P, int64_t tfi, int64_t tsi, bool &active) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lf = lane % P.wf, ls = lane / P.wf;
+  const int warps_f = P.tile_f / P.wf;
+  const int wfi = warp % warps_f, wsi = warp / warps_f;
+  const int64_t f = tfi * P.tile_f + wfi * P.wf + lf;
+  const int64_t s = tsi * P.tile_s + wsi * (32 / P.wf) + ls;
+  active = f < P.n_fast && s < P.n_slow;
+  return active ? s * P.n_fast + f : tsi * P.tile_s * P.n_fast + tfi * P.tile_f;
 }
 
-template <class YT, bool WEIGHTED, bool CHECKED, int JC>
-__device__ __forceinline__ void tile_loop(const FastParams &P, const Pixel &px, const TileShared &S, const FixFmt F,
-                                          double cfix, double dfixB, int tid, int nthr, int n_out, int n_in,
-                                          int i_lo, int i_hi, float &acc_s, float &acc_c, unsigned int &oob) {
-  const int64_t K = P.K;
-  for (int i0 = i_lo; i0 < i_hi; i0 += JC) {
-    const int jn = min(JC, i_hi - i0);
-    // the chunk's inner legs into this thread's shared slots, four at a time
-    // (all of them side by side in registers would crowd the gather loop)
-    bool bad = false;
-#pragma unroll 4
-    for (int j = 0; j < jn; j++) {
-      const int i = i0 + j;
-      double dx, dy, dz;
-      leg_diffs(P, px, false, i, dx, dy, dz);
-      const uint32_t r = leg_fix(dx, dy, dz, cfix, dfixB) - ((uint32_t)S.base[n_out + i] << F.fb);
-      bad |= r >= ((uint32_t)(S.ext[n_out + i] + 1) << F.fb);
-      S.brel[j * nthr + tid] = r;
-    }
-    uint64_t B64[JC];
+// The legs of one side of a method's term: a point element (TFM), a column or a
+// row of an RCA, read through its coordinate columns.
+enum LegKind : int { POINT, COLUMN, ROW };
+__host__ __device__ constexpr LegKind leg_kind(int method, bool outer) {
+  return method == TFM ? POINT : ((method == RCA_COLTX) == outer ? COLUMN : ROW);
+}
+template <int METHOD, bool OUTER>
+struct Legs {
+  static constexpr LegKind KIND = leg_kind(METHOD, OUTER);
+  static constexpr bool DELAYED = (METHOD == RCA_ROWTX) != OUTER;
+  const double *x, *y, *z;
+  __device__ __forceinline__ explicit Legs(const FastParams &P) {
+    const bool tx = KIND == COLUMN || (KIND == POINT && OUTER);
+    const int N = tx ? P.Nt : P.Nr;
+    x = tx ? P.Gt : P.Gr;
+    y = x + N;
+    z = y + N;
+  }
+  // The exact FP64 leg of element e (as exact_leg).
+  __device__ __forceinline__ double operator()(const FastParams &P, const Pixel &px, int e) const {
+    const double l = leg_time(KIND == ROW ? px.gx_r : __dsub_rn(__ldg(x + e), px.xo),
+                              KIND == COLUMN ? px.gy_c : __dsub_rn(__ldg(y + e), px.yo),
+                              __dsub_rn(__ldg(z + e), px.zo), P.ocp);
+    return DELAYED ? __dadd_rn(l, px.delay_ms) : l;
+  }
+};
+
+// One tile of image points (tile indices tfi along the fast axis, tsi along the
+// slow axis) with the frame described by P; smem_raw holds the legs of
+// P.out_block outer elements per thread. No thread reads another's legs, so
+// there is no barrier. Called by the one-frame kernel and by the persistent
+// batch kernel.
+template <class YT, bool WEIGHTED, int METHOD>
+__device__ __forceinline__ void gather_tile(const FastParams &P, int64_t tfi, int64_t tsi, unsigned char *smem_raw) {
+  __shared__ double s_mag[GATHER_JC];
+  if (threadIdx.x < GATHER_JC) s_mag[threadIdx.x] = 4503599627370496.0 + (double)(threadIdx.x * P.K);
+  __syncthreads();
+  const int nthr = blockDim.x;
+  double *tab = reinterpret_cast<double *>(smem_raw) + threadIdx.x;  // leg of outer element o0 + o: tab[o * nthr]
+  float *ws = reinterpret_cast<float *>(smem_raw + (size_t)P.out_block * nthr * sizeof(double));  // weights [o][GATHER_JC]
+  const int n_out = METHOD == RCA_ROWTX ? P.Nr : P.Nt, n_in = METHOD == RCA_ROWTX ? P.Nt : P.Nr;
+  const Legs<METHOD, true> outer(P);
+  const Legs<METHOD, false> inner(P);
+  const int i_lo = P.in_lo, i_hi = P.in_hi > 0 ? P.in_hi : n_in;
+  const int64_t ostride = P.ycol_o > 0 ? P.ycol_o : n_in;  // columns per outer element
+  bool active;
+  const int64_t no = tile_point(P, tfi, tsi, active);
+  Pixel px;
+  pixel_of(P, no, px);
+  // 2^52 + j * K, read from shared memory: as uniform values each use would move them to a register first
+  double mag[GATHER_JC];
 #pragma unroll
-    for (int j = 0; j < JC; j++) {
-      B64[j] = 0;
-      if (j < jn) {
-        const int i = i0 + j;
-        const uint32_t hi = (uint32_t)(ycol_inner(P, i) * K + S.base[n_out + i]);
-        B64[j] = ((uint64_t)S.brel[j * nthr + tid] << F.lo_shift) + ((uint64_t)hi << 32);
+  for (int j = 0; j < GATHER_JC; j++) mag[j] = s_mag[j];
+  const YT *Y = reinterpret_cast<const YT *>(P.Y);
+  const int64_t ystep = ostride * P.K * (int64_t)sizeof(YT);  // bytes between the columns of neighbouring outer elements
+  const double Kf = (double)P.K, Fs = P.Fs;
+  float acc_s = 0.0f, acc_c = 0.0f;
+  unsigned int oob = 0;
+  for (int o0 = 0; o0 < n_out; o0 += P.out_block) {
+    const int on = min(P.out_block, n_out - o0);
+    LegBounds bA;
+#pragma unroll 4
+    for (int o = 0; o < on; o++) {
+      const double l = outer(P, px, o0 + o);
+      tab[o * nthr] = l;
+      bA.add(l);
+    }
+    // no vote for a NaN leg, a negative Fs, or sample numbers beyond 32 bits
+    const bool fin = bA.finite() && P.Fs > 0.0 && P.K < (int64_t(1) << 28);
+    const double mnA = bA.min_leg(), mxA = bA.max_leg();
+    for (int i0 = i_lo; i0 < i_hi; i0 += GATHER_JC) {
+      const int jn = min(GATHER_JC, i_hi - i0);
+      double B[GATHER_JC];
+      LegBounds bB;
+#pragma unroll
+      for (int j = 0; j < GATHER_JC; j++) {
+        if (j >= jn) {
+          B[j] = B[0];  // past the last inner element: never gathered
+          continue;
+        }
+        B[j] = inner(P, px, i0 + j);
+        bB.add(B[j]);
       }
-    }
-    if (__any_sync(0xffffffffu, bad)) {
-      // an inner leg outside the tile's bound: this chunk through the exact path
-      for (int o = 0; o < n_out; o++)
-        neumaier(acc_s, acc_c, exact_partial<YT, WEIGHTED>(P, px, o, i0, jn, n_in, oob));
-      continue;
-    }
-    if (jn == JC) {
-      // compensation every four outer elements
+      const bool ok = fin && bB.finite();
+      const double mnB = bB.min_leg(), mxB = bB.max_leg();
+      const int64_t col = o0 * ostride + ycol_inner(P, i0);
+      const char *yc = reinterpret_cast<const char *>(Y + col * P.K);  // the chunk's first column, outer element o
+      const float *w = ws;                                            // and its weights
+      if (WEIGHTED) {
+        __syncthreads();  // the last chunk's weights are read
+        for (int e = threadIdx.x; e < on * GATHER_JC; e += nthr) {
+          const int j = e % GATHER_JC;
+          ws[e] = j < jn ? __ldg(P.w + col + e / GATHER_JC * ostride + j) : 0.0f;
+        }
+        __syncthreads();
+      }
+      const bool in = ok && __dmul_rn(__dadd_rn(mnA, mnB), Fs) >= 0.0 && __dmul_rn(__dadd_rn(mxA, mxB), Fs) < Kf;
       int o = 0;
-      for (; o + 4 <= n_out; o += 4) {
-        const uint64_t A2[2] = {((uint64_t)S.arel[o * nthr + tid] << F.lo_shift) + ((uint64_t)S.ahi[o] << 32),
-                                ((uint64_t)S.arel[(o + 1) * nthr + tid] << F.lo_shift) + ((uint64_t)S.ahi[o + 1] << 32)};
-        const float p0 = chunk_terms<YT, WEIGHTED, CHECKED, true, JC, 2>(P, px, B64, A2, o, i0, JC, n_in, F.amb_lo, oob);
-        const uint64_t A3[2] = {((uint64_t)S.arel[(o + 2) * nthr + tid] << F.lo_shift) + ((uint64_t)S.ahi[o + 2] << 32),
-                                ((uint64_t)S.arel[(o + 3) * nthr + tid] << F.lo_shift) + ((uint64_t)S.ahi[o + 3] << 32)};
-        const float p1 = chunk_terms<YT, WEIGHTED, CHECKED, true, JC, 2>(P, px, B64, A3, o + 2, i0, JC, n_in, F.amb_lo, oob);
-        neumaier(acc_s, acc_c, p0 + p1);
-      }
-      for (; o + 2 <= n_out; o += 2) {
-        const uint64_t A2[2] = {((uint64_t)S.arel[o * nthr + tid] << F.lo_shift) + ((uint64_t)S.ahi[o] << 32),
-                                ((uint64_t)S.arel[(o + 1) * nthr + tid] << F.lo_shift) + ((uint64_t)S.ahi[o + 1] << 32)};
-        neumaier(acc_s, acc_c, chunk_terms<YT, WEIGHTED, CHECKED, true, JC, 2>(P, px, B64, A2, o, i0, JC, n_in, F.amb_lo, oob));
-      }
-      for (; o < n_out; o++) {
-        const uint64_t A1[1] = {((uint64_t)S.arel[o * nthr + tid] << F.lo_shift) + ((uint64_t)S.ahi[o] << 32)};
-        neumaier(acc_s, acc_c, chunk_terms<YT, WEIGHTED, CHECKED, true, JC, 1>(P, px, B64, A1, o, i0, JC, n_in, F.amb_lo, oob));
-      }
-    } else {
-      for (int o = 0; o < n_out; o++) {
-        const uint64_t A1[1] = {((uint64_t)S.arel[o * nthr + tid] << F.lo_shift) + ((uint64_t)S.ahi[o] << 32)};
-        neumaier(acc_s, acc_c, chunk_terms<YT, WEIGHTED, CHECKED, false, JC, 1>(P, px, B64, A1, o, i0, jn, n_in, F.amb_lo, oob));
+      if (__all_sync(0xffffffffu, in)) {
+        constexpr int NO = GATHER_NO;
+        auto outer_legs = [&](int g, double(&a)[NO]) {
+#pragma unroll
+          for (int q = 0; q < NO; q++) a[q] = tab[(g + q) * nthr];
+        };
+        if (jn == GATHER_JC && on >= 2 * NO) {
+          // two groups alternate: the gathers of one are issued before the other is summed
+          uint32_t y0[NO][GATHER_JC], y1[NO][GATHER_JC];
+          auto issue = [&](int g, const char *c, uint32_t(&y)[NO][GATHER_JC]) {
+            double a[NO];
+            outer_legs(g, a);
+            gather_issue<YT, true, NO>(P, a, B, mag, Fs, c, ystep, jn, y);
+          };
+          issue(0, yc, y0);
+          for (; o + 2 * NO <= on; o += 2 * NO, w += 2 * NO * GATHER_JC) {
+            issue(o + NO, yc + NO * ystep, y1);
+            // FP32 storage compensates every 32 terms (whole-image error against FP64 3.2e-8 on the 64x64-element
+            // frame; 64 terms: 3.5e-8); BF16's own rounding is 10^4 times larger, so 64 do there (0.439 against 0.478 ms)
+            float p0 = gather_sum<YT, WEIGHTED, NO>(y0, w);
+            if (sizeof(YT) == 4) neumaier(acc_s, acc_c, p0);
+            yc += 2 * NO * ystep;
+            if (o + 4 * NO <= on) issue(o + 2 * NO, yc, y0);
+            const float p1 = gather_sum<YT, WEIGHTED, NO>(y1, w + NO * GATHER_JC);
+            neumaier(acc_s, acc_c, sizeof(YT) == 4 ? p1 : p0 + p1);
+          }
+        }
+        for (; o + NO <= on; o += NO, yc += NO * ystep, w += NO * GATHER_JC) {  // the last, partly filled chunk
+          double a[NO];
+          outer_legs(o, a);
+          uint32_t y[NO][GATHER_JC];
+          gather_issue<YT, false, NO>(P, a, B, mag, Fs, yc, ystep, jn, y);
+          neumaier(acc_s, acc_c, gather_sum<YT, WEIGHTED, NO>(y, w));
+        }
+        for (; o < on; o++, yc += ystep, w += GATHER_JC) {
+          const double a0[1] = {tab[o * nthr]};
+          uint32_t y[1][GATHER_JC];
+          gather_issue<YT, false, 1>(P, a0, B, mag, Fs, yc, ystep, jn, y);
+          neumaier(acc_s, acc_c, gather_sum<YT, WEIGHTED, 1>(y, w));
+        }
+      } else {
+        for (; o < on; o++, yc += ystep, w += GATHER_JC) {
+          const double a0[1] = {tab[o * nthr]};
+          const double lo = __dmul_rn(__dadd_rn(a0[0], mnB), Fs), hi = __dmul_rn(__dadd_rn(a0[0], mxB), Fs);
+          if (__all_sync(0xffffffffu, ok && lo >= 0.0 && hi < Kf)) {
+            uint32_t y[1][GATHER_JC];
+            gather_issue<YT, false, 1>(P, a0, B, mag, Fs, yc, ystep, jn, y);
+            neumaier(acc_s, acc_c, gather_sum<YT, WEIGHTED, 1>(y, w));
+          } else if (__all_sync(0xffffffffu, ok && (lo >= Kf || hi <= -1.0))) {
+            oob += jn;
+          } else {
+            neumaier(acc_s, acc_c, gather_tested<YT, WEIGHTED>(P, a0[0], B, Fs, Kf, yc, w, jn, oob));
+          }
+        }
       }
     }
   }
+  if (active) P.Im[no] = P.accumulate ? P.Im[no] + (acc_s + acc_c) : acc_s + acc_c;
+  add_count(P.oob, active ? oob : 0u);
+}
+
+template <class YT, bool WEIGHTED, int METHOD>
+__global__ void __launch_bounds__(256, 2) das_fast_kernel(const FastParams P) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  gather_tile<YT, WEIGHTED, METHOD>(P, blockIdx.x, (int64_t)blockIdx.y + P.slow_tile0, smem_raw);
 }
 
 // Everything a tile needs before its terms: the image point of each thread,
@@ -527,15 +615,8 @@ __device__ __forceinline__ void tile_setup(const FastParams &P, int64_t tfi, int
   S.red = reinterpret_cast<double *>(S.arel);
   S.stat = reinterpret_cast<int *>(S.red + nwarps * 8);
 
-  // ---- image point of this thread (inactive lanes repeat the tile's first point) ----
-  const int lf = lane % P.wf, ls = lane / P.wf;
-  const int warps_f = P.tile_f / P.wf;
-  const int wfi = warp % warps_f, wsi = warp / warps_f;
-  const int64_t f = tfi * P.tile_f + wfi * P.wf + lf;
-  const int64_t s = tsi * P.tile_s + wsi * (32 / P.wf) + ls;
-  const bool active = f < P.n_fast && s < P.n_slow;
-  const int64_t no = active ? s * P.n_fast + f : tsi * P.tile_s * P.n_fast + tfi * P.tile_f;
-
+  bool active;
+  const int64_t no = tile_point(P, tfi, tsi, active);
   Pixel px;
   pixel_of(P, no, px);
 
@@ -677,60 +758,6 @@ __device__ __forceinline__ void tile_setup(const FastParams &P, int64_t tfi, int
 
 }  // namespace
 
-// One tile of image points (tile indices tfi along the fast axis, tsi along
-// the slow axis) with the frame described by P; smem_raw holds the tile's
-// shared arrays (fast_smem_bytes). Called by the one-frame kernel and by the
-// persistent batch kernel.
-//
-// 1. The box bounding the tile's points and delays gives every element's leg
-//    range over the tile (leg_range): an integer base and extent per leg,
-//    and the tile's fixed-point format.
-// 2. Each point's outer legs are converted once (leg_fix) into shared memory,
-//    relative to their bases; each inner leg is converted once per point in
-//    the main loop. A leg outside its bound (which the box bound rules out up
-//    to rounding) sends its tile (outer) or chunk (inner) to the exact path
-//    before any gather depends on it.
-template <class YT, bool WEIGHTED, int JC>
-__device__ __forceinline__ void fast_tile(const FastParams &P, int64_t tfi, int64_t tsi, unsigned char *smem_raw) {
-  TileCtx T;
-  tile_setup(P, tfi, tsi, smem_raw, T);
-  float acc_s = 0.0f, acc_c = 0.0f;
-  unsigned int oob = 0;
-  const YT *__restrict__ Yp = reinterpret_cast<const YT *>(P.Y);
-  const Pixel px = T.px;  // a copy for the calls that take it by reference
-  if (T.exact_tile) {
-    // every term through the exact FP64 index
-    for (int o = 0; o < T.n_out; o++) {
-      float part = 0.0f;
-      for (int i = T.i_lo; i < T.i_hi; i++) {
-        int k;
-        const int64_t col = ycol(P, T.n_in, o, i);
-        if (exact_index(P, px, o, i, k)) {
-          float y = load_sample(Yp + col * P.K + k);
-          part = WEIGHTED ? fmaf(__ldg(P.w + col), y, part) : part + y;
-        } else {
-          oob++;
-        }
-      }
-      neumaier(acc_s, acc_c, part);
-    }
-  } else if (T.in_bounds) {
-    tile_loop<YT, WEIGHTED, false, JC>(P, px, T.S, T.F, T.cfix, T.dfixB, T.tid, T.nthr, T.n_out, T.n_in, T.i_lo,
-                                       T.i_hi, acc_s, acc_c, oob);
-  } else {
-    tile_loop<YT, WEIGHTED, true, JC>(P, px, T.S, T.F, T.cfix, T.dfixB, T.tid, T.nthr, T.n_out, T.n_in, T.i_lo,
-                                      T.i_hi, acc_s, acc_c, oob);
-  }
-  if (T.active) P.Im[T.no] = P.accumulate ? P.Im[T.no] + (acc_s + acc_c) : acc_s + acc_c;
-  add_count(P.oob, T.active ? oob : 0u);
-}
-
-template <class YT, bool WEIGHTED, int JC>
-__global__ void __launch_bounds__(256, 2) das_fast_kernel(const FastParams P) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  fast_tile<YT, WEIGHTED, JC>(P, blockIdx.x, (int64_t)blockIdx.y + P.slow_tile0, smem_raw);
-}
-
 // Persistent batch kernel: CTAs take (frame, tile) work items from a queue
 // (items sorted by decreasing cost on the host) until it is empty. The frame
 // descriptor is staged in shared memory; every frame's tile has blockDim.x
@@ -750,8 +777,9 @@ __global__ void __launch_bounds__(128, 3) das_batch_kernel(const FastParams *__r
     const int4 w = items[it];
     if (threadIdx.x == 0) sP = frames[w.x];
     __syncthreads();
-    if (sP.jc == 8) fast_tile<YT, false, 8>(sP, w.y, w.z, smem_raw);
-    else fast_tile<YT, false, 16>(sP, w.y, w.z, smem_raw);
+    if (sP.method == TFM) gather_tile<YT, false, TFM>(sP, w.y, w.z, smem_raw);
+    else if (sP.method == RCA_COLTX) gather_tile<YT, false, RCA_COLTX>(sP, w.y, w.z, smem_raw);
+    else gather_tile<YT, false, RCA_ROWTX>(sP, w.y, w.z, smem_raw);
     __syncthreads();
   }
 }
@@ -805,6 +833,10 @@ size_t fast_smem_bytes(const FastParams &P, int nthr) {
   return fast_smem_bytes_dev(P, n_out, n_in, nthr);
 }
 
+size_t gather_smem_bytes(const FastParams &P, int nthr) {
+  return (size_t)P.out_block * (nthr * sizeof(double) + (P.w ? GATHER_JC * sizeof(float) : 0));
+}
+
 template <class YT, bool W>
 static cudaError_t launch_fast_t(const FastParams &P, cudaStream_t st) {
   if (P.method == SAFT) {
@@ -814,8 +846,10 @@ static cudaError_t launch_fast_t(const FastParams &P, cudaStream_t st) {
     return cudaGetLastError();
   }
   const int nthr = P.tile_f * P.tile_s;
-  const size_t smem = fast_smem_bytes(P, nthr);
-  auto kern = (P.jc == 8) ? das_fast_kernel<YT, W, 8> : das_fast_kernel<YT, W, 16>;
+  const size_t smem = gather_smem_bytes(P, nthr);
+  auto kern = P.method == TFM         ? das_fast_kernel<YT, W, TFM>
+              : P.method == RCA_COLTX ? das_fast_kernel<YT, W, RCA_COLTX>
+                                      : das_fast_kernel<YT, W, RCA_ROWTX>;
   cudaError_t e = ensure_smem(kern, smem);
   if (e != cudaSuccess) return e;
   const int64_t gx = (P.n_fast + P.tile_f - 1) / P.tile_f;

@@ -25,7 +25,8 @@ struct FastParams {
   // image tiling: point n = s*n_fast + f
   int64_t n_fast, n_slow;
   int tile_f, tile_s, wf;  // tile extents; warp lanes along the fast axis
-  int jc;                  // inner elements per register chunk: 8 or 16
+  int out_block;           // gathers: outer elements whose legs are tabled at a time
+  int jc;                  // scatter: inner elements per window batch, 8 or 16
   int64_t slow_tile0, slow_tile1;  // slow-tile range of this launch
   int64_t no0, no1;                // point range (SAFT launches)
   // inner-element range [in_lo, in_hi) of this launch (in_hi == 0: all inner
@@ -40,7 +41,25 @@ struct FastParams {
   unsigned long long *bad;  // gather index violations (bounds-checked builds)
 };
 
-size_t fast_smem_bytes(const FastParams &P, int nthr);
+// Points along the fast axis of a gather warp's patch of the image: on a hinted
+// TFM grid 4 (depth) x 8, else 8 x 4 (see plain_patch_f).
+inline int gather_patch_f(int method, bool hint, int tile_s) {
+  if (!hint) return 32;
+  return method == 1 /* TFM */ && tile_s % 8 == 0 ? 4 : 8;
+}
+// Outer elements tabled at a time, in even blocks. Every block recomputes the
+// inner legs; 52 x 128 threads x 8 bytes leave room for four tiles on an SM. One
+// block of up to 64 pays for the fourth (64x64 elements: 0.417 against 0.425 ms,
+// 61x47: 0.173 against 0.192), two of 64 do not (128 outer elements: 1.02
+// against 0.91 ms with three of 44), nor do tiles of the persistent batch or
+// weighted ones, whose weights share the table's space (0.544 against 0.521).
+inline int gather_out_block(int n_out, bool single) {
+  if (single && n_out <= 64) return n_out > 0 ? n_out : 1;
+  const int n = (n_out + 51) / 52;
+  return n > 0 ? ((n_out + n - 1) / n + 3) / 4 * 4 : 4;
+}
+size_t fast_smem_bytes(const FastParams &P, int nthr);    // tile arrays of the scatter
+size_t gather_smem_bytes(const FastParams &P, int nthr);  // leg table of the gather (P.out_block)
 cudaError_t launch_fast(const FastParams &P, bool bf16, cudaStream_t st);
 // Adjoint on the forward's tiles: Ya[k(n,c), c] += w[c] * X[n] (FP32 A-scans;
 // P.w may be NULL). Adds into Ya, which the caller zeroes first.

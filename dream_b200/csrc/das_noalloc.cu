@@ -107,11 +107,11 @@ extern "C" int dream_das_batch_run_noalloc(const dream_das_frame *fr, int n_fram
     const int r = batch_frame_params(fr[f], F);
     if (r) return r;
     F.oob = d_oob;
-    smem = std::max(smem, fast_smem_bytes(F, 128));
+    if (fast_smem_bytes(F, 128) > 220 * 1024)
+      return set_last_error(DREAM_ERR_UNSUPPORTED, "a frame has too many outer elements for the batch kernel");
+    smem = std::max(smem, gather_smem_bytes(F, 128));
     order[f] = f;
   }
-  if (smem > 220 * 1024)
-    return set_last_error(DREAM_ERR_UNSUPPORTED, "a frame has too many outer elements for the batch kernel");
   // largest per-tile cost first (as dream_das_batch_create)
   std::stable_sort(order, order + n_frames, [&](int a, int b) {
     return (double)T[a].Nt * T[a].Nr > (double)T[b].Nt * T[b].Nr;
