@@ -11,15 +11,23 @@
 // bit for bit; FFTW's fftconv_p differs from it by rounding only.
 //
 // Layout. A CTA owns 4 warps x 32 lanes x R consecutive outputs of one
-// column; its window of A (outputs + B_M - 1 samples, zero outside the
-// column) and B are staged in shared memory. Lane l of warp w holds outputs
-// k = k_w + R*l + r. Stepping j downwards, lane l needs A[k_w + R*l + r - j]:
-// a window of R samples that slides by one per step. Steps go in groups of
-// R: the lane loads the group's R new A samples and R B samples (broadcasts)
-// up front, then does R x R products and adds from registers, so the only
-// serial latency is each output's FP64 add (8 cycles). A warp skips the
-// steps in which all its outputs would only meet samples outside the column
-// (the triangle ends of a long-by-long convolution).
+// column; its window of A (outputs + B_M - 1 samples, zero outside the column)
+// and B, reversed, are staged in shared memory. Lane l of warp w holds outputs
+// k = k_w + R*l + r. Stepping j downwards, lane l needs A[k_w + R*l + r - j]: a
+// window of R samples that slides by one per step, so a step is one new A
+// sample, one B sample (a broadcast) and R products and adds. R is odd, which
+// puts the 32 lanes' samples in distinct banks with no padding, so every
+// shared-memory read has a constant offset. The samples live in a ring of P
+// registers, refilled P - R steps ahead of their use; P steps make one trip,
+// after which every ring position has its old role. A warp skips the steps in
+// which all its outputs would only meet samples outside the column (the
+// triangle ends of a long-by-long convolution).
+//
+// Bound: the FP64 pipe, a product and an add per term (they must not fuse), at
+// 0.86 of its rate. Full-matrix-capture synthesis of 101 elements (10201 columns
+// 2000 * 2000, then * 150; 4.7e10 terms) 6.2 ms against 5.3 at the pipe's rate;
+// with 64-bit clamped indices, a padded window and three rotating buffers (226
+// registers) it took 12.3.
 //
 // '+=' / '-=' add into existing values; out-of-column terms then contribute
 // the exact neutral element (-0 for +=, +0 for -=), so a stored -0 stays -0
@@ -39,21 +47,19 @@
 namespace dream {
 namespace {
 
-constexpr int CONV_WARPS = 4;  // small CTAs: long pulses leave few tiles per column
-constexpr int CONV_R = 8;                                   // outputs per lane
-constexpr int CONV_T = CONV_WARPS * 32 * CONV_R;            // outputs per CTA
-constexpr int64_t CONV_LMAX = 8192;                         // B samples staged in shared memory
+constexpr int CONV_WARPS = 4;         // small CTAs: long pulses leave few tiles per column
+constexpr int64_t CONV_LMAX = 8192;   // B samples staged in shared memory
+// R outputs per lane (odd); ring of P A samples = steps per trip; B samples read ahead (divides P)
+constexpr int conv_p(int R) { return R + 3; }
+constexpr int conv_y(int R) { return conv_p(R) / 2; }
+constexpr int conv_t(int R) { return CONV_WARPS * 32 * R; }  // outputs per CTA
 
-// A-window slots: CONV_T + L samples plus 2R read ahead by the last groups.
-__host__ __device__ constexpr int64_t conv_window(int64_t L) { return CONV_T + L + 2 * CONV_R; }
+// B slots (L samples, then those read ahead by the last trip) and A-window slots.
+constexpr int64_t conv_b_slots(int R, int64_t L) { return L + conv_p(R) + conv_y(R); }
+constexpr int64_t conv_window(int R, int64_t L) { return conv_t(R) + L + 2 * conv_p(R); }
 
-// Shared-memory position of window sample q: one pad slot per 16 samples, so
-// the 32 lanes' reads at a stride of R samples fall in distinct banks (two
-// wavefronts per warp, the minimum for 8-byte values).
-__host__ __device__ constexpr int64_t conv_sw(int64_t q) { return q + (q >> 4); }
-
-__host__ __device__ constexpr size_t conv_smem_bytes(int64_t L) {
-  return (size_t)(L + conv_sw(conv_window(L)) + 1) * sizeof(double);  // B, then the A window
+constexpr size_t conv_smem_bytes(int R, int64_t L) {
+  return (size_t)(conv_b_slots(R, L) + conv_window(R, L)) * sizeof(double);
 }
 
 template <int MODE>
@@ -61,26 +67,27 @@ __device__ __forceinline__ double conv_acc(double acc, double prod) {
   return MODE == 2 ? __dsub_rn(acc, prod) : __dadd_rn(acc, prod);
 }
 
-// R steps of R outputs: acc[r] (op)= A[i0 + r + s0 + u] * B[L-1-s0-u] for
-// u = 0..R-1 in that order, with the A samples in cur (t < R) and nxt.
-// FULL groups have all R steps inside [s0, s_end).
-template <int MODE, bool FULL>
-__device__ __forceinline__ void conv_group(double (&acc)[CONV_R], const double (&cur)[CONV_R],
-                                           const double (&nxt)[CONV_R], const double (&yv)[CONV_R], int64_t s0,
-                                           int64_t s_end, int64_t i0, int64_t M, double neutral) {
+// One trip: steps 0 .. P - 1 (PART: the first n of them) from the lane's A
+// samples xp and the B samples yp; X holds samples 0 .. P - 1, Y the first
+// B samples. TEST: sample t of the trip is A[i0 + t]; products of samples
+// outside [0, M) become `neutral`.
+template <int MODE, int R, bool PART, bool TEST>
+__device__ __forceinline__ void conv_trip(double (&acc)[R], double (&X)[conv_p(R)], double (&Y)[conv_y(R)],
+                                          const double *xp, const double *yp, int n, int64_t i0, int64_t M,
+                                          double neutral) {
+  constexpr int CP = conv_p(R), CY = conv_y(R);
 #pragma unroll
-  for (int u = 0; u < CONV_R; u++) {
-    if (!FULL && s0 + u >= s_end) break;  // uniform across the warp
+  for (int u = 0; u < CP; u++) {
+    if (PART && u >= n) break;  // uniform across the warp
+    const double y = Y[u % CY];
+    Y[u % CY] = yp[u + CY];
 #pragma unroll
-    for (int r = 0; r < CONV_R; r++) {
-      const double xv = (r + u < CONV_R) ? cur[r + u] : nxt[r + u - CONV_R];
-      double prod = __dmul_rn(xv, yv[u]);
-      if (MODE != 0) {
-        const int64_t i = i0 + r + s0 + u;
-        if (i < 0 || i >= M) prod = neutral;
-      }
+    for (int r = 0; r < R; r++) {
+      double prod = __dmul_rn(X[(u + r) % CP], y);
+      if (TEST && (i0 + u + r < 0 || i0 + u + r >= M)) prod = neutral;
       acc[r] = conv_acc<MODE>(acc[r], prod);
     }
+    X[u] = xp[u + CP];
   }
 }
 
@@ -97,87 +104,61 @@ __device__ __forceinline__ int64_t centre_out_tile(int64_t y, int64_t n) {
 // Column n of the output convolves A column n % na with B column n / nb
 // (na = N, nb = 1 for fftconv_p / conv_p; the full-matrix-capture synthesis
 // pairs every receive column with every transmit column).
-template <int MODE>
+template <int MODE, int R>
 __global__ void __launch_bounds__(CONV_WARPS * 32) conv_p_kernel(const double *__restrict__ A, int64_t M, int64_t N,
                                                                   const double *__restrict__ B, int64_t L,
                                                                   int64_t ldb, double *__restrict__ Y, int64_t NY,
-                                                                  int64_t na, int64_t nb) {
+                                                                  int64_t tiles, int64_t na, int64_t nb) {
+  constexpr int CP = conv_p(R), CY = conv_y(R);
   extern __shared__ __align__(16) double conv_sm[];
-  double *ys = conv_sm;      // [L]
-  double *xs = conv_sm + L;  // xs[conv_sw(q)] = A[k_cta - (L - 1) + q] (0 outside the column)
+  double *ys = conv_sm;                    // ys[s] = B[L - 1 - s]
+  double *xs = conv_sm + conv_b_slots(R, L);  // xs[q] = A[k_cta - (L - 1) + q] (0 outside the column)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t k_cta = centre_out_tile(blockIdx.y, gridDim.y) * CONV_T;
-  const int64_t base = k_cta - (L - 1);
-  const int64_t W = conv_window(L);
+  const int W = (int)conv_window(R, L), Li = (int)L;
   const double neutral = MODE == 2 ? 0.0 : -0.0;
-  for (int64_t n = blockIdx.x; n < N; n += gridDim.x) {
-    const double *x = A + (n % na) * M;
-    const double *y = B + (n / nb) * ldb;
-    double *z = Y + n * NY;
-    __syncthreads();  // the previous column's window is no longer read
-    for (int64_t q = tid; q < L; q += blockDim.x) ys[q] = y[q];
-    for (int64_t q = tid; q < W; q += blockDim.x) {
-      const int64_t i = base + q;
-      xs[conv_sw(q)] = (i >= 0 && i < M) ? x[i] : 0.0;
-    }
-    __syncthreads();
-    const int q0 = warp * 32 * CONV_R + CONV_R * lane;  // window start of this lane at step s = 0
-    // step s = L-1-j: output k_r takes A[i], i = base + q0 + r + s (xs index q0 + r + s).
-    // Steps where every output of the warp sees only samples outside the
-    // column contribute nothing (neutral terms) and are skipped: the warp's
-    // samples span i in [k_w - (L-1) + s, k_w + 32R - 1 - (L-1) + s].
-    const int64_t k_w = k_cta + warp * 32 * CONV_R;
-    const int64_t s_begin = std::max<int64_t>(0, (L - 1) - (k_w + 32 * CONV_R - 1));
-    const int64_t s_end = std::min<int64_t>(L, M + (L - 1) - k_w);
-    // group of R steps starting at s0: lane sample t (0 <= t < 2R) is
-    // window sample q0 + s0 + t; the B samples are ys[L-1-s0-u]
-    auto xsamp = [&](int64_t t) { return xs[conv_sw(q0 + t)]; };
-    auto bsamp = [&](int64_t s) { return ys[std::max<int64_t>(L - 1 - s, 0)]; };  // clamped past the end, unused
-    // A samples in three buffers (the group's, the next group's, the one after
-    // being loaded), B samples in two; six groups per loop trip make every
-    // buffer's role fixed, so nothing is copied between groups.
-    double acc[CONV_R], X0[CONV_R], X1[CONV_R], X2[CONV_R], Y0[CONV_R], Y1[CONV_R];
-#pragma unroll
-    for (int r = 0; r < CONV_R; r++) {
-      const int64_t k = k_cta + q0 + r;
-      acc[r] = MODE == 0 ? 0.0 : (k < NY ? z[k] : 0.0);
-      X0[r] = xsamp(s_begin + r);
-      X1[r] = xsamp(s_begin + CONV_R + r);
-      Y0[r] = bsamp(s_begin + r);
-    }
-    // One group: the following group's samples are loaded first (they do not
-    // depend on the sums, so their latency overlaps this group's arithmetic),
-    // then R x R products and adds; only each output's FP64 add is serial.
-    auto group = [&](int64_t s0, const double(&cur)[CONV_R], const double(&nxt)[CONV_R], double(&load)[CONV_R],
-                     const double(&yv)[CONV_R], double(&yload)[CONV_R]) {
-#pragma unroll
-      for (int u = 0; u < CONV_R; u++) {
-        load[u] = xsamp(std::min<int64_t>(s0 + 2 * CONV_R + u, W - 1 - q0));
-        yload[u] = bsamp(s0 + CONV_R + u);
+  for (int64_t tile = blockIdx.y; tile < tiles; tile += gridDim.y) {
+    const int64_t k_cta = centre_out_tile(tile, tiles) * conv_t(R);
+    const int64_t base = k_cta - (L - 1);
+    // Step s takes sample base + q0 + r + s for output r. Steps where the warp's
+    // samples, base + w0 + s .. base + w0 + 32R - 1 + s, all fall outside the
+    // column contribute nothing and are skipped.
+    const int w0 = warp * 32 * R, q0 = w0 + R * lane;
+    const int64_t k_w = k_cta + w0;
+    const int s_begin = (int)std::max<int64_t>(0, (L - 1) - (k_w + 32 * R - 1));
+    const int s_end = (int)std::max<int64_t>(s_begin, std::min<int64_t>(L, M + (L - 1) - k_w));
+    for (int64_t n = blockIdx.x; n < N; n += gridDim.x) {
+      const double *x = A + (n % na) * M;
+      const double *y = B + (n / nb) * ldb;
+      double *z = Y + n * NY;
+      __syncthreads();  // the previous column's window is no longer read
+      for (int q = tid; q < (int)conv_b_slots(R, L); q += CONV_WARPS * 32) ys[q] = q < Li ? y[Li - 1 - q] : 0.0;
+      for (int q = tid; q < W; q += CONV_WARPS * 32) {
+        const int64_t i = base + q;
+        xs[q] = (i >= 0 && i < M) ? x[i] : 0.0;
       }
-      if (s0 + CONV_R <= s_end)  // a full group: no exit test between the steps
-        conv_group<MODE, true>(acc, cur, nxt, yv, s0, s_end, base + q0, M, neutral);
-      else
-        conv_group<MODE, false>(acc, cur, nxt, yv, s0, s_end, base + q0, M, neutral);
-    };
-    for (int64_t s0 = s_begin; s0 < s_end;) {
-      group(s0, X0, X1, X2, Y0, Y1);
-      if ((s0 += CONV_R) >= s_end) break;
-      group(s0, X1, X2, X0, Y1, Y0);
-      if ((s0 += CONV_R) >= s_end) break;
-      group(s0, X2, X0, X1, Y0, Y1);
-      if ((s0 += CONV_R) >= s_end) break;
-      group(s0, X0, X1, X2, Y1, Y0);
-      if ((s0 += CONV_R) >= s_end) break;
-      group(s0, X1, X2, X0, Y0, Y1);
-      if ((s0 += CONV_R) >= s_end) break;
-      group(s0, X2, X0, X1, Y1, Y0);
-      s0 += CONV_R;
-    }
+      __syncthreads();
+      const double *xp = xs + q0 + s_begin, *yp = ys + s_begin;
+      double acc[R], X[CP], Yb[CY];
 #pragma unroll
-    for (int r = 0; r < CONV_R; r++) {
-      const int64_t k = k_cta + q0 + r;
-      if (k < NY) z[k] = acc[r];
+      for (int r = 0; r < R; r++) acc[r] = (MODE != 0 && k_cta + q0 + r < NY) ? z[k_cta + q0 + r] : 0.0;
+#pragma unroll
+      for (int t = 0; t < CP; t++) X[t] = xp[t];
+#pragma unroll
+      for (int t = 0; t < CY; t++) Yb[t] = yp[t];
+      int left = s_end - s_begin;
+      int64_t i_w = base + w0 + s_begin;  // the warp's first sample of the trip
+      for (; left >= CP; left -= CP, xp += CP, yp += CP, i_w += CP) {
+        if (MODE != 0 && (i_w < 0 || i_w + 32 * R + CP > M))
+          conv_trip<MODE, R, false, true>(acc, X, Yb, xp, yp, CP, i_w + R * lane, M, neutral);
+        else
+          conv_trip<MODE, R, false, false>(acc, X, Yb, xp, yp, CP, 0, M, neutral);
+      }
+      conv_trip<MODE, R, true, MODE != 0>(acc, X, Yb, xp, yp, left, i_w + R * lane, M, neutral);
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const int64_t k = k_cta + q0 + r;
+        if (k < NY) z[k] = acc[r];
+      }
     }
   }
 }
@@ -205,14 +186,21 @@ template <int MODE>
 cudaError_t launch_mode(const double *A, int64_t M, int64_t N, const double *B, int64_t L, int64_t ldb, double *Y,
                         int64_t NY, cudaStream_t st, int64_t na, int64_t nb) {
   const unsigned gy = (unsigned)std::min<int64_t>(N, 65535);
-  if (L <= CONV_LMAX && (NY + CONV_T - 1) / CONV_T <= 65535) {
-    const size_t smem = conv_smem_bytes(L);
-    cudaError_t e = ensure_smem(conv_p_kernel<MODE>, smem);
+  // 7 outputs per lane; 5 where that leaves few tiles per SM (2000-sample columns * 2000: 101 columns 0.083 against
+  // 0.099 ms, 1024 and more columns alike) and B is short enough that shared memory does not decide (8000 samples
+  // x 16 columns of 20000: 0.50 against 0.40)
+  const int64_t tiles7 = N * ((NY + conv_t(7) - 1) / conv_t(7));
+  const int R = (tiles7 < 4096 && L <= 4096) ? 5 : 7;
+  const int64_t gt = (NY + conv_t(R) - 1) / conv_t(R);
+  if (L <= CONV_LMAX) {
+    const size_t smem = conv_smem_bytes(R, L);
+    auto kern = R == 5 ? conv_p_kernel<MODE, 5> : conv_p_kernel<MODE, 7>;
+    cudaError_t e = ensure_smem(kern, smem);
     if (e != cudaSuccess) return e;
     // x: columns (fastest, so every column's middle tile launches before any
     // column's edge tiles), y: tiles in centre-out order
-    dim3 grid((unsigned)std::min<int64_t>(N, 1 << 30), (unsigned)((NY + CONV_T - 1) / CONV_T));
-    conv_p_kernel<MODE><<<grid, CONV_WARPS * 32, smem, st>>>(A, M, N, B, L, ldb, Y, NY, na, nb);
+    dim3 grid((unsigned)std::min<int64_t>(N, 1 << 30), (unsigned)std::min<int64_t>(gt, 65535));
+    kern<<<grid, CONV_WARPS * 32, smem, st>>>(A, M, N, B, L, ldb, Y, NY, gt, na, nb);
   } else {
     dim3 grid((unsigned)((NY + 255) / 256), gy);
     conv_p_global_kernel<MODE><<<grid, 256, 0, st>>>(A, M, N, B, L, ldb, Y, NY, na, nb);
