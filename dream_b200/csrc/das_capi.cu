@@ -338,34 +338,26 @@ int zero_length_ascans(dream_das_plan *p, void *dIm, unsigned long long *doob, c
   return 0;
 }
 
-// Tile of the operator's adjoint: the user's, or the largest CTA whose
-// outer-leg table (n_out x threads x 4 B) fits in 96 KB, 16 x 8 points on a
-// hinted grid (8 x 32 for frames of fewer points than two waves of 128-point
-// tiles, whose set-up then serves twice the points) and 256 consecutive points
-// otherwise. TFM on a hinted grid: 8 x 32 points, long along the slow axis,
-// where a column's sample window grows slowest relative to the tile's terms
-// (64x64-element TFM frame 1.25 -> 1.20 ms, 32x32-element CG configuration
-// 0.130 -> 0.120 ms, against 16 x 8). RCA volumes keep the short tile: 32
-// points along their slow axis spread a stripe's leg beyond the window
-// (128x128 frame: 108.7 against 81.7 ms).
+// Tile of the operator's adjoint: the user's, or on a hinted TFM grid 16 x 16
+// points (64x64 elements, 512x512 points 0.80 ms, 37x53 elements 0.35; 8 x 32
+// points 0.79 and 0.46), on an RCA volume 8 x 16, whose windows grow fastest with
+// the tile (128x128 elements, 128x128x256 points 61.4 ms; 8 x 8 93.9, 16 x 8
+// 81), on both 8 x 8 where that would leave SMs without a tile (64x64 elements,
+// 150x125 points 0.32 against 0.57 ms); 256 consecutive points without a hint.
 void scatter_tile(const dream_das_plan *p, FastParams &F) {
-  const int n_out = (F.method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt;
   const bool hint = p->n_fast > 0;
-  F.wf = hint ? 8 : 32;
   if (p->tile_f > 0) {
     F.tile_f = p->tile_f;
     F.tile_s = p->tile_s;
-    return;
+  } else if (hint) {
+    F.tile_f = F.method == DREAM_DAS_TFM ? 16 : 8;
+    F.tile_s = 16;
+    if (p->No < (int64_t)p->sm_count * F.tile_f * F.tile_s) F.tile_f = F.tile_s = 8;
+  } else {
+    F.tile_f = 256;
+    F.tile_s = 1;
   }
-  const bool small = hint && p->No < (int64_t)p->sm_count * 8 * 128;
-  int nthr = (hint && !small) ? 128 : 256;
-  while (nthr > 32 && (size_t)n_out * nthr * 4 > 96 * 1024) nthr >>= 1;
-  F.tile_f = !hint ? nthr : (small ? 8 : (nthr >= 64 ? 16 : 8));
-  F.tile_s = nthr / F.tile_f;
-  if (hint && F.method == DREAM_DAS_TFM && (size_t)n_out * 256 * 4 <= 96 * 1024) {
-    F.tile_f = 8;
-    F.tile_s = 32;
-  }
+  F.wf = hint ? 8 : 32;
 }
 
 // Tile of the gathers: the user's, or 128 points, 8 x 16 on a TFM grid and 16 x
@@ -382,10 +374,9 @@ void gather_tile(const dream_das_plan *p, int method, int &tf, int &ts, int &wf)
   wf = gather_patch_f(method, hint, ts);
 }
 
-// Grid axes, chunk and adjoint tile of the FP32/BF16-storage kernels for plan p
-// (F.method, Nt, Nr, No must be set).
-int tile_params(const dream_das_plan *p, FastParams &F, int jc) {
-  F.jc = jc ? jc : (p->jc ? p->jc : 16);
+// Grid axes of the FP32/BF16-storage kernels for plan p, and its refusal of
+// frames with too many elements (F.method, Nt, Nr, No must be set).
+int grid_params(const dream_das_plan *p, FastParams &F) {
   if (p->n_fast > 0) {
     F.n_fast = p->n_fast;
     F.n_slow = p->No / p->n_fast;
@@ -393,14 +384,18 @@ int tile_params(const dream_das_plan *p, FastParams &F, int jc) {
     F.n_fast = p->No;
     F.n_slow = 1;
   }
-  scatter_tile(p, F);
-  if (fast_smem_bytes(F, F.tile_f * F.tile_s) > 220 * 1024)
+  const int n_out = (F.method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt;
+  const int n_in = (F.method == DREAM_DAS_RCA_ROWTX) ? F.Nt : F.Nr;
+  int nthr = 256;  // automatic tiles shrink with the outer elements; a tile set by the caller does not
+  while (nthr > 32 && (size_t)n_out * nthr * 4 > 96 * 1024) nthr >>= 1;
+  if (too_many_elements(n_out, n_in, p->tile_f > 0 ? p->tile_f * p->tile_s : nthr))
     return fail(DREAM_ERR_UNSUPPORTED, "too many elements on the outer loop for the FP32/BF16 storage kernels");
   return 0;
 }
+
 // The same with the gathers' tile.
 int gather_params(const dream_das_plan *p, FastParams &F) {
-  int r = tile_params(p, F, 0);
+  int r = grid_params(p, F);
   if (r) return r;
   gather_tile(p, F.method, F.tile_f, F.tile_s, F.wf);
   F.out_block = gather_out_block((F.method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt, F.w == nullptr);
@@ -797,8 +792,9 @@ static int op_scatter(dream_das_plan *p, const float *X, const float *dW, float 
   if (p->No == 0 || p->K == 0) return 0;
   FastParams F = p->geo;
   F.w = dW;
-  int r = tile_params(p, F, 0);
+  int r = grid_params(p, F);
   if (r) return r;
+  scatter_tile(p, F);
   if (!apply_shard(p, F)) return 0;
   const int64_t slow_tiles = (F.n_slow + F.tile_s - 1) / F.tile_s;
   const int64_t chunk = slow_tile_chunk(F, terms_per_pixel(p));
@@ -929,7 +925,6 @@ int batch_frame_params(const dream_das_frame &d, FastParams &F) {
     F.tile_s = 1;
   }
   F.wf = gather_patch_f(F.method, d.n_fast > 0, F.tile_s);
-  F.jc = d.jc ? d.jc : 16;
   F.out_block = gather_out_block((F.method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt, false);
   return 0;
 }
@@ -979,7 +974,8 @@ int dream_das_batch_create(dream_das_batch **out, const dream_das_frame *fr, int
       dream_das_batch_destroy(b);
       return r;
     }
-    if (fast_smem_bytes(F, 128) > 220 * 1024) {
+    if (too_many_elements(F.method == DREAM_DAS_RCA_ROWTX ? F.Nr : F.Nt, F.method == DREAM_DAS_RCA_ROWTX ? F.Nt : F.Nr,
+                          128)) {
       dream_das_batch_destroy(b);
       return fail(DREAM_ERR_UNSUPPORTED, "a frame has too many outer elements for the batch kernel");
     }

@@ -9,25 +9,8 @@
 // grid's fastest extent n_fast; otherwise consecutive points), so the 32
 // gathers of one warp fall on one or two 128-byte lines of the A-scan.
 //
-// Scatter (adjoint): the same indices from fixed-point legs. A term's sample
-// index is trunc(RN(RN(a + b) * Fs)) with a, b the two FP64 leg times of the
-// reference (extra_src/das.cc:392-404 and its RCA/SAFT counterparts). Each leg
-// is computed once per (pixel, element), scaled by Fs and stored as fixed point
-// relative to a tile-wide integer base, in one of two formats chosen per tile:
-//   fine: 24 fraction bits, legs spreading over < 127 samples in the tile;
-//         rounding <= 2^-25 per leg, delta = 2^-22, band 2*delta = 2^-21;
-//   wide: 20 fraction bits (coarse grids, spreads up to 4000 samples);
-//         rounding <= 2^-21 per leg, delta = 2^-19, band 2^-18.
-// For legs below 2^26 samples RN(a*Fs) + RN(b*Fs) differs from
-// RN(RN(a+b)*Fs) by at most 3 ulp(2^27) < 2^-24.4, so in both formats the
-// fixed-point sum is within delta of the exact p, and floor(A + B + delta)
-// equals the exact floor whenever the fractional part of the shifted sum is
-// at least 2*delta. Terms inside the band (about 1 in 2 million with the
-// fine format) take an exact FP64 recomputation. The finer format matters
-// for speed: a warp with one ambiguous lane runs the serial FP64 path. The
-// selected indices are identical to the FP64 plain kernel's. The fixed-point
-// leg's 64-bit sum has the term's window cell in its high word and the fraction
-// in its low word.
+// Scatter (adjoint): the same indices, added into shared-memory windows of the
+// tile's columns (below, at scatter_windows).
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -38,18 +21,6 @@
 namespace dream {
 
 namespace {
-
-// Relative fixed-point format of a tile: fb fraction bits, shifted by
-// lo_shift = 32 - fb to the top of the low word of A64 + B64; delta in 2^-fb
-// units; amb_lo = 2*delta in the 2^-32 units of the low word.
-struct FixFmt {
-  int fb, lo_shift;
-  uint32_t delta, amb_lo;
-};
-constexpr FixFmt FMT_FINE{24, 8, 4, 8u << 8};    // delta 2^-22
-constexpr FixFmt FMT_WIDE{20, 12, 2, 4u << 12};  // delta 2^-19
-constexpr int FINE_EXTENT = 126;                 // max integer spread of a leg over a tile, fine format
-constexpr int WIDE_EXTENT = 4000;                // the same, wide format (< 2^12)
 
 template <class YT>
 __device__ __forceinline__ float load_sample(const YT *p);
@@ -177,21 +148,6 @@ __device__ __noinline__ bool exact_index(const FastParams &P, const Pixel &px, i
   return false;
 }
 
-// Layout of the tile's shared arrays (TileShared): per-element bases,
-// extents and column words first, then (from a 16-byte boundary) the outer
-// legs and the staged inner legs of every thread. The set-up's reduction
-// scratch lives at the start of the outer-leg table until the legs are
-// written. The total is a multiple of 16, so the scatter's windows that follow
-// can be read as int4; for 128 outer and 128 inner elements on a 128-point
-// tile it is 76288 bytes, three blocks per SM.
-__host__ __device__ __forceinline__ size_t tile_head_bytes(int n_out, int n_in) {
-  return ((size_t)(2 * (n_out + n_in) + n_out) * sizeof(int) + 15) & ~(size_t)15;
-}
-__host__ __device__ __forceinline__ size_t fast_smem_bytes_dev(const FastParams &P, int n_out, int n_in, int nthr) {
-  const size_t legs = (size_t)(n_out + (P.jc == 8 ? 8 : 16)) * nthr * sizeof(uint32_t);
-  return tile_head_bytes(n_out, n_in) + ((legs + 15) & ~(size_t)15);
-}
-
 // A-scan column of term (outer o, inner i): o * n_in + i for a full Y. A Y
 // holding only the columns of inner elements [ycol_i0, ycol_i0 + ycol_o) (an
 // inner-element shard) has ycol_o columns per outer element.
@@ -203,20 +159,7 @@ __device__ __forceinline__ int64_t ycol(const FastParams &P, int n_in, int o, in
   return ycol_outer(P, n_in, o) + ycol_inner(P, i);
 }
 
-// Fixed-point leg: round(L * 2^fb) modulo 2^32, L = |d| * ocp * Fs + delay * Fs
-// the leg in samples, from cfix = ocp * Fs * 2^fb and dfix = delay * Fs * 2^fb.
-// This is not the reference's rounding chain: it only has to lie within
-// 2^-(fb+1) + 2^-24 of the exact FP64 leg, which holds for |L| and
-// |delay * Fs| below 2^23 (a few units of 2^-53 relative, plus the final
-// rounding); the tile bound keeps every fast-path leg in that range. Adding
-// 1.5 * 2^52 leaves the nearest integer in the low mantissa word.
-__device__ __forceinline__ uint32_t leg_fix(double dx, double dy, double dz, double cfix, double dfix) {
-  const double ss = fma(dz, dz, fma(dy, dy, dx * dx));
-  const double t = fma(__dsqrt_rn(ss), cfix, dfix);
-  return (uint32_t)__double2loint(__dadd_rn(t, 6755399441055744.0));
-}
-
-constexpr double LEG_LIMIT = 8388608.0;  // 2^23 samples: fixed-point legs and delays stay below it
+constexpr double LEG_LIMIT = 8388608.0;  // 2^23 samples: window bases and extents stay below it
 
 // Range of |g - c| for c in [c0, c1].
 __device__ __forceinline__ void offset_range(double g, double c0, double c1, double &lo, double &hi) {
@@ -260,16 +203,6 @@ __device__ __forceinline__ void leg_range(const FastParams &P, const TileBox &B,
   Lmin = (sqrt(lx * lx + ly * ly + lz * lz) * P.ocp + (dl ? B.lo[3] : 0.0)) * P.Fs;
   Lmax = (sqrt(hx * hx + hy * hy + hz * hz) * P.ocp + (dl ? B.hi[3] : 0.0)) * P.Fs;
 }
-
-struct TileShared {
-  double *red;     // [warps][8]: box reduction (set-up only; shares arel's space)
-  int *stat;       // [warps][8]: classification reduction (set-up only; shares arel's space)
-  int *base;       // [n_out + n_in]: integer base of each leg over the tile (outer first)
-  int *ext;        // [n_out + n_in]: bound of (floor(leg) - base)
-  uint32_t *ahi;   // [n_out]: high word of the outer legs (column offset + base)
-  uint32_t *arel;  // [n_out][nthreads]: outer legs, fixed point relative to base, + delta
-  uint32_t *brel;  // [JC][nthreads]: the current chunk's inner legs, relative to base
-};
 
 // ---------------------------------------------------------------------------
 // Gather: one tile of image points, every sample index by the reference's own
@@ -580,182 +513,6 @@ __global__ void __launch_bounds__(256, 2) das_fast_kernel(const FastParams P) {
   gather_tile<YT, WEIGHTED, METHOD>(P, blockIdx.x, (int64_t)blockIdx.y + P.slow_tile0, smem_raw);
 }
 
-// Everything a tile needs before its terms: the image point of each thread,
-// the leg bounds and fixed-point format of the tile, and (unless the tile
-// takes the exact path) the outer legs in shared memory.
-struct TileCtx {
-  Pixel px;
-  int64_t no;
-  bool active, exact_tile, in_bounds;
-  bool vec_safe;  // in bounds, and every scatter window row ends inside its A-scan
-  int tid, nthr, n_out, n_in, i_lo, i_hi;
-  FixFmt F;
-  double cfix, dfixB;
-  int ext_outer, ext_inner;  // largest (top - base) of the outer and of the inner legs
-  TileShared S;
-};
-
-__device__ __forceinline__ void tile_setup(const FastParams &P, int64_t tfi, int64_t tsi, unsigned char *smem_raw,
-                                           TileCtx &T) {
-  const int tid = threadIdx.x;
-  const int nthr = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
-  const int n_out = (P.method == RCA_ROWTX) ? P.Nr : P.Nt;
-  const int n_in = (P.method == RCA_ROWTX) ? P.Nt : P.Nr;
-  // inner elements of this launch: all of them unless the caller sets a range
-  const int i_lo = P.in_lo, i_hi = P.in_hi > 0 ? P.in_hi : n_in;
-
-  TileShared S;
-  S.base = reinterpret_cast<int *>(smem_raw);
-  S.ext = S.base + n_out + n_in;
-  S.ahi = reinterpret_cast<uint32_t *>(S.ext + n_out + n_in);
-  S.arel = reinterpret_cast<uint32_t *>(smem_raw + tile_head_bytes(n_out, n_in));
-  S.brel = S.arel + n_out * nthr;
-  // n_out * nthr words hold the nwarps * 8 doubles and ints of the set-up
-  S.red = reinterpret_cast<double *>(S.arel);
-  S.stat = reinterpret_cast<int *>(S.red + nwarps * 8);
-
-  bool active;
-  const int64_t no = tile_point(P, tfi, tsi, active);
-  Pixel px;
-  pixel_of(P, no, px);
-
-  // ---- 1. tile box, leg bounds, classification ----
-  {
-    double mn[4] = {px.xo, px.yo, px.zo, px.delay_ms}, mx[4] = {px.xo, px.yo, px.zo, px.delay_ms};
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        mn[q] = fmin(mn[q], __shfl_xor_sync(0xffffffffu, mn[q], off));
-        mx[q] = fmax(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], off));
-      }
-    if (lane == 0)
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        S.red[warp * 8 + q] = mn[q];
-        S.red[warp * 8 + 4 + q] = mx[q];
-      }
-  }
-  __syncthreads();
-  TileBox box;
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    box.lo[q] = S.red[q];
-    box.hi[q] = S.red[4 + q];
-  }
-  for (int w = 1; w < nwarps; w++)
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      box.lo[q] = fmin(box.lo[q], S.red[w * 8 + q]);
-      box.hi[q] = fmax(box.hi[q], S.red[w * 8 + 4 + q]);
-    }
-  // delays beyond the fixed-point range send the tile to the exact path
-  int bad = !(fabs(box.lo[3] * P.Fs) < LEG_LIMIT && fabs(box.hi[3] * P.Fs) < LEG_LIMIT);
-  int ext_max = 0, extA = 0, loA = INT_MAX, hiA = INT_MIN, loB = INT_MAX, hiB = INT_MIN;
-  for (int e = tid; e < n_out + n_in; e += nthr) {
-    const bool outer = e < n_out;
-    const int el = outer ? e : e - n_out;
-    if (!outer && (el < i_lo || el >= i_hi)) {
-      S.base[e] = 0;
-      S.ext[e] = 0;
-      continue;
-    }
-    double Lmin, Lmax;
-    leg_range(P, box, outer, el, Lmin, Lmax);
-    int b = 0, t = 0;
-    if (Lmin > -LEG_LIMIT && Lmax < LEG_LIMIT && Lmin <= Lmax) {
-      b = ((int)floor(Lmin) - 1) & ~3;  // a multiple of 4: the scatter's windows start 16-byte aligned
-      t = (int)floor(Lmax) + 1;
-    } else {
-      bad = 1;
-    }
-    S.base[e] = b;
-    S.ext[e] = t - b;
-    ext_max = max(ext_max, t - b);
-    if (outer) extA = max(extA, t - b);
-    if (outer) {
-      loA = min(loA, b);
-      hiA = max(hiA, t);
-    } else {
-      loB = min(loB, b);
-      hiB = max(hiB, t);
-    }
-  }
-  bad = __reduce_or_sync(0xffffffffu, bad);
-  ext_max = __reduce_max_sync(0xffffffffu, ext_max);
-  loA = __reduce_min_sync(0xffffffffu, loA);
-  hiA = __reduce_max_sync(0xffffffffu, hiA);
-  loB = __reduce_min_sync(0xffffffffu, loB);
-  hiB = __reduce_max_sync(0xffffffffu, hiB);
-  extA = __reduce_max_sync(0xffffffffu, extA);
-  if (lane == 0) {
-    S.stat[warp * 8 + 6] = extA;
-    S.stat[warp * 8 + 0] = bad;
-    S.stat[warp * 8 + 1] = ext_max;
-    S.stat[warp * 8 + 2] = loA;
-    S.stat[warp * 8 + 3] = hiA;
-    S.stat[warp * 8 + 4] = loB;
-    S.stat[warp * 8 + 5] = hiB;
-  }
-  __syncthreads();
-  for (int w = 0; w < nwarps; w++) {
-    bad |= S.stat[w * 8 + 0];
-    ext_max = max(ext_max, S.stat[w * 8 + 1]);
-    loA = min(loA, S.stat[w * 8 + 2]);
-    hiA = max(hiA, S.stat[w * 8 + 3]);
-    loB = min(loB, S.stat[w * 8 + 4]);
-    hiB = max(hiB, S.stat[w * 8 + 5]);
-    extA = max(extA, S.stat[w * 8 + 6]);
-  }
-  __syncthreads();  // the scratch is read: the outer legs below may overwrite it
-  const int64_t stride = P.ycol_o > 0 ? P.ycol_o : n_in;
-  bool exact_tile = bad || ext_max > WIDE_EXTENT || loA > hiA ||
-                    (int64_t)n_out * stride * P.K + (int64_t)hiA + hiB + 8448 >= (int64_t(1) << 32) ||
-                    (int64_t)loA + loB < -(int64_t(1) << 30);
-  // a non-ambiguous term's floor index lies in [loA + loB, hiA + hiB + 2]
-  const bool in_bounds = (int64_t)loA + loB >= 0 && (int64_t)hiA + hiB + 2 < P.K;
-
-  const FixFmt F = ext_max > FINE_EXTENT ? FMT_WIDE : FMT_FINE;
-  const double scale = (double)(1u << F.fb);
-  const double cfix = P.ocp * P.Fs * scale;
-  const double dfix = px.delay_ms * P.Fs * scale;
-  if (!exact_tile) {
-    // ---- 2. outer legs, relative to their bases, plus the delta shift ----
-    int leg_bad = 0;
-#pragma unroll 4
-    for (int o = 0; o < n_out; o++) {
-      double dx, dy, dz;
-      leg_diffs(P, px, true, o, dx, dy, dz);
-      const uint32_t r = leg_fix(dx, dy, dz, cfix, P.method == RCA_ROWTX ? 0.0 : dfix) - ((uint32_t)S.base[o] << F.fb);
-      leg_bad |= r >= ((uint32_t)(S.ext[o] + 1) << F.fb);
-      S.arel[o * nthr + tid] = r + F.delta;
-    }
-    for (int o = tid; o < n_out; o += nthr) S.ahi[o] = (uint32_t)(ycol_outer(P, n_in, o) * P.K + S.base[o]);
-    exact_tile = __syncthreads_or(leg_bad) != 0;
-  }
-  T.px = px;
-  T.no = no;
-  T.active = active;
-  T.exact_tile = exact_tile;
-  T.in_bounds = in_bounds;
-  // a window row ends by base_o + ext_o + base_i + ext_i + 7 <= hiA + hiB + 7
-  T.vec_safe = in_bounds && (int64_t)hiA + hiB + 7 <= P.K;
-  T.tid = tid;
-  T.nthr = nthr;
-  T.n_out = n_out;
-  T.n_in = n_in;
-  T.i_lo = i_lo;
-  T.i_hi = i_hi;
-  T.F = F;
-  T.cfix = cfix;
-  T.dfixB = P.method == RCA_ROWTX ? dfix : 0.0;
-  T.ext_outer = extA;
-  T.ext_inner = 0;
-  for (int e = n_out + i_lo; e < n_out + i_hi; e++) T.ext_inner = max(T.ext_inner, S.ext[e]);
-  T.S = S;
-}
-
 }  // namespace
 
 // Persistent batch kernel: CTAs take (frame, tile) work items from a queue
@@ -826,12 +583,6 @@ __global__ void f32_to_bf16_kernel(const float *__restrict__ x, __nv_bfloat16 *_
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-
-size_t fast_smem_bytes(const FastParams &P, int nthr) {
-  const int n_out = (P.method == RCA_ROWTX) ? P.Nr : P.Nt;
-  const int n_in = (P.method == RCA_ROWTX) ? P.Nt : P.Nr;
-  return fast_smem_bytes_dev(P, n_out, n_in, nthr);
-}
 
 size_t gather_smem_bytes(const FastParams &P, int nthr) {
   return (size_t)P.out_block * (nthr * sizeof(double) + (P.w ? GATHER_JC * sizeof(float) : 0));
@@ -922,16 +673,56 @@ cudaError_t convert_f32_to_bf16(const float *x, void *y, int64_t n, cudaStream_t
 
 // ===========================================================================
 // Adjoint (scatter) on pixel tiles: Ya[k(n,c), c] += w[c] * x[n] for the
-// tile's image points n and every A-scan column c, at the forward's indices
-// (fixed-point floors outside the ambiguity band, the FP64 chain inside it).
-// Each term is added with a global reduction; the 32 lanes of a warp hit one
-// column at nearby samples, so a warp's reductions fall on a few sectors.
+// tile's image points n and every A-scan column c, at the forward's indices.
 // Ya must be zeroed (or hold the partial sum to add to) before the launch.
+//
+// The box bounding the tile's points and delays gives every element's leg range
+// (leg_range), hence an integer base (a multiple of 4) and extent per leg; a
+// column's samples then lie in the window [base_o + base_i, + ext_o + ext_i +
+// 2). Per batch of 2 outer x 8 inner elements every term is added into its
+// column's window in shared memory (the addition of the truncation carries the
+// window row and the inner base, the row address the outer base), then a fixed
+// group of threads per row adds the row to the A-scan with 4-wide vector
+// reductions, the weight applied once per sample, and clears it. Two window
+// buffers alternate, so one block barrier per batch suffices (between its adds
+// and its flush).
+//
+// Bound: instruction issue (0.54 of the slots; 13.7 instructions per 32 terms, of
+// which the index chain, the cell's address and the shared addition are 5, the
+// legs of two blocks of outer elements about 2) and the shared-memory / L1 data
+// pipe (0.73: a warp's additions to one cell take a wavefront each, 2.7 per
+// instruction with 8 x 4 points per warp). 64x64 elements, K = 3000, 512x512
+// points: 0.80 ms, weighted 0.89; with fixed-point legs, an ambiguity test and
+// batches of one outer x 16 inner elements 0.83 and 0.99 (37x53 elements 0.35
+// against 0.48, 32x32 and 256x256 points 0.077 against 0.098). The adds carry no
+// guard and the flush no test for zeros: either costs a branch per term (1.2 and
+// 0.97 ms).
 // ===========================================================================
 
 namespace {
 
-// Exact scatter of terms (o, i0 .. i0+jn-1) of one image point.
+constexpr int SCATTER_JC = 8, SCATTER_NO = 2, SCATTER_ROWS = SCATTER_NO * SCATTER_JC;
+// Samples per window row; tiles of wider windows add every term with a global reduction.
+constexpr int SCATTER_WCAP = 192;
+
+// be of every element, then (16-byte aligned) the two window buffers, then the outer legs.
+__host__ __device__ constexpr size_t scatter_head_bytes(int n_out, int n_in) {
+  return ((size_t)2 * (n_out + n_in) * sizeof(int) + 15) & ~(size_t)15;
+}
+constexpr size_t SCATTER_WIN_BYTES = 2 * (size_t)SCATTER_ROWS * SCATTER_WCAP * sizeof(int);
+
+__device__ __forceinline__ void red_add_v4(float *p, float4 v) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+               : "memory");
+}
+__device__ __forceinline__ void red_add(const float *p, float v) {
+  asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
+__device__ __forceinline__ void red_add_shared(uint32_t a, int v) {
+  asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+// Scatter of terms (o, i0 .. i0+jn-1) of one image point, straight into Ya.
 template <bool WEIGHTED>
 __device__ __noinline__ void exact_scatter(const FastParams &P, const Pixel &px, int o, int i0, int jn, int n_in,
                                            float xn, float *Ya) {
@@ -942,114 +733,141 @@ __device__ __noinline__ void exact_scatter(const FastParams &P, const Pixel &px,
   }
 }
 
-template <bool WEIGHTED, bool CHECKED, int JC>
-__device__ __forceinline__ void scatter_loop(const FastParams &P, const TileCtx &T, float xn, float *Ya) {
-  const int64_t K = P.K;
-  const TileShared &S = T.S;
-  const FixFmt F = T.F;
-  const int tid = T.tid, nthr = T.nthr, n_out = T.n_out, n_in = T.n_in;
-  const Pixel px = T.px;  // a copy for the exact path (by reference), so T stays in registers
-  for (int i0 = T.i_lo; i0 < T.i_hi; i0 += JC) {
-    const int jn = min(JC, T.i_hi - i0);
-    bool bad = false;
-#pragma unroll 1
-    for (int j = 0; j < jn; j++) {
-      const int i = i0 + j;
-      double dx, dy, dz;
-      leg_diffs(P, px, false, i, dx, dy, dz);
-      const uint32_t r = leg_fix(dx, dy, dz, T.cfix, T.dfixB) - ((uint32_t)S.base[n_out + i] << F.fb);
-      bad |= r >= ((uint32_t)(S.ext[n_out + i] + 1) << F.fb);
-      S.brel[j * nthr + tid] = r;
-    }
-    if (__any_sync(0xffffffffu, bad)) {
-      if (T.active)
-        for (int o = 0; o < n_out; o++) exact_scatter<WEIGHTED>(P, px, o, i0, jn, n_in, xn, Ya);
-      continue;
-    }
-    uint64_t B64[JC];
+struct ScatterTile {
+  int2 *be;                  // [n_out + n_in]: integer base of each leg over the tile, bound of floor(leg) - base
+  bool usable;               // every base and extent is valid
+  bool low;                  // some term may lie before sample 0
+  bool in_bounds;            // every term of the tile is in bounds
+  int ext_outer, ext_inner;  // largest extents
+};
+
+// Leg bounds of the tile; `scratch`: (blockDim.x / 32) * 8 doubles and as many ints.
+__device__ __forceinline__ void scatter_setup(const FastParams &P, const Pixel &px, unsigned char *smem, double *scratch,
+                                              int n_out, int n_in, int i_lo, int i_hi, ScatterTile &T) {
+  const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
+  T.be = reinterpret_cast<int2 *>(smem);
+  double *red = scratch;
+  int *stat = reinterpret_cast<int *>(red + nwarps * 8);
+  {
+    double mn[4] = {px.xo, px.yo, px.zo, px.delay_ms}, mx[4] = {px.xo, px.yo, px.zo, px.delay_ms};
 #pragma unroll
-    for (int j = 0; j < JC; j++) {
-      B64[j] = 0;
-      if (j < jn) {
-        const uint32_t hi = (uint32_t)(ycol_inner(P, i0 + j) * K + S.base[n_out + i0 + j]);
-        B64[j] = ((uint64_t)S.brel[j * nthr + tid] << F.lo_shift) + ((uint64_t)hi << 32);
-      }
-    }
-    for (int o = 0; o < n_out; o++) {
-      const uint64_t A64 = ((uint64_t)S.arel[o * nthr + tid] << F.lo_shift) + ((uint64_t)S.ahi[o] << 32);
-      uint64_t sj[JC];
-      uint32_t m = 0xffffffffu;
+    for (int off = 16; off > 0; off >>= 1)
 #pragma unroll
-      for (int j = 0; j < JC; j++) {
-        sj[j] = A64 + B64[j];
-        if (j < jn) m = min(m, (uint32_t)sj[j]);
+      for (int q = 0; q < 4; q++) {
+        mn[q] = fmin(mn[q], __shfl_xor_sync(0xffffffffu, mn[q], off));
+        mx[q] = fmax(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], off));
       }
-      if (m < F.amb_lo) {  // an ambiguous term: this outer element's chunk through the exact indices
-        if (T.active) exact_scatter<WEIGHTED>(P, px, o, i0, jn, n_in, xn, Ya);
-        continue;
-      }
-      const int64_t colo = ycol_outer(P, n_in, o);
+    if (lane == 0)
 #pragma unroll
-      for (int j = 0; j < JC; j++) {
-        if (j < jn && T.active) {
-          const float v = WEIGHTED ? __ldg(P.w + colo + ycol_inner(P, i0 + j)) * xn : xn;
-          const uint32_t off = (uint32_t)(sj[j] >> 32);
-          if (CHECKED) {
-            const int64_t col0 = (colo + ycol_inner(P, i0 + j)) * K;
-            const int32_t kk = (int32_t)(off - (uint32_t)col0);
-            if (kk >= 0 && kk < K) atomicAdd(Ya + col0 + kk, v);
-            else if (kk == -1) atomicAdd(Ya + col0, v);
-          } else {
-            atomicAdd(Ya + off, v);
-          }
-        }
+      for (int q = 0; q < 4; q++) {
+        red[warp * 8 + q] = mn[q];
+        red[warp * 8 + 4 + q] = mx[q];
       }
-    }
   }
+  __syncthreads();
+  TileBox box;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    box.lo[q] = red[q];
+    box.hi[q] = red[4 + q];
+  }
+  for (int w = 1; w < nwarps; w++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      box.lo[q] = fmin(box.lo[q], red[w * 8 + q]);
+      box.hi[q] = fmax(box.hi[q], red[w * 8 + 4 + q]);
+    }
+  int bad = !(P.Fs > 0.0), extA = 0, extB = 0, loA = INT_MAX, hiA = INT_MIN, loB = INT_MAX, hiB = INT_MIN;
+  for (int e = tid; e < n_out + n_in; e += nthr) {
+    const bool outer = e < n_out;
+    const int el = outer ? e : e - n_out;
+    int b = 0, t = 0;
+    if (outer || (el >= i_lo && el < i_hi)) {
+      double Lmin, Lmax;
+      leg_range(P, box, outer, el, Lmin, Lmax);
+      if (Lmin > -LEG_LIMIT && Lmax < LEG_LIMIT && Lmin <= Lmax) {
+        b = ((int)floor(Lmin) - 1) & ~3;  // a multiple of 4: windows start 16-byte aligned
+        t = (int)floor(Lmax) + 1;
+      } else {
+        bad = 1;
+      }
+      if (outer) {
+        extA = max(extA, t - b);
+        loA = min(loA, b);
+        hiA = max(hiA, t);
+      } else {
+        extB = max(extB, t - b);
+        loB = min(loB, b);
+        hiB = max(hiB, t);
+      }
+    }
+    T.be[e] = make_int2(b, t - b);
+  }
+  bad = __reduce_or_sync(0xffffffffu, bad);
+  extA = __reduce_max_sync(0xffffffffu, extA);
+  extB = __reduce_max_sync(0xffffffffu, extB);
+  loA = __reduce_min_sync(0xffffffffu, loA);
+  hiA = __reduce_max_sync(0xffffffffu, hiA);
+  loB = __reduce_min_sync(0xffffffffu, loB);
+  hiB = __reduce_max_sync(0xffffffffu, hiB);
+  if (lane == 0) {
+    int *s = stat + warp * 8;
+    s[0] = bad, s[1] = extA, s[2] = extB, s[3] = loA, s[4] = hiA, s[5] = loB, s[6] = hiB;
+  }
+  __syncthreads();
+  for (int w = 0; w < nwarps; w++) {
+    const int *s = stat + w * 8;
+    bad |= s[0];
+    extA = max(extA, s[1]);
+    extB = max(extB, s[2]);
+    loA = min(loA, s[3]);
+    hiA = max(hiA, s[4]);
+    loB = min(loB, s[5]);
+    hiB = max(hiB, s[6]);
+  }
+  __syncthreads();  // the scratch is read
+  T.usable = !bad && loA <= hiA && loB <= hiB;
+  T.low = (int64_t)loA + loB < 0;
+  T.in_bounds = !T.low && (int64_t)hiA + hiB + 2 < P.K;
+  T.ext_outer = extA;
+  T.ext_inner = extB;
 }
 
-
-// Samples per shared-memory window row (windows wider than this send their
-// tile to the direct-reduction path). Two buffers of JC rows alternate, so
-// 256-point tiles of 64 outer elements keep two CTAs per SM.
-constexpr int SCATTER_WCAP = 192;
-
-__device__ __forceinline__ void red_add_v4(float *p, float4 v) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
-               : "memory");
+// Whether a leg (ms) lies inside its window range (bases and extents leave a
+// sample on each side), so that the sum of two such legs, whatever its
+// rounding, falls on a cell of the row.
+__device__ __forceinline__ bool leg_inside(double l, double Fs, int2 be) {
+  const double t = l * Fs - (double)be.x;
+  return t >= 0.5 && t < (double)be.y + 0.5;
 }
 
-// Window scatter of one tile: for outer element o and a chunk of inner
-// elements, every term goes into the shared-memory window of its column (the
-// tile's sample range [base_o + base_i, ... + WS), 16-byte aligned because the
-// bases are multiples of 4); then the windows are added to Ya with 4-wide
-// vector reductions (the weight applied once per sample) and cleared; two
-// buffers alternate, one block barrier per (o, chunk). A term's slot is the
-// high word of A64 + B64 when both hold only the relative legs (the inner leg
-// carrying its row). The windows hold fixed-point
-// integers, x scaled by 2^(22 - E) with max |x| over the tile below 2^E, so
-// the shared-memory additions are native integer atomics, exact and
-// independent of their order (a slot receives at most one term per thread
-// per batch, at most 256 terms of magnitude up to 2^22, and a batch taken
-// back subtracts exactly what it added); each value is rounded once, to within
-// 2^-22 of the tile's largest |x|.
-template <bool WEIGHTED, bool CHECKED, int JC>
-__device__ __forceinline__ void scatter_window_loop(const FastParams &P, const TileCtx &T, float xn_f, float *Ya,
-                                                    float *winf, int WS) {
-  int *win = reinterpret_cast<int *>(winf);
+// The windows hold fixed-point integers, x scaled by 2^(22 - E) with max |x|
+// over the tile below 2^E, so the shared-memory additions are native integer
+// atomics, exact and independent of their order (a slot receives at most one
+// term per thread per batch, at most 256 terms of magnitude up to 2^22); each
+// value is rounded once, to within 2^-22 of the tile's largest |x|. Every leg
+// inside its bound puts its terms on cells of the row, so the adds need no guard;
+// the flush drops the cells outside the A-scan. Only where times may be negative
+// are terms tested one by one (p in (-1, 0) belongs to sample 0, p = -1 does not).
+template <bool WEIGHTED, int METHOD>
+__device__ __forceinline__ void scatter_windows(const FastParams &P, const ScatterTile &T, const Pixel &px, bool active,
+                                                float xn_f, float *Ya, int *win, double *legs, int n_out, int n_in,
+                                                int i_lo, int i_hi) {
+  constexpr int JC = SCATTER_JC, NO = SCATTER_NO, ROWS = SCATTER_ROWS;
+  const int tid = threadIdx.x, nthr = blockDim.x;
   const int64_t K = P.K;
-  const TileShared &S = T.S;
-  const FixFmt F = T.F;
-  const int tid = T.tid, nthr = T.nthr, n_out = T.n_out, n_in = T.n_in;
-  const bool active = T.active;
-  const Pixel px = T.px;
-  const bool vec = !CHECKED && ((K & 3) == 0) && ((reinterpret_cast<uintptr_t>(Ya) & 15) == 0);
+  const int WS = (T.ext_outer + T.ext_inner + 4 + 3) & ~3;  // window samples per row
+  const Legs<METHOD, true> outer(P);
+  const Legs<METHOD, false> inner(P);
+  const double Fs = P.Fs, Kf = (double)K;
+  const bool aligned = (K & 3) == 0 && (reinterpret_cast<uintptr_t>(Ya) & 15) == 0;  // rows start on 16 bytes
+  double *tab = legs + tid;  // leg of outer element o0 + o: tab[o * nthr]
   // fixed-point scale of the tile: max |x| < 2^E, values scaled by 2^(22 - E)
   float mx = fabsf(xn_f);
   for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
   __shared__ float s_mx[8];
   if ((tid & 31) == 0) s_mx[tid >> 5] = mx;
-  for (int e = tid; e < 2 * JC * WS; e += nthr) win[e] = 0;
+  for (int e = tid; e < 2 * ROWS * WS; e += nthr) win[e] = 0;
   __syncthreads();
   mx = 0.0f;
   for (int w = 0; w < (nthr >> 5); w++) mx = fmaxf(mx, s_mx[w]);
@@ -1058,171 +876,194 @@ __device__ __forceinline__ void scatter_window_loop(const FastParams &P, const T
   frexpf(mx, &E);
   const float qscale = ldexpf(1.0f, 22 - E), iS = ldexpf(1.0f, E - 22);
   const int xn = __float2int_rn(xn_f * qscale);
-  // flush: a fixed group of nthr / JC threads per window row (one division
-  // per tile, none per cell)
-  const int tpr = nthr / JC;
-  const int fr = tid / tpr, fq = tid - fr * tpr;
-  // Two window buffers alternate per (outer element, chunk): the adds of one
-  // batch and the flush of the previous one need only the barrier between a
-  // batch's adds and its flush (a buffer is added to again only after the
-  // next batch's barrier, which every thread reaches after its flush).
-  int it = 0;
-  for (int i0 = T.i_lo; i0 < T.i_hi; i0 += JC) {
-    const int jn = min(JC, T.i_hi - i0);
+  // flush: a fixed group of nthr / ROWS threads per window row (q, j)
+  const int tpr = nthr / ROWS, fr = tid / tpr, fq = tid - fr * tpr, fro = fr / JC, fri = fr % JC;
+  const int64_t ostride = P.ycol_o > 0 ? P.ycol_o : n_in;  // columns per outer element
+  const int64_t ystep = SCATTER_NO * ostride * K;
+  const uint32_t win_a = (uint32_t)__cvta_generic_to_shared(win);
+  uint32_t buf = 0;  // byte offset of the batch's buffer
+  for (int o0 = 0; o0 < n_out; o0 += P.out_block) {
+    const int on = min(P.out_block, n_out - o0);
     bool bad = false;
 #pragma unroll 4
-    for (int j = 0; j < jn; j++) {
-      const int i = i0 + j;
-      double dx, dy, dz;
-      leg_diffs(P, px, false, i, dx, dy, dz);
-      const uint32_t r = leg_fix(dx, dy, dz, T.cfix, T.dfixB) - ((uint32_t)S.base[n_out + i] << F.fb);
-      bad |= r >= ((uint32_t)(S.ext[n_out + i] + 1) << F.fb);
-      S.brel[j * nthr + tid] = r;
+    for (int o = 0; o < on; o++) {
+      const double l = outer(P, px, o0 + o);
+      bad = bad || !leg_inside(l, Fs, T.be[o0 + o]);
+      tab[o * nthr] = l;
     }
-    if (__syncthreads_or(bad)) {
-      // an inner leg outside the tile's bound: this chunk through the exact indices, straight to Ya
-      if (active)
-        for (int o = 0; o < n_out; o++) exact_scatter<WEIGHTED>(P, px, o, i0, jn, n_in, xn_f, Ya);
-      continue;
-    }
-    // the high word of B64[j] starts at row j of the window: the sum's high
-    // word is the term's window cell
-    uint64_t B64[JC];
+    const bool outer_bad = __syncthreads_or(bad) != 0;
+    for (int i0 = i_lo; i0 < i_hi; i0 += JC) {
+      const int jn = min(JC, i_hi - i0);
+      double B[JC], mag[JC];
+      bad = false;
 #pragma unroll
-    for (int j = 0; j < JC; j++)
-      B64[j] = (j < jn) ? ((uint64_t)S.brel[j * nthr + tid] << F.lo_shift) + ((uint64_t)(j * WS) << 32) : 0;
-    const bool full = jn == JC;
-    // this thread's flush row fr: the inner element's part of its column, base and extent
-    const bool my_row = fr < jn;
-    const int64_t col_r = my_row ? ycol_inner(P, i0 + fr) : 0;
-    const int64_t ostride = P.ycol_o > 0 ? P.ycol_o : n_in;  // columns per outer element
-    float *ycl = Ya + col_r * K;  // this row's column for outer element o, stepped per o
-    const int base_r = my_row ? S.base[n_out + i0 + fr] : 0, ext_r = my_row ? S.ext[n_out + i0 + fr] : 0;
-    for (int o = 0; o < n_out; o++) {
-      const uint64_t A64 = (uint64_t)S.arel[o * nthr + tid] << F.lo_shift;
-      int *wb = win + (it & 1) * (JC * WS);  // this batch's buffer
-      // Adds first, ambiguity test after: in the rare ambiguous batch the same
-      // integer values are taken back out of the same cells (exact) and the
-      // chunk goes through the exact indices, so no term's sum is kept.
-      uint32_t mc[2] = {0xffffffffu, 0xffffffffu};  // two chains, two terms per step
-      if (full) {
-#pragma unroll
-        for (int j = 0; j < JC; j += 2) {
-          const uint64_t s0 = A64 + B64[j], s1 = A64 + B64[j + 1];
-          atomicAdd(wb + (uint32_t)(s0 >> 32), xn);
-          atomicAdd(wb + (uint32_t)(s1 >> 32), xn);
-          mc[(j >> 1) & 1] = min(mc[(j >> 1) & 1], min((uint32_t)s0, (uint32_t)s1));
+      for (int j = 0; j < JC; j++) {
+        if (j >= jn) {  // past the last inner element: never added
+          B[j] = B[0];
+          mag[j] = mag[0];
+          continue;
         }
-      } else {
+        const int2 be = T.be[n_out + i0 + j];
+        B[j] = inner(P, px, i0 + j);
+        bad = bad || !leg_inside(B[j], Fs, be);
+        mag[j] = 6755399441055744.0 + (double)(j * WS - be.x);  // 1.5 * 2^52: row j, less the inner base
+      }
+      if (__syncthreads_or(bad) || outer_bad) {
+        // a leg outside the tile's bound (not expected): straight to Ya
+        const Pixel c = px;  // a copy for the call by reference: px stays in registers
+        if (active)
+          for (int o = 0; o < on; o++) exact_scatter<WEIGHTED>(P, c, o0 + o, i0, jn, n_in, xn_f, Ya);
+        continue;
+      }
+      // this thread's flush row: the inner element's column, base and extent
+      const bool my_row = fri < jn;
+      const int col_r = i0 + (my_row ? fri : 0);
+      const int2 be_r = T.be[n_out + col_r];
+      const int64_t fcol = (o0 + fro) * ostride + ycol_inner(P, col_r);
+      float *yrow = Ya + fcol * K + be_r.x;
+      const float *wrow = WEIGHTED ? P.w + fcol : nullptr;
+      float w_next = WEIGHTED && my_row && fro < on ? __ldg(wrow) : 0.0f;  // read a batch ahead
+      for (int o = 0; o < on; o += NO, yrow += ystep) {
+        const bool flush = my_row && o + fro < on;
+        const float sc = WEIGHTED ? iS * w_next : iS;  // a power of two: the weight's product rounds once either way
+        if (WEIGHTED && my_row && o + NO + fro < on) w_next = __ldg(wrow += NO * ostride);
+        const int2 be_o = T.be[o0 + (flush ? o + fro : o)];
+        if (!T.low && jn == JC && o + NO <= on) {
+          uint32_t cell[NO][JC];
 #pragma unroll
-        for (int j = 0; j < JC; j++)
-          if (j < jn) {
-            const uint64_t s0 = A64 + B64[j];
-            atomicAdd(wb + (uint32_t)(s0 >> 32), xn);
-            mc[0] = min(mc[0], (uint32_t)s0);
+          for (int q = 0; q < NO; q++) {
+            const double a = tab[(o + q) * nthr];
+            const uint32_t row = win_a + buf + (uint32_t)(q * JC * WS - T.be[o0 + o + q].x) * 4u;
+#pragma unroll
+            for (int j = 0; j < JC; j++)
+              cell[q][j] = row + 4u * (uint32_t)__double2loint(__dadd_rz(__dmul_rn(__dadd_rn(a, B[j]), Fs), mag[j]));
           }
-      }
-      // Inactive lanes carry x = 0 and add nothing, so they need no test.
-      if (min(mc[0], mc[1]) < F.amb_lo) {
-        // an ambiguous term: take this outer element's adds back and use the exact indices
-        for (int j = 0; j < jn; j++) atomicSub(wb + (uint32_t)((A64 + B64[j]) >> 32), xn);
-        for (int j = 0; j < jn; j++) {
-          int k;
-          if (exact_index(P, px, o, i0 + j, k)) {
-            const int slot = k - (S.base[o] + S.base[n_out + i0 + j]);
-            const int wr = (S.ext[o] + S.ext[n_out + i0 + j] + 4 + 3) & ~3;  // the row's flushed width
-            if (slot >= 0 && slot < wr) atomicAdd(wb + j * WS + slot, xn);
-            else atomicAdd(Ya + ycol(P, n_in, o, i0 + j) * K + k, WEIGHTED ? __ldg(P.w + ycol(P, n_in, o, i0 + j)) * xn_f : xn_f);
-          }
-        }
-      }
-      __syncthreads();
-      if (my_row) {
-        // row fr of the window: sample kb + t of column col; the terms of
-        // (o, i) lie in its first ext_o + ext_i + 3 cells
-        const int64_t kb = (int64_t)S.base[o] + base_r;  // a multiple of 4
-        const int wr = (S.ext[o] + ext_r + 4 + 3) & ~3;
-        const float sc = WEIGHTED ? iS * __ldg(P.w + o * ostride + col_r) : iS;  // iS a power of two: one rounding either way
-        int *wrow = wb + fr * WS;
-        if (vec && T.vec_safe) {  // every vector of the row lies inside the A-scan
-          for (int t = fq * 4; t < wr; t += tpr * 4) {
-            int4 *wp = reinterpret_cast<int4 *>(wrow + t);
-            const int4 vi = *wp;
-            if (vi.x | vi.y | vi.z | vi.w) {
-              *wp = make_int4(0, 0, 0, 0);
-              red_add_v4(ycl + kb + t, make_float4((float)vi.x * sc, (float)vi.y * sc, (float)vi.z * sc, (float)vi.w * sc));
+#pragma unroll
+          for (int q = 0; q < NO; q++)
+#pragma unroll
+            for (int j = 0; j < JC; j++) red_add_shared(cell[q][j], xn);
+        } else {
+#pragma unroll
+          for (int q = 0; q < NO; q++) {
+            if (o + q >= on) break;
+            const double a = tab[(o + q) * nthr];
+            const uint32_t row = win_a + buf + (uint32_t)(q * JC * WS - T.be[o0 + o + q].x) * 4u;
+#pragma unroll
+            for (int j = 0; j < JC; j++) {
+              const double p = __dmul_rn(__dadd_rn(a, B[j]), Fs);
+              if (j < jn && p > -1.0) red_add_shared(row + 4u * (uint32_t)__double2loint(__dadd_rz(p, mag[j])), xn);
             }
           }
-        } else if (vec) {
-          for (int t = fq * 4; t < wr; t += tpr * 4) {
-            int4 *wp = reinterpret_cast<int4 *>(wrow + t);
+        }
+        __syncthreads();
+        // samples kb + t of the row; its terms lie in the first ext_o + ext_i + 3 cells
+        const int wr = flush ? be_o.y + be_r.y + 4 : 0;
+        const int64_t kb = (int64_t)be_o.x + be_r.x;  // a multiple of 4
+        if (aligned && kb >= 0 && kb + ((wr + 3) & ~3) <= K) {
+          int4 *wp = reinterpret_cast<int4 *>(reinterpret_cast<char *>(win) + buf) + (fr * WS >> 2) + fq;
+          float *y = yrow + be_o.x + fq * 4;
+          for (int t = fq * 4; t < wr; t += tpr * 4, wp += tpr, y += tpr * 4) {
             const int4 vi = *wp;
-            if (vi.x | vi.y | vi.z | vi.w) {
-              *wp = make_int4(0, 0, 0, 0);
-              const float4 v = make_float4((float)vi.x * sc, (float)vi.y * sc, (float)vi.z * sc, (float)vi.w * sc);
-              const int64_t k0 = kb + t;
-              if (k0 >= 0 && k0 + 4 <= K) {
-                red_add_v4(ycl + k0, v);
-              } else {  // a window edge beyond the A-scan holds only zeros; added one by one to stay inside
-                const float vv[4] = {v.x, v.y, v.z, v.w};
-                for (int q = 0; q < 4; q++)
-                  if (vv[q] != 0.0f && k0 + q >= 0 && k0 + q < K) atomicAdd(ycl + k0 + q, vv[q]);
-              }
-            }
+            *wp = make_int4(0, 0, 0, 0);
+            red_add_v4(y, make_float4((float)vi.x * sc, (float)vi.y * sc, (float)vi.z * sc, (float)vi.w * sc));
           }
         } else {
+          int *cells = win + buf / 4 + fr * WS;
           for (int t = fq; t < wr; t += tpr) {
-            const int vi = wrow[t];
+            const int vi = cells[t];
             if (vi != 0) {
-              wrow[t] = 0;
+              cells[t] = 0;
               int64_t k = kb + t;
               if (k == -1) k = 0;  // p in (-1, 0): sample 0 after truncation toward zero
-              if (k >= 0 && k < K) atomicAdd(ycl + k, (float)vi * sc);
+              if (k >= 0 && k < K) atomicAdd(yrow + (k - be_r.x), (float)vi * sc);
             }
           }
         }
+        buf ^= (uint32_t)(ROWS * WS) * 4u;
       }
-      ycl += ostride * K;
-      it++;
     }
   }
 }
 
-template <bool WEIGHTED, int JC>
+template <bool WEIGHTED, int METHOD>
 __global__ void __launch_bounds__(256, 2) das_scatter_kernel(const FastParams P, const float *__restrict__ X,
                                                              float *__restrict__ Ya) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  TileCtx T;
-  tile_setup(P, blockIdx.x, (int64_t)blockIdx.y + P.slow_tile0, smem_raw, T);
-  const float xn = T.active ? __ldg(X + T.no) : 0.0f;
-  const int WS = (T.ext_outer + T.ext_inner + 4 + 3) & ~3;  // window samples per column
-  float *win = reinterpret_cast<float *>(smem_raw + fast_smem_bytes_dev(P, T.n_out, T.n_in, T.nthr));
-  if (!T.exact_tile && WS <= SCATTER_WCAP) {
-    if (T.in_bounds) scatter_window_loop<WEIGHTED, false, JC>(P, T, xn, Ya, win, WS);
-    else scatter_window_loop<WEIGHTED, true, JC>(P, T, xn, Ya, win, WS);
-  } else if (T.exact_tile) {
-    const Pixel px = T.px;  // a copy: the exact path takes it by reference, T stays in registers
-    if (T.active)
-      for (int o = 0; o < T.n_out; o++)
-        for (int i0 = T.i_lo; i0 < T.i_hi; i0 += 16)
-          exact_scatter<WEIGHTED>(P, px, o, i0, min(16, T.i_hi - i0), T.n_in, xn, Ya);
-  } else if (T.in_bounds) {
-    scatter_loop<WEIGHTED, false, JC>(P, T, xn, Ya);
-  } else {
-    scatter_loop<WEIGHTED, true, JC>(P, T, xn, Ya);
+  const int n_out = METHOD == RCA_ROWTX ? P.Nr : P.Nt, n_in = METHOD == RCA_ROWTX ? P.Nt : P.Nr;
+  const int i_lo = P.in_lo, i_hi = P.in_hi > 0 ? P.in_hi : n_in;
+  int *win = reinterpret_cast<int *>(smem_raw + scatter_head_bytes(n_out, n_in));
+  double *legs = reinterpret_cast<double *>(smem_raw + scatter_head_bytes(n_out, n_in) + SCATTER_WIN_BYTES);
+  bool active;
+  const int64_t no = tile_point(P, blockIdx.x, (int64_t)blockIdx.y + P.slow_tile0, active);
+  Pixel px;
+  pixel_of(P, no, px);
+  ScatterTile T;
+  scatter_setup(P, px, smem_raw, reinterpret_cast<double *>(win), n_out, n_in, i_lo, i_hi, T);
+  const float xn = active ? __ldg(X + no) : 0.0f;
+  if (T.usable && T.ext_outer + T.ext_inner + 7 <= SCATTER_WCAP) {
+    scatter_windows<WEIGHTED, METHOD>(P, T, px, active, xn, Ya, win, legs, n_out, n_in, i_lo, i_hi);
+    return;
+  }
+  // windows wider than the shared-memory rows, or legs outside the integer range: every term added on its own
+  if (!active) return;
+  const Legs<METHOD, true> outer(P);
+  const Legs<METHOD, false> inner(P);
+  const int64_t ostride = P.ycol_o > 0 ? P.ycol_o : n_in;
+  const double Kf = (double)P.K;
+  double *tab = legs + threadIdx.x;
+  const bool plain = T.usable && T.in_bounds && P.K < (int64_t(1) << 28);  // sample numbers of a chunk fit 32 bits
+  for (int o0 = 0; o0 < n_out; o0 += P.out_block) {
+    const int on = min(P.out_block, n_out - o0);
+    for (int o = 0; o < on; o++) tab[o * blockDim.x] = outer(P, px, o0 + o);
+    for (int i0 = i_lo; i0 < i_hi; i0 += SCATTER_JC) {
+      const int jn = min(SCATTER_JC, i_hi - i0);
+      double B[SCATTER_JC];
+#pragma unroll
+      for (int j = 0; j < SCATTER_JC; j++) B[j] = j < jn ? inner(P, px, i0 + j) : 0.0;
+      for (int o = 0; o < on; o++) {
+        const double a = tab[o * blockDim.x];
+        const int64_t col = (o0 + o) * ostride + ycol_inner(P, i0);
+        float *y = Ya + col * P.K;
+        if (plain && jn == SCATTER_JC) {
+#pragma unroll
+          for (int j = 0; j < SCATTER_JC; j++) {
+            const double p = __dmul_rn(__dadd_rn(a, B[j]), P.Fs);
+            const uint32_t k = (uint32_t)__double2loint(__dadd_rz(p, 4503599627370496.0 + (double)(j * P.K)));
+            red_add(elem_addr<float>(reinterpret_cast<const char *>(y), k), WEIGHTED ? __ldg(P.w + col + j) * xn : xn);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < SCATTER_JC; j++) {
+            const double p = __dmul_rn(__dadd_rn(a, B[j]), P.Fs);
+            if (j < jn && p > -1.0 && p < Kf)
+              atomicAdd(y + j * P.K + trunc_index(p), WEIGHTED ? __ldg(P.w + col + j) * xn : xn);
+          }
+        }
+      }
+    }
   }
 }
 
 }  // namespace
 
-// Tile scatter over the same tiles and slow-tile ranges as launch_fast (P as
-// for the forward; P.w optional). Ya is not zeroed here.
-cudaError_t launch_scatter(const FastParams &P, const float *X, float *Ya, cudaStream_t st) {
+// Tile scatter over the slow-tile range of P (P.w optional). Ya is not zeroed here.
+cudaError_t launch_scatter(const FastParams &P0, const float *X, float *Ya, cudaStream_t st) {
+  FastParams P = P0;
   const int nthr = P.tile_f * P.tile_s;
-  // the tile's arrays, then two buffers of one (outer, inner chunk) batch's windows
-  const size_t smem = fast_smem_bytes(P, nthr) + 2 * (size_t)(P.jc == 8 ? 8 : 16) * SCATTER_WCAP * sizeof(float);
-  auto kern = P.w ? (P.jc == 8 ? das_scatter_kernel<true, 8> : das_scatter_kernel<true, 16>)
-                  : (P.jc == 8 ? das_scatter_kernel<false, 8> : das_scatter_kernel<false, 16>);
+  const int n_out = P.method == RCA_ROWTX ? P.Nr : P.Nt, n_in = P.method == RCA_ROWTX ? P.Nt : P.Nr;
+  // even blocks of at most 40 outer elements, fewer where thousands of elements' bounds take the space
+  const size_t fixed = scatter_head_bytes(n_out, n_in) + SCATTER_WIN_BYTES;
+  const int64_t room = ((int64_t)220 * 1024 - (int64_t)fixed) / (int64_t)(nthr * sizeof(double));
+  const int most = (int)std::max<int64_t>(2, std::min<int64_t>(40, room));
+  const int blocks = (n_out + most - 1) / most;
+  P.out_block = std::min(most, ((n_out + blocks - 1) / blocks + 1) & ~1);
+  const size_t smem = fixed + std::max<size_t>((size_t)P.out_block * nthr * sizeof(double), 1024);
+#define SCATTER_KERNEL(W)                                         \
+  (P.method == TFM         ? das_scatter_kernel<W, TFM>           \
+   : P.method == RCA_COLTX ? das_scatter_kernel<W, RCA_COLTX>     \
+                           : das_scatter_kernel<W, RCA_ROWTX>)
+  auto kern = P.w ? SCATTER_KERNEL(true) : SCATTER_KERNEL(false);
+#undef SCATTER_KERNEL
   cudaError_t e = ensure_smem(kern, smem);
   if (e != cudaSuccess) return e;
   const int64_t gx = (P.n_fast + P.tile_f - 1) / P.tile_f;

@@ -25,8 +25,7 @@ struct FastParams {
   // image tiling: point n = s*n_fast + f
   int64_t n_fast, n_slow;
   int tile_f, tile_s, wf;  // tile extents; warp lanes along the fast axis
-  int out_block;           // gathers: outer elements whose legs are tabled at a time
-  int jc;                  // scatter: inner elements per window batch, 8 or 16
+  int out_block;           // outer elements whose legs are tabled at a time
   int64_t slow_tile0, slow_tile1;  // slow-tile range of this launch
   int64_t no0, no1;                // point range (SAFT launches)
   // inner-element range [in_lo, in_hi) of this launch (in_hi == 0: all inner
@@ -58,7 +57,12 @@ inline int gather_out_block(int n_out, bool single) {
   const int n = (n_out + 51) / 52;
   return n > 0 ? ((n_out + n - 1) / n + 3) / 4 * 4 : 4;
 }
-size_t fast_smem_bytes(const FastParams &P, int nthr);    // tile arrays of the scatter
+// Frames with more elements than this limit allows on a tile of nthr points are
+// refused by every storage-precision entry (gather and scatter alike).
+inline bool too_many_elements(int n_out, int n_in, int nthr) {
+  const size_t head = ((size_t)(3 * n_out + 2 * n_in) * 4 + 15) & ~(size_t)15;
+  return head + (((size_t)(n_out + 16) * nthr * 4 + 15) & ~(size_t)15) > 220 * 1024;
+}
 size_t gather_smem_bytes(const FastParams &P, int nthr);  // leg table of the gather (P.out_block)
 cudaError_t launch_fast(const FastParams &P, bool bf16, cudaStream_t st);
 // Adjoint on the forward's tiles: Ya[k(n,c), c] += w[c] * X[n] (FP32 A-scans;

@@ -107,7 +107,7 @@ extern "C" int dream_das_batch_run_noalloc(const dream_das_frame *fr, int n_fram
     const int r = batch_frame_params(fr[f], F);
     if (r) return r;
     F.oob = d_oob;
-    if (fast_smem_bytes(F, 128) > 220 * 1024)
+    if (too_many_elements(F.method == DREAM_DAS_RCA_ROWTX ? F.Nr : F.Nt, F.method == DREAM_DAS_RCA_ROWTX ? F.Nt : F.Nr, 128))
       return set_last_error(DREAM_ERR_UNSUPPORTED, "a frame has too many outer elements for the batch kernel");
     smem = std::max(smem, gather_smem_bytes(F, 128));
     order[f] = f;

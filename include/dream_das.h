@@ -220,15 +220,15 @@ int dream_das_set_grid_hint(dream_das_plan *plan, int64_t n_fast);
  * is a multiple of 8 and tile_s of 4, without one tile_s must be 1).
  * (0, 0) restores the automatic choice. Used by the autotuner. Automatic,
  * on a hinted grid: 8 x 16 points for the gathers on TFM frames and 16 x 8 on RCA
- * volumes, 8 x 32 for the operator's adjoint on TFM frames; 128 consecutive
- * points (the adjoint: 256) without a hint; the adjoint takes fewer points when
- * many outer elements would overflow its tile's shared memory.
+ * volumes; for the operator's adjoint 16 x 16 and 8 x 16, or 8 x 8 where that
+ * would leave SMs without a tile; 128 consecutive points (the adjoint: 256)
+ * without a hint.
  */
 int dream_das_set_tile(dream_das_plan *plan, int tile_f, int tile_s);
 int dream_das_get_tile(const dream_das_plan *plan, int *tile_f, int *tile_s);
 
-/* Inner elements per window batch of the operator's adjoint: 8 or 16 (0 =
- * automatic, 16). The gathers do not depend on it. */
+/* Accepted for compatibility (0, 8 or 16): the F32_STORE / BF16_STORE kernels
+ * have one register chunk of inner elements. */
 int dream_das_set_chunk(dream_das_plan *plan, int jc);
 
 /*
