@@ -55,6 +55,7 @@ SIGNATURES = {
     "dream_das_uni_run": (_i, [_vp, _vp, _pd, _d, _d, _d, _vp, _i, _pi64]),
     "dream_das_uni_run_device": (_i, [_vp, _vp, _pd, _d, _d, _d, _vp, _i, _pi64, _vp]),
     "dream_das_set_grid_hint": (_i, [_vp, _i64]),
+    "dream_das_detect_grid": (_i, [_vp, _vp, _pi64, _vp]),
     "dream_das_set_tile": (_i, [_vp, _i, _i]),
     "dream_das_set_chunk": (_i, [_vp, _i]),
     "dream_das_set_inner_shard": (_i, [_vp, _i64, _i64]),

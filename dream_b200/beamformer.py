@@ -145,7 +145,8 @@ def das_generic(dtype, Y, Gt, Gr, Ro, dt, delay, cp, method, err_level="stop", d
     prec = _lib.PREC_F64 if np.dtype(dtype) == np.float64 else _lib.PREC_F32
     key = ("das", das_type, K, No, Nt, Nr, prec, dev)
     plan = _plan(key, lambda: _lib.plan_create(das_type, K, No, Nt, Nr, prec, dev))
-    _set_hint(plan, grid_hint(Ro))
+    if das_type != _lib.SAFT:  # SAFT kernels take no grid
+        _set_hint(plan, grid_hint(Ro))
     Im = np.zeros(No, dtype=dtype)
     oob = ctypes.c_int64(0)
     p = lambda a: a.ctypes.data_as(ctypes.c_void_p) if a is not None and a.size else None
@@ -158,8 +159,8 @@ def das_generic(dtype, Y, Gt, Gr, Ro, dt, delay, cp, method, err_level="stop", d
 
 
 def _set_hint(plan, h):
-    """The plan's grid hint (only speed depends on it: the plain kernels give
-    each warp an 8 x 4 patch of the grid instead of 32 consecutive points)."""
+    """The plan's grid hint (only speed depends on it: the plain TFM and RCA
+    kernels then work on 2-D tiles of the grid instead of consecutive points)."""
     if getattr(plan, "hint", None) != h:
         _lib.check(_lib.load().dream_das_set_grid_hint(plan.handle, int(h)))
         plan.hint = h
@@ -169,7 +170,10 @@ def _torch_fortran(t, dtype, device):
     """Column-major device copy. Host data in pinned memory is uploaded
     asynchronously (the caller's stream orders it before the kernel)."""
     import torch
-    tdt = torch.float64 if np.dtype(dtype) == np.float64 else torch.float32
+    tdt = torch.float64 if dtype is np.float64 or np.dtype(dtype) == np.float64 else torch.float32
+    if (isinstance(t, torch.Tensor) and t.dtype is tdt and t.device == device and t.dim() == 2 and t.stride(0) == 1
+            and t.stride(1) == t.shape[0] and not t.requires_grad):
+        return t  # already in place
     if not _is_torch(t):
         t = torch.as_tensor(np.asarray(t))
     if t.device.type == "cpu" and t.dtype == tdt:
@@ -196,10 +200,10 @@ def _das_torch(dtype, Y, Gt, Gr, Ro, dt, delay, cp, das_type, level, dev):
     prec = _lib.PREC_F64 if np.dtype(dtype) == np.float64 else _lib.PREC_F32
     key = ("das", das_type, K, No, Nt, Nr, prec, dev)
     plan = _plan(key, lambda: _lib.plan_create(das_type, K, No, Nt, Nr, prec, dev))
-    _set_hint(plan, grid_hint(Ro))
+    stream = torch.cuda.current_stream(device).cuda_stream
+    _set_hint(plan, _device_grid_hint(plan, Ro, stream))
     Im = torch.empty(No, dtype=Y.dtype, device=device)
     oob = ctypes.c_int64(0)
-    stream = torch.cuda.current_stream(device).cuda_stream
     ptr = lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None and t.numel() else None
     st = _lib.check(_lib.load().dream_das_run_device(
         plan.handle, ptr(Y), ptr(Ro), ptr(Gt), ptr(Gr), float(dt),
@@ -305,10 +309,22 @@ def grid_hint(Ro) -> int:
     return n if (n > 0 and No % n == 0 and n < No) else 0
 
 
+def _device_grid_hint(plan, Ro, stream) -> int:
+    """``grid_hint`` of a plan's image points on the device: one kernel and one
+    read-back on the stream."""
+    n = ctypes.c_int64(0)
+    _lib.check(_lib.load().dream_das_detect_grid(plan.handle, ctypes.c_void_p(Ro.data_ptr()), ctypes.byref(n),
+                                                 ctypes.c_void_p(stream)))
+    return n.value
+
+
 def _fast_plan(das_type, K, No, Nt, Nr, prec, dev, hint, tile=None):
+    """The cached plan with its hint and tile set; ``hint`` may be a function of the plan."""
     key = ("fast", das_type, K, No, Nt, Nr, prec, dev)
     plan = _plan(key, lambda: _lib.plan_create(das_type, K, No, Nt, Nr, prec, dev))
     L = _lib.load()
+    if callable(hint):
+        hint = hint(plan)
     if getattr(plan, "hint", None) != hint:
         _lib.check(L.dream_das_set_grid_hint(plan.handle, int(hint)))
         plan.hint = hint
@@ -401,15 +417,24 @@ def das_mixed(Y, Gt, Gr, Ro, dt, delay, cp, method, err_level="stop", device="cu
             raise RuntimeError("das: inner-element shard out of range")
         if C != n_out * (hi - lo):
             raise RuntimeError(f"das: an inner-element shard [{lo}, {hi}) needs {n_out * (hi - lo)} A-scans, got {C}")
-    h = grid_hint(Ro if not on_host else np.asarray(Ro)) if hint == "auto" else int(hint or 0)
+    st_ = stream if stream is not None else torch.cuda.current_stream(device_t).cuda_stream
+    if hint != "auto":
+        h = int(hint or 0)
+    elif stream is None:
+        h = lambda p: _device_grid_hint(p, Ro_t, st_)
+    else:  # a stream of the caller's: the points are read on torch's, which made them
+        h = grid_hint(Ro_t)
     plan = _fast_plan(das_type, K, No, Nt, Nr, prec, dev, h, tile)
     Im = torch.empty(No, dtype=torch.float32, device=device_t)
-    d_oob = torch.zeros(1, dtype=torch.int64, device=device_t)
-    st_ = stream if stream is not None else torch.cuda.current_stream(device_t).cuda_stream
     ptr = lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None and t.numel() else None
     L = _lib.load()
     common = (plan.handle, ptr(Yt), ptr(Ro_t), ptr(Gt_t), ptr(Gr_t), float(dt),
               _lib.DELAY_MULTIPLE if multi else _lib.DELAY_SINGLE, ptr(dl_t), float(cp))
+    if weights is None and inner is None and stream is None:
+        n_oob = ctypes.c_int64(0)
+        _report(_lib.check(L.dream_das_run_device(*common, ptr(Im), level, ctypes.byref(n_oob), ctypes.c_void_p(st_))))
+        return Im.cpu().numpy() if on_host else Im
+    d_oob = torch.zeros(1, dtype=torch.int64, device=device_t)
     if weights is not None:
         w = torch.as_tensor(weights, dtype=torch.float32, device=device_t).reshape(-1).contiguous()
         need = Nt if (das_type == _lib.SAFT or Nr == 0) else Nt * Nr
@@ -417,14 +442,14 @@ def das_mixed(Y, Gt, Gr, Ro, dt, delay, cp, method, err_level="stop", device="cu
             raise RuntimeError(f"das: weights need {need} values (one per A-scan column)")
         _lib.check(L.dream_das_weighted_run_device(*common, ptr(w), ptr(Im), ptr(d_oob),
                                                    ctypes.c_void_p(st_)))
-    elif inner is not None:
+    elif inner is None:
+        _lib.check(L.dream_das_run_device_async(*common, ptr(Im), ptr(d_oob), ctypes.c_void_p(st_)))
+    else:
         _lib.check(L.dream_das_set_inner_shard(plan.handle, lo, hi))
         try:
             _lib.check(L.dream_das_run_device_async(*common, ptr(Im), ptr(d_oob), ctypes.c_void_p(st_)))
         finally:
             _lib.check(L.dream_das_set_inner_shard(plan.handle, 0, 0))
-    else:
-        _lib.check(L.dream_das_run_device_async(*common, ptr(Im), ptr(d_oob), ctypes.c_void_p(st_)))
     oob = int(d_oob.item())
     st = 0 if oob == 0 else {_lib.LVL_IGNORE: 1, _lib.LVL_WARN: 2, _lib.LVL_STOP: 3}[level]
     _report(st)

@@ -323,6 +323,20 @@ int prepare_das(dream_das_plan *p, PlainLaunch &L, const void *dY, const void *d
   return 0;
 }
 
+// Smallest n > 0 whose x or y differs from point 0's. Blocks advance through the
+// points together and stop once a change lies before their next ones.
+template <class T>
+__global__ void first_change_kernel(const T *Ro, int64_t No, unsigned long long *first) {
+  const T x0 = Ro[0], y0 = Ro[No];
+  for (int64_t n0 = (int64_t)blockIdx.x * blockDim.x; n0 < No; n0 += (int64_t)gridDim.x * blockDim.x) {
+    if (*(volatile unsigned long long *)first < (unsigned long long)n0) return;
+    const int64_t n = n0 + threadIdx.x;
+    const bool change = n < No && (Ro[n] != x0 || Ro[n + No] != y0);
+    const unsigned int b = __ballot_sync(0xffffffffu, change);
+    if (b && (threadIdx.x & 31) == __ffs(b) - 1) atomicMin(first, (unsigned long long)n);
+  }
+}
+
 __global__ void add_u64_kernel(unsigned long long *ctr, unsigned long long v) { *ctr += v; }
 
 // K == 0 (or no element pairs) has no in-bounds sample: the image is all
@@ -641,6 +655,29 @@ int64_t dream_das_plan_bound_violations(dream_das_plan *p) {
   CU(cudaDeviceSynchronize());
   CU(cudaMemcpy(&v, p->bBad.p, sizeof(v), cudaMemcpyDeviceToHost));
   return (int64_t)v;
+}
+
+int dream_das_detect_grid(dream_das_plan *p, const void *dRo, int64_t *n_fast, void *stream) {
+  DREAM_API_TRY
+  if (p == nullptr || n_fast == nullptr) return fail(DREAM_ERR_ARGUMENT, "NULL argument");
+  *n_fast = 0;
+  if (p->No < 2 || effective_method(p) == DREAM_DAS_SAFT) return 0;  // SAFT kernels take no grid
+  if (dRo == nullptr) return fail(DREAM_ERR_ARGUMENT, "NULL Ro");
+  std::lock_guard<std::mutex> lk(p->mu);
+  DeviceGuard g(p->device);
+  cudaStream_t st = (cudaStream_t)stream;
+  unsigned long long *first = (unsigned long long *)p->bOob.p;
+  CU(cudaMemsetAsync(first, 0xff, sizeof(unsigned long long), st));
+  const int blocks = (int)std::min<int64_t>((p->No + 255) / 256, 2 * (int64_t)p->sm_count);
+  if (geo_size(p) == 8) first_change_kernel<double><<<blocks, 256, 0, st>>>((const double *)dRo, p->No, first);
+  else first_change_kernel<float><<<blocks, 256, 0, st>>>((const float *)dRo, p->No, first);
+  CU(cudaGetLastError());
+  CU(cudaMemcpyAsync(p->h_oob, first, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+  CU(cudaStreamSynchronize(st));
+  const int64_t n = *p->h_oob < (unsigned long long)p->No ? (int64_t)*p->h_oob : p->No;
+  *n_fast = (n > 0 && n < p->No && p->No % n == 0) ? n : 0;
+  return 0;
+  DREAM_API_CATCH
 }
 
 int dream_das_set_grid_hint(dream_das_plan *p, int64_t n_fast) {

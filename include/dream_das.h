@@ -214,6 +214,14 @@ int64_t dream_das_plan_bound_violations(dream_das_plan *plan);
 int dream_das_set_grid_hint(dream_das_plan *plan, int64_t n_fast);
 
 /*
+ * The grid hint of the image points dRo (No x 3 on the device, in the plan's
+ * geometry precision): the number of leading points that share x and y when it
+ * divides No and is smaller, else 0 (and 0 for SAFT, whose kernels take no
+ * grid). Does not set it. Blocks until the stream has reached the answer.
+ */
+int dream_das_detect_grid(dream_das_plan *plan, const void *dRo, int64_t *n_fast, void *stream);
+
+/*
  * Tile of image points per CTA for the F32_STORE / BF16_STORE kernels:
  * tile_f points along the fast grid axis x tile_s along the slow axis
  * (tile_f*tile_s threads, 32..256, a multiple of 32; with a grid hint tile_f
