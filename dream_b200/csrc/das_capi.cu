@@ -374,18 +374,13 @@ void scatter_tile(const dream_das_plan *p, FastParams &F) {
   F.wf = hint ? 8 : 32;
 }
 
-// Tile of the gathers: the user's, or 128 points, 8 x 16 on a TFM grid and 16 x
-// 8 on an RCA's (64 and 256 points measure within 3 % of these; see gather_patch_f).
-void gather_tile(const dream_das_plan *p, int method, int &tf, int &ts, int &wf) {
+// Tile of the gathers: the user's, or 128 points, 8 x 16 on a hinted grid (64 and
+// 256 points measure within 4 % of these; see gather_patch_f).
+void gather_tile(const dream_das_plan *p, int &tf, int &ts, int &wf) {
   const bool hint = p->n_fast > 0;
-  if (p->tile_f > 0) {
-    tf = p->tile_f;
-    ts = p->tile_s;
-  } else {
-    tf = !hint ? 128 : (method == DREAM_DAS_TFM ? 8 : 16);
-    ts = 128 / tf;
-  }
-  wf = gather_patch_f(method, hint, ts);
+  tf = p->tile_f > 0 ? p->tile_f : (hint ? 8 : 128);
+  ts = p->tile_f > 0 ? p->tile_s : 128 / tf;
+  wf = gather_patch_f(hint, ts);
 }
 
 // Grid axes of the FP32/BF16-storage kernels for plan p, and its refusal of
@@ -411,7 +406,7 @@ int grid_params(const dream_das_plan *p, FastParams &F) {
 int gather_params(const dream_das_plan *p, FastParams &F) {
   int r = grid_params(p, F);
   if (r) return r;
-  gather_tile(p, F.method, F.tile_f, F.tile_s, F.wf);
+  gather_tile(p, F.tile_f, F.tile_s, F.wf);
   F.out_block = gather_out_block((F.method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt, F.w == nullptr);
   return 0;
 }
@@ -753,7 +748,7 @@ int dream_das_get_tile(const dream_das_plan *p, int *tile_f, int *tile_s) {
   DREAM_API_TRY
   if (p == nullptr || tile_f == nullptr || tile_s == nullptr) return fail(DREAM_ERR_ARGUMENT, "NULL argument");
   int wf = 0;
-  gather_tile(p, effective_method(p), *tile_f, *tile_s, wf);
+  gather_tile(p, *tile_f, *tile_s, wf);
   return 0;
   DREAM_API_CATCH
 }
@@ -953,7 +948,7 @@ int batch_frame_params(const dream_das_frame &d, FastParams &F) {
   if (d.n_fast > 0) {
     F.n_fast = d.n_fast;
     F.n_slow = d.No / d.n_fast;
-    F.tile_f = d.tile_f ? d.tile_f : (F.method == DREAM_DAS_TFM ? 8 : 16);
+    F.tile_f = d.tile_f ? d.tile_f : 8;
     F.tile_s = d.tile_s ? d.tile_s : 128 / F.tile_f;
   } else {
     F.n_fast = d.No;
@@ -961,7 +956,7 @@ int batch_frame_params(const dream_das_frame &d, FastParams &F) {
     F.tile_f = 128;
     F.tile_s = 1;
   }
-  F.wf = gather_patch_f(F.method, d.n_fast > 0, F.tile_s);
+  F.wf = gather_patch_f(d.n_fast > 0, F.tile_s);
   F.out_block = gather_out_block((F.method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt, false);
   return 0;
 }
