@@ -208,6 +208,50 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
   return v;
 }
 
+// Adds this step's amplitudes in lane order, lanes with the same key (a sample
+// number whose top bit is clear) into the same sample *h.
+template <class Key>
+__device__ __forceinline__ void ordered_adds(bool in, Key key, double ai, double *h, int lane, double *stage) {
+  // lanes adding into the same sample form a group; the others get unique keys
+  const unsigned int group = __match_any_sync(0xffffffffu, in ? key : ~(Key)lane);
+  const int len = __popc(group);
+  const bool leader = in && (group & ((1u << lane) - 1u)) == 0u;  // lowest lane of its group
+  // a run: the group's lanes are lane .. lane + len - 1
+  const bool run = (group >> lane) == (len == 32 ? 0xffffffffu : (1u << len) - 1u);
+  if (__all_sync(0xffffffffu, !leader || run)) {
+    stage[lane] = ai;
+    __syncwarp();
+    if (leader) {
+      double acc = __dadd_rn(*h, ai);
+      const double *q = stage + lane + 1;
+      int k = len - 1;
+      for (; k >= 8; k -= 8, q += 8) {
+#pragma unroll
+        for (int u = 0; u < 8; u++) acc = __dadd_rn(acc, q[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 7; u++)
+        if (u < k) acc = __dadd_rn(acc, q[u]);
+      *h = acc;
+    }
+  } else {
+    // each leader walks its group's lanes in ascending order (its own first);
+    // the warp takes as many steps as the largest group has members
+    const unsigned int steps = __reduce_max_sync(0xffffffffu, leader ? (unsigned)len : 0u);
+    double acc = leader ? *h : 0.0;
+    unsigned int rem = leader ? group : 0u;
+    for (unsigned int k = 0; k < steps; k++) {
+      const int src = rem ? __ffs(rem) - 1 : lane;
+      const bool add = rem != 0u;
+      rem &= rem - 1u;
+      const double aj = __shfl_sync(0xffffffffu, ai, src);
+      if (add) acc = __dadd_rn(acc, aj);
+    }
+    if (leader) *h = acc;
+  }
+  __syncwarp();  // this step's sums (and stage reads) complete before the next step
+}
+
 // One warp step: lane's term (if valid) at surface element (ix, iy) of the
 // element V is added to its sample, every sample receiving its terms in lane
 // order. Lanes that hit the same sample are grouped (__match_any_sync); the
@@ -219,30 +263,15 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 // SKIP: steps with no term in the SIR skip the amplitudes and the sums (arrays,
 // whose live elements still place most terms outside short windows); without
 // it the amplitude divisions overlap the index computation.
-// PLAIN: term_plain holds for every lane's element.
-template <bool SKIP, bool PLAIN>
+template <bool SKIP>
 __device__ __forceinline__ void term_step(const RectParams &P, const ElemView &V, bool valid, int ix, int iy,
                                           int lane, int64_t w0, int64_t w1, double *h, double *stage,
                                           unsigned long long &oob, unsigned int &flags, bool last) {
   bool in = false;
   int64_t it = 0;
   double r = 1.0;  // idle lanes: a finite amplitude that is never added
-  double ai = 0.0, rh = 0.0;
-  if (PLAIN) {
-    const double rx = __dsub_rn(V.xo, __ldg(P.xs + (valid ? ix : 0)));
-    const double ry = __dsub_rn(V.yo, __ldg(P.ys + (valid ? iy : 0)));
-    r = rect_root(__dadd_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)), V.rz2), rh);
-    if (!SKIP) ai = rect_amplitude(P, V.w, r, rh);
-    const int q = rect_number(P, r, __fma_rn(-V.dl, P.inv_dt, RECT_MAGIC));
-    it = q >> RECT_FB;
-    if (rect_near(q)) it = __double2ll_rn(rect_q(r, V.dl, P));
-    in = valid && it >= 0 && it < P.nt;
-    oob += valid && !in ? 1u : 0u;
-    if (valid && !in && last) flags |= RECT_LAST_OOB;
-    const bool inside = it >= w0 && it < w1;  // true whenever the window bound holds
-    if (in && !inside) flags |= RECT_MISS;
-    in = in && inside;
-  } else if (valid) {
+  double ai = 0.0;
+  if (valid) {
     const double rx = __dsub_rn(V.xo, __ldg(P.xs + ix));
     const double ry = __dsub_rn(V.yo, __ldg(P.ys + iy));
     r = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)), V.rz2));
@@ -267,92 +296,86 @@ __device__ __forceinline__ void term_step(const RectParams &P, const ElemView &V
   }
   if (SKIP) {
     if (!__any_sync(0xffffffffu, in)) return;  // no term of this step lands in the SIR
-    if (PLAIN) {
-      ai = rect_amplitude(P, V.w, r, rh);
-    } else {
-      ai = __ddiv_rn(V.w, __dmul_rn(RECT_TWO_PI, r));
-      ai = __ddiv_rn(ai, P.dt);
-      ai = __dmul_rn(ai, 1000.0);
-    }
+    ai = __ddiv_rn(V.w, __dmul_rn(RECT_TWO_PI, r));
+    ai = __ddiv_rn(ai, P.dt);
+    ai = __dmul_rn(ai, 1000.0);
   }
-  // lanes adding into the same sample form a group; the others get unique keys
-  const unsigned long long key = in ? (unsigned long long)it : ~0ull - (unsigned long long)lane;
-  const unsigned int group = __match_any_sync(0xffffffffu, key);
-  const int len = __popc(group);
-  const bool leader = in && (group & ((1u << lane) - 1u)) == 0u;  // lowest lane of its group
-  // a run: the group's lanes are lane .. lane + len - 1
-  const bool run = (group >> lane) == (len == 32 ? 0xffffffffu : (1u << len) - 1u);
-  if (__all_sync(0xffffffffu, !leader || run)) {
-    stage[lane] = ai;
-    __syncwarp();
-    if (leader) {
-      double acc = __dadd_rn(h[it], ai);
-      const double *q = stage + lane + 1;
-      int k = len - 1;
-      for (; k >= 4; k -= 4, q += 4) {
-        acc = __dadd_rn(acc, q[0]);
-        acc = __dadd_rn(acc, q[1]);
-        acc = __dadd_rn(acc, q[2]);
-        acc = __dadd_rn(acc, q[3]);
-      }
-      for (; k > 0; k--, q++) acc = __dadd_rn(acc, q[0]);
-      h[it] = acc;
-    }
-  } else {
-    // each leader walks its group's lanes in ascending order (its own first);
-    // the warp takes as many steps as the largest group has members
-    const unsigned int steps = __reduce_max_sync(0xffffffffu, leader ? (unsigned)len : 0u);
-    double acc = leader ? h[it] : 0.0;
-    unsigned int rem = leader ? group : 0u;
-    for (unsigned int k = 0; k < steps; k++) {
-      const int src = rem ? __ffs(rem) - 1 : lane;
-      const bool add = rem != 0u;
-      rem &= rem - 1u;
-      const double aj = __shfl_sync(0xffffffffu, ai, src);
-      if (add) acc = __dadd_rn(acc, aj);
-    }
-    if (leader) h[it] = acc;
+  ordered_adds(in, (unsigned long long)it, ai, h + it, lane, stage);
+}
+
+// The same step for an element that is term_plain, at a surface element whose
+// centre differs by rx from the point in x and by ry2 squared in y; c0 as for
+// rect_number. hits counts the terms added (the others are out of bounds).
+template <bool SKIP>
+__device__ __forceinline__ void plain_step(const RectParams &P, const ElemView &V, double c0, bool valid, double rx,
+                                           double ry2, int lane, int w0, int wn, double *h, double *stage,
+                                           unsigned int &hits, unsigned int &flags) {
+  double rh;
+  const double r = rect_root(__dadd_rn(__dadd_rn(__dmul_rn(rx, rx), ry2), V.rz2), rh);
+  double ai = SKIP ? 0.0 : rect_amplitude(P, V.w, r, rh);
+  const int q = rect_number(P, r, c0);
+  int it = q >> RECT_FB;
+  if (rect_near(q)) it = __double2int_rn(rect_q(r, V.dl, P));
+  const unsigned int slot = (unsigned int)(it - w0);
+  const bool in = valid && slot < (unsigned int)wn;
+  hits += in ? 1u : 0u;
+  if (valid && !in && (unsigned int)it < (unsigned int)P.nt) flags |= RECT_MISS;  // not expected
+  if (SKIP) {
+    if (!__any_sync(0xffffffffu, in)) return;  // no term of this step lands in the SIR
+    ai = rect_amplitude(P, V.w, r, rh);
   }
-  __syncwarp();  // this step's sums (and stage reads) complete before the next step
+  ordered_adds(in, slot, ai, h + it, lane, stage);
 }
 
 // All terms of one element, 32 per step. P.row_steps: a step stays inside a row
 // (the sample index is monotone along it on either side of the point's
 // projection, so equal samples are neighbours); else steps run on across rows.
-template <bool SKIP, bool PLAIN>
-__device__ __forceinline__ void element_steps(const RectParams &P, const ElemView &V, int lane, int64_t w0, int64_t w1,
-                                              double *h, double *stage, unsigned long long &oob, unsigned int &flags,
-                                              bool last) {
-  if (P.row_steps) {
-    for (int iy = 0; iy < P.ny; iy++)
-      for (int ix = 0; ix < P.nx; ix += 32)
-        term_step<SKIP, PLAIN>(P, V, ix + lane < P.nx, ix + lane, iy, lane, w0, w1, h, stage, oob, flags, last);
-    return;
-  }
-  const int64_t E = (int64_t)P.nx * P.ny;
-  // this lane's surface element e = iy*nx + ix, advanced by 32 per step without a division
-  int iy = lane / P.nx;
-  int ix = lane - iy * P.nx;
-  for (int64_t e0 = 0; e0 < E; e0 += 32) {
-    term_step<SKIP, PLAIN>(P, V, e0 + lane < E, ix, iy, lane, w0, w1, h, stage, oob, flags, last);
-    ix += 32;
-    while (ix >= P.nx) {  // once for rows of 32 or more elements
-      ix -= P.nx;
-      iy++;
-    }
-  }
-}
 template <bool SKIP>
 __device__ __forceinline__ void element_terms(const RectParams &P, const ElemView &V, int lane, int64_t w0, int64_t w1,
                                               double *h, double *stage, unsigned long long &oob, unsigned int &flags,
                                               bool last) {
-  if (term_plain(P, V)) element_steps<SKIP, true>(P, V, lane, w0, w1, h, stage, oob, flags, last);
-  else element_steps<SKIP, false>(P, V, lane, w0, w1, h, stage, oob, flags, last);
+  const int64_t E = (int64_t)P.nx * P.ny;
+  const bool plain = term_plain(P, V);
+  if (plain) {
+    const double c0 = __fma_rn(-V.dl, P.inv_dt, RECT_MAGIC);
+    const int lo = (int)w0, wn = (int)(w1 - w0);
+    unsigned int hits = 0;
+    if (P.row_steps) {
+      for (int iy = 0; iy < P.ny; iy++) {
+        const double ry = __dsub_rn(V.yo, __ldg(P.ys + iy)), ry2 = __dmul_rn(ry, ry);
+        for (int x0 = 0; x0 < P.nx; x0 += 32) {
+          const int ix = x0 + lane;
+          const double rx = __dsub_rn(V.xo, __ldg(P.xs + min(ix, P.nx - 1)));
+          plain_step<SKIP>(P, V, c0, ix < P.nx, rx, ry2, lane, lo, wn, h, stage, hits, flags);
+        }
+      }
+    } else {
+      // this lane's surface element e = iy*nx + ix, advanced by 32 per step without a division
+      int iy = lane / P.nx, ix = lane - iy * P.nx;
+      for (int64_t e0 = 0; e0 < E; e0 += 32) {
+        const bool valid = e0 + lane < E;
+        const double rx = __dsub_rn(V.xo, __ldg(P.xs + ix)), ry = __dsub_rn(V.yo, __ldg(P.ys + (valid ? iy : 0)));
+        plain_step<SKIP>(P, V, c0, valid, rx, __dmul_rn(ry, ry), lane, lo, wn, h, stage, hits, flags);
+        for (ix += 32; ix >= P.nx; ix -= P.nx) iy++;  // once for rows of 32 or more elements
+      }
+    }
+    const unsigned long long missed = (unsigned long long)E - warp_sum_u64(hits);
+    if (lane == 0 && missed) {
+      oob += missed;
+      if (last) flags |= RECT_LAST_OOB;
+    }
+    return;
+  }
+  int iy = lane / P.nx, ix = lane - iy * P.nx;
+  for (int64_t e0 = 0; e0 < E; e0 += 32) {
+    term_step<SKIP>(P, V, e0 + lane < E, ix, iy, lane, w0, w1, h, stage, oob, flags, last);
+    for (ix += 32; ix >= P.nx; ix -= P.nx) iy++;
+  }
 }
 
 // ARR = false: dreamrect (one element at the origin, P.M == 1), ARR = true: arrays.
 template <bool ARR>
-__global__ void __launch_bounds__(RECT_WARPS * 32) rect_kernel(const RectParams P) {
+__global__ void __launch_bounds__(RECT_WARPS * 32, 4) rect_kernel(const RectParams P) {
   extern __shared__ __align__(16) double rect_dyn[];  // [warps][32] staged amplitudes, then [warps][P.win]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double *stage = rect_dyn + warp * 32;
@@ -864,7 +887,7 @@ int rect_device(RectBuffers &rb, const double *dRo, int64_t No, double a, double
   P.inv_dt = 1.0 / dt;
   P.k1 = P.c1 * P.inv_dt;
   const auto ranged = [](double v) { return std::fabs(v) > 0x1p-100 && std::fabs(v) < 0x1p100; };
-  P.plain_range = ranged(dt) && ranged(cp) && ranged(P.c1) && ranged(P.inv_dt);
+  P.plain_range = nt <= INT32_MAX && ranged(dt) && ranged(cp) && ranged(P.c1) && ranged(P.inv_dt);
   P.ab = std::fabs(a) + std::fabs(b);
   P.nt = nt;
   P.delay = ddelay;
@@ -876,8 +899,8 @@ int rect_device(RectBuffers &rb, const double *dRo, int64_t No, double a, double
   const auto kernel = A.single ? rect_kernel<false> : rect_kernel<true>;
   if (e == cudaSuccess) e = ensure_smem(kernel, RECT_SMEM_MAX);
   // dreamrect: one point per lane where that is the faster form. With c windows on an SM a round takes about 1 + c/50
-  // times a lone warp's 71 ns per term; one warp per point takes 6.8 ps per term and point (both on the 60000-element
-  // field above: 8000 points 4.25 against 3.83 ms, 16000 4.28 against 6.8).
+  // times a lone warp's 71 ns per term; one warp per point takes 6.4 ps per term and point (both on the 60000-element
+  // field above: 8000 points 4.25 against 3.51 ms, 16000 4.28 against 6.3).
   const int64_t lane_win = A.single ? window_bound(el, a, b, dt, cp, nt) : 0, lane_smem = (lane_win + 1) * 32 * 8;
   bool lanes = false;
   if (A.single && nt <= INT32_MAX && lane_smem <= RECT_SMEM_MAX) {
@@ -886,12 +909,12 @@ int rect_device(RectBuffers &rb, const double *dRo, int64_t No, double a, double
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t c = std::min<int64_t>(16, (227 * 1024) / (lane_smem + 1024));
     const int64_t rounds = (No + 32 * c * sms - 1) / (32 * c * sms);
-    lanes = (double)rounds * (1.0 + 0.02 * c) * 10440.0 < (double)No;
+    lanes = (double)rounds * (1.0 + 0.02 * c) * 11100.0 < (double)No;
   }
   if (lanes && e == cudaSuccess) e = ensure_smem(rect_lane_kernel, RECT_SMEM_MAX);
   // Steps that end with the rows where the lanes this leaves idle cost less than the steps that straddle two rows (and
   // whose equal samples are then no neighbours): 30-element rows of arrays 10.1 against 14.4 ms, 200-element rows of
-  // one element 38.0 against 36.4, 8-element rows 0.77 against 0.30.
+  // one element 38.0 against 36.4, 8-element rows 0.77 against 0.30 (IEEE root and 64-bit samples in all of these).
   P.row_steps = nx >= 20 && (nx % 32 == 0 || nx % 32 > 10);
   for (int full = 0; full < 2 && e == cudaSuccess; full++) {
     int64_t win = full ? 0 : window_bound(el, a, b, dt, cp, nt);
