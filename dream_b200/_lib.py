@@ -31,6 +31,7 @@ LVL_NONE, LVL_IGNORE, LVL_WARN, LVL_STOP = 0, 1, 2, 3
 DELAY_SINGLE, DELAY_MULTIPLE = 0, 1
 CONV_EQU, CONV_SUM, CONV_NEG = 0, 1, 2
 PREC_F64, PREC_F32, PREC_F32_STORE, PREC_BF16_STORE = 0, 1, 2, 3
+CG_SCRATCH_BYTES = 8256
 
 # every symbol include/dream_das.h declares: name -> (restype, argtypes)
 _i, _i64, _d, _vp = ctypes.c_int, ctypes.c_int64, ctypes.c_double, ctypes.c_void_p
@@ -56,6 +57,8 @@ SIGNATURES = {
     "dream_das_uni_run_device": (_i, [_vp, _vp, _pd, _d, _d, _d, _vp, _i, _pi64, _vp]),
     "dream_das_set_grid_hint": (_i, [_vp, _i64]),
     "dream_das_detect_grid": (_i, [_vp, _vp, _pi64, _vp]),
+    "dream_das_cg_start": (_i, [_vp, _i64, _vp, _i, _vp]),
+    "dream_das_cg_step": (_i, [_vp, _vp, _vp, _vp, _i64, ctypes.c_float, _vp, _vp, _i, _vp]),
     "dream_das_set_tile": (_i, [_vp, _i, _i]),
     "dream_das_set_chunk": (_i, [_vp, _i]),
     "dream_das_set_inner_shard": (_i, [_vp, _i64, _i64]),

@@ -202,6 +202,10 @@ def cg_reconstruct(op: DASOperator, Y, w, lam: float = 1e-3, iters: int = 30, x0
     x = torch.zeros_like(b) if x0 is None else x0.clone()
     r = b - (op.forward(op.adjoint(x, w), w) + lam * x) if x0 is not None else b.clone()
     p = r.clone()
+    dual = x0 is not None and torch.autograd.forward_ad.unpack_dual(x0).tangent is not None
+    if type(op) is DASOperator and isinstance(lam, (int, float)) and iters > 0 and not dual \
+            and _same_vectors(b, x, r, p):
+        return x, _cg_steps(op, w, float(lam), iters, x, r, p)
     rs = torch.dot(r, r)
     hist = []
     for _ in range(iters):
@@ -214,6 +218,29 @@ def cg_reconstruct(op: DASOperator, Y, w, lam: float = 1e-3, iters: int = 30, x0
         p = r + (rs_new / rs) * p
         rs = rs_new
     return x, torch.stack(hist).sqrt() if hist else torch.zeros(0, device=b.device)
+
+
+def _same_vectors(*vs):
+    """Plain contiguous FP32 vectors like the first, no part of a graph: what
+    the native updates work on in place. An x0 of another type or layout, or
+    one that carries gradients, is left to torch."""
+    return all(type(v) is torch.Tensor and v.dtype == torch.float32 and v.shape == vs[0].shape
+               and v.device == vs[0].device and v.is_contiguous() and not v.requires_grad for v in vs)
+
+
+def _cg_steps(op, w, lam, iters, x, r, p):
+    """Iterations of ``cg_reconstruct`` on x, r and p in place (csrc/cg.cu);
+    returns the residual norms."""
+    w = op._weights(w)
+    rs = torch.empty(iters, dtype=torch.float32, device=x.device)
+    scratch = torch.empty(_lib.CG_SCRATCH_BYTES, dtype=torch.uint8, device=x.device)
+    n, dev, stream = x.numel(), op.device.index, op._stream()
+    _lib.check(op._L.dream_das_cg_start(_p(r), n, _p(scratch), dev, stream))
+    for i in range(iters):
+        Ap = op.forward(op.adjoint(p, w), w)
+        _lib.check(op._L.dream_das_cg_step(_p(x), _p(r), _p(p), _p(Ap), n, lam, ctypes.c_void_p(rs.data_ptr() + 4 * i),
+                                           _p(scratch), dev, stream))
+    return rs.sqrt()
 
 
 class CGGraph:

@@ -310,6 +310,22 @@ int dream_das_op_backward(dream_das_plan *plan, const float *dG, const float *dY
                           float *dYgrad, float *dWgrad, void *stream);
 
 /*
+ * Vector updates of conjugate gradients on (A + lam I) x = b around an
+ * operator that the caller applies, for n FP32 values, FP64 dot products and
+ * CUDA device `device`. cg_start sets up d_scratch (DREAM_CG_SCRATCH_BYTES on
+ * the device, 8-byte aligned, one per solve) from the first residual r. cg_step
+ * takes d_Ap = A p (overwritten) and makes
+ *   Ap += lam p,  alpha = <r,r> / <p,Ap>,  x += alpha p,  r -= alpha Ap,
+ *   *d_rs = <r,r>,  p = r + (<r,r> / its last value) p.
+ * Both are asynchronous on `stream` and may be captured; the calls of one
+ * solve have to be ordered.
+ */
+#define DREAM_CG_SCRATCH_BYTES 8256
+int dream_das_cg_start(const float *d_r, int64_t n, void *d_scratch, int device, void *stream);
+int dream_das_cg_step(float *d_x, float *d_r, float *d_p, float *d_Ap, int64_t n, float lam, float *d_rs,
+                      void *d_scratch, int device, void *stream);
+
+/*
  * Batched DAS: many frames of uneven element counts, A-scan lengths and
  * image sizes in ONE persistent launch. No reference counterpart (the
  * reference beamforms one frame per call); each frame has the meaning of
