@@ -503,22 +503,21 @@ int launch_fast_plan(dream_das_plan *p, const void *dY, const void *dRo, const v
   const int64_t slow_tiles = (F.n_slow + F.tile_s - 1) / F.tile_s;
   const int64_t chunk = slow_tile_chunk(F, tpp);
   // L2 blocking: A-scans larger than the budget are beamformed in passes over
-  // ranges of inner elements (multiples of the 16-term register chunk), each
+  // ranges of inner elements (multiples of 16), each
   // pass adding its terms into the image, so the A-scans of one pass stay in
   // L2 while every image point gathers from them.
   const int n_in = (method == DREAM_DAS_RCA_ROWTX) ? F.Nt : F.Nr;
   if (!apply_shard(p, F)) return 0;  // Y holds the columns of inner elements [shard_lo, shard_hi) only
   const int64_t col_bytes = (int64_t)n_out * p->K * (bf16 ? 2 : 4);  // A-scans of one inner element
   const int64_t y_bytes = col_bytes * n_in;
-  // automatic: once the A-scans exceed 112 MB (most of the 126 MB L2), even
-  // passes of at most 96 MB, widths multiples of the 16-term register chunk
-  // (RCA 128x128, K 4096: FP32 268 MB in passes of 48/48/32 columns, 51.6 ->
-  // 40.0 ms; BF16 134 MB in two of 64, 36.7 -> 34.5 ms; smaller passes lose
-  // more to the per-pass leg set-up than they gain in L2 hits)
-  const int64_t budget = p->l2_block > 0 ? p->l2_block : (int64_t(96) << 20);
-  const int64_t split_above = p->l2_block > 0 ? budget : (int64_t(112) << 20);
+  // automatic: even passes of at most 136 MB, a little more than the 126 MB L2,
+  // widths multiples of 16 columns (RCA 128x128, K 4096, 128x128x256 points: FP32
+  // 268 MB in two passes 25.6 ms, in three 26.5, in five 27.5; one pass 25.1, but
+  // 3.8 against 3.6 for 64x64x128 points, which lie further apart; BF16 134 MB in
+  // one pass 11.6, in two 11.9: a pass sets up its legs again)
+  const int64_t budget = p->l2_block > 0 ? p->l2_block : (int64_t(136) << 20);
   int pass_w = n_in;
-  if (in_hi == 0 && p->l2_block >= 0 && y_bytes > split_above) {
+  if (in_hi == 0 && p->l2_block >= 0 && y_bytes > budget) {
     const int64_t n_pass = (y_bytes + budget - 1) / budget;
     pass_w = (int)std::max<int64_t>(16, ((n_in + n_pass - 1) / n_pass + 15) / 16 * 16);
     pass_w = std::min(pass_w, n_in);

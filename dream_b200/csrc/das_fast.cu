@@ -336,8 +336,9 @@ struct LegBounds {
   __device__ __forceinline__ double max_leg() const { return __hiloint2double(word(hi), hi < 0 ? 0 : -1); }
 };
 
-// The image point of this thread (inactive lanes repeat the tile's first point).
-__device__ __forceinline__ int64_t tile_point(const FastParams &P, int64_t tfi, int64_t tsi, bool &active) {
+// The image point of this thread (inactive lanes repeat the tile's first point);
+// lines in the order of volume_line.
+__device__ __forceinline__ int64_t tile_point(const FastParams &P, int64_t tfi, int64_t tsi, uint32_t row, bool &active) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int lf = lane % P.wf, ls = lane / P.wf;
   const int warps_f = P.tile_f / P.wf;
@@ -345,7 +346,15 @@ __device__ __forceinline__ int64_t tile_point(const FastParams &P, int64_t tfi, 
   const int64_t f = tfi * P.tile_f + wfi * P.wf + lf;
   const int64_t s = tsi * P.tile_s + wsi * (32 / P.wf) + ls;
   active = f < P.n_fast && s < P.n_slow;
-  return active ? s * P.n_fast + f : tsi * P.tile_s * P.n_fast + tfi * P.tile_f;
+  return active ? volume_line(s, row, P.n_slow) * P.n_fast + f
+                : volume_line(tsi * P.tile_s, row, P.n_slow) * P.n_fast + tfi * P.tile_f;
+}
+
+// Whether a block looks for rows of lines: RCAs, which image volumes, with terms
+// enough to pay for the search.
+template <int METHOD>
+__device__ __forceinline__ bool volume_tiles(const FastParams &P) {
+  return METHOD != TFM && P.Nt * P.Nr >= VOLUME_TERMS;
 }
 
 // The legs of one side of a method's term: a point element (TFM), a column or a
@@ -394,9 +403,15 @@ __device__ __forceinline__ void gather_tile(const FastParams &P, int64_t tfi, in
   const int i_lo = P.in_lo, i_hi = P.in_hi > 0 ? P.in_hi : n_in;
   const int64_t ostride = P.ycol_o > 0 ? P.ycol_o : n_in;  // columns per outer element
   bool active;
-  const int64_t no = tile_point(P, tfi, tsi, active);
+  __shared__ uint32_t s_row;
+  if (METHOD != TFM) {
+    const uint32_t row = volume_tiles<METHOD>(P) ? volume_row(P.Ro, P.No, P.n_fast, P.n_slow) : 0;
+    if (threadIdx.x == 0) s_row = row;
+    __syncthreads();
+  }
+  auto point = [&]() { return tile_point(P, tfi, tsi, METHOD != TFM ? *(volatile uint32_t *)&s_row : 0, active); };
   Pixel px;
-  pixel_of(P, no, px);
+  pixel_of(P, point(), px);
   // 2^52 + j * K, read from shared memory: as uniform values each use would move them to a register first
   double mag[GATHER_JC];
 #pragma unroll
@@ -503,6 +518,7 @@ __device__ __forceinline__ void gather_tile(const FastParams &P, int64_t tfi, in
       }
     }
   }
+  const int64_t no = point();  // worked out again: the loop has no register for it
   if (active) P.Im[no] = P.accumulate ? P.Im[no] + (acc_s + acc_c) : acc_s + acc_c;
   add_count(P.oob, active ? oob : 0u);
 }
@@ -994,7 +1010,8 @@ __global__ void __launch_bounds__(256, 2) das_scatter_kernel(const FastParams P,
   int *win = reinterpret_cast<int *>(smem_raw + scatter_head_bytes(n_out, n_in));
   double *legs = reinterpret_cast<double *>(smem_raw + scatter_head_bytes(n_out, n_in) + SCATTER_WIN_BYTES);
   bool active;
-  const int64_t no = tile_point(P, blockIdx.x, (int64_t)blockIdx.y + P.slow_tile0, active);
+  const uint32_t row = volume_tiles<METHOD>(P) ? volume_row(P.Ro, P.No, P.n_fast, P.n_slow) : 0;
+  const int64_t no = tile_point(P, blockIdx.x, (int64_t)blockIdx.y + P.slow_tile0, row, active);
   Pixel px;
   pixel_of(P, no, px);
   ScatterTile T;

@@ -44,7 +44,7 @@ constexpr int plain_tile_threads(int64_t n_in, size_t elem) {
   return plain_table_bytes(n_in, elem, bd) <= 200 * 1024 ? bd : 0;
 }
 // Tile of image points of such a block on a hinted grid.
-constexpr int plain_tile_f(int method, int threads) { return (threads >= 128 ? 2 : 1) * plain_patch_f(method); }
+constexpr int plain_tile_f(int method, int threads) { return threads >= 128 ? 8 : plain_patch_f(method); }
 constexpr int plain_tile_s(int method, int threads) { return threads / plain_tile_f(method, threads); }
 
 struct PlainLaunch {

@@ -305,13 +305,17 @@ __global__ void __launch_bounds__(BD, MINB * 128 / BD) das_plain_tile_kernel(con
   int64_t no_raw, first;
   bool active;
   if (P.n_fast > 0) {
-    constexpr int PF = plain_patch_f(M), TF = plain_tile_f(M, BD), WF = TF / PF;  // lanes, points, warps along the fast axis
-    const int64_t f0 = (int64_t)blockIdx.x * TF, s0 = (P.no0 + blockIdx.y) * plain_tile_s(M, BD);
-    const int64_t f = f0 + (warp % WF) * PF + lane % PF;
-    const int64_t s = s0 + (warp / WF) * (32 / PF) + lane / PF;
+    constexpr int TF = plain_tile_f(M, BD), TS = plain_tile_s(M, BD);
+    // patches of 8 x 4 points become 4 x 8 where a volume's lines are neighbours in two directions
+    const uint32_t row =
+        !UNI && M != TFM && P.Nt * P.Nr >= VOLUME_TERMS ? volume_row(P.Ro, P.No, P.n_fast, P.n_slow) : 0;
+    const int pf = TS % 8 == 0 && row ? 4 : plain_patch_f(M), wf = TF / pf;  // lanes and warps along the fast axis
+    const int64_t f0 = (int64_t)blockIdx.x * TF, s0 = (P.no0 + blockIdx.y) * TS;
+    const int64_t f = f0 + (warp % wf) * pf + lane % pf;
+    const int64_t s = s0 + (warp / wf) * (32 / pf) + lane / pf;
     active = f < P.n_fast && s < P.n_slow;
-    no_raw = s * P.n_fast + f;
-    first = s0 * P.n_fast + f0;
+    no_raw = volume_line(s, row, P.n_slow) * P.n_fast + f;
+    first = volume_line(s0, row, P.n_slow) * P.n_fast + f0;
   } else {
     no_raw = P.no0 + (int64_t)blockIdx.x * BD + tid;
     active = no_raw < P.no1;

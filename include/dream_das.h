@@ -259,8 +259,8 @@ int dream_das_set_inner_shard(dream_das_plan *plan, int64_t lo, int64_t hi);
  * than the budget are beamformed in passes over ranges of inner elements (a
  * multiple of 16 each) whose A-scans take at most `bytes`, each pass adding
  * into the image: the pass's samples stay in L2 while every image point
- * gathers from them. 0 = automatic (passes of at most 96 MB when the A-scans
- * exceed 160 MB), < 0 = never split. The image changes only by FP32 rounding.
+ * gathers from them. 0 = automatic (even passes of at most 136 MB),
+ * < 0 = never split. The image changes only by FP32 rounding.
  */
 int dream_das_set_l2_block(dream_das_plan *plan, int64_t bytes);
 
