@@ -128,7 +128,7 @@ struct dream_das_plan {
   DevBuf bY, bRo, bGt, bGr, bDelay, bIm, bOob, bY16;
   int64_t n_fast = 0;          // grid hint (0: none)
   int tile_f = 0, tile_s = 0;  // user / autotuner tile (0: automatic)
-  int jc = 0;                  // user / autotuner inner chunk (0: automatic)
+  int jc = 0;                  // inner chunk asked for (kept, without effect: the kernels have one)
   int64_t l2_block = 0;        // A-scan bytes per inner-element pass (0: automatic, < 0: never split)
   // inner-element shard: Y holds only inner elements [shard_lo, shard_hi) (0, 0: all of them)
   int64_t shard_lo = 0, shard_hi = 0;
@@ -355,9 +355,9 @@ int zero_length_ascans(dream_das_plan *p, void *dIm, unsigned long long *doob, c
 // Tile of the operator's adjoint: the user's, or on a hinted TFM grid 16 x 16
 // points (64x64 elements, 512x512 points 0.80 ms, 37x53 elements 0.35; 8 x 32
 // points 0.79 and 0.46), on an RCA volume 8 x 16, whose windows grow fastest with
-// the tile (128x128 elements, 128x128x256 points 61.4 ms; 8 x 8 93.9, 16 x 8
-// 81), on both 8 x 8 where that would leave SMs without a tile (64x64 elements,
-// 150x125 points 0.32 against 0.57 ms); 256 consecutive points without a hint.
+// the tile (128x128 elements, 128x128x256 points 54.7 ms; in tiles along one row
+// of lines 61.4, 8 x 8 93.9, 16 x 8 81), on both 8 x 8 where that would leave SMs
+// without a tile (64x64 elements, 150x125 points 0.32 against 0.57 ms); 256 consecutive points without a hint.
 void scatter_tile(const dream_das_plan *p, FastParams &F) {
   const bool hint = p->n_fast > 0;
   if (p->tile_f > 0) {
@@ -1259,7 +1259,8 @@ static void finish_read_back(void *Im, const void *staged, size_t bytes) {
 // multiples of 8 (at most 15). Every chunk's kernel recomputes the image
 // points' outer legs, so more, shorter chunks cost more than they save at the
 // ends of the pipeline: on the 64x64-element TFM frame from pinned memory,
-// 4 chunks of 16 take 1.50 ms, 8 of 8 take 1.94 ms and 8/16/16/16/8 1.55 ms.
+// (an earlier gather of 0.55 ms a frame) 4 chunks of 16 took 1.50 ms, 8 of 8
+// 1.94 and 8/16/16/16/8 1.55.
 static std::vector<int> upload_chunks(int n_in) {
   constexpr int UPLOAD_CHUNKS = 4;
   const int n = std::max(1, std::min({UPLOAD_CHUNKS, 15, (n_in + 7) / 8}));

@@ -223,7 +223,7 @@ __device__ __forceinline__ void leg_range(const FastParams &P, const TileBox &B,
 // 0.17 ms), the L1 data pipe at 0.46. Fixed-point legs with an ambiguity test
 // and an FP64 fallback, the form this replaces, took 0.505 ms there, 0.069
 // against 0.037 for 32x32 elements and 256x256 points (no per-tile set-up with
-// block barriers here), 38.0 against 27.3 for the 128x128-element RCA volume.
+// block barriers here), 38.0 against 25.6 for the 128x128-element RCA volume.
 //
 // Layout: 8 inner legs and the 8 addends of the truncation in registers, the
 // outer legs in shared memory (a thread reads only its own: no barrier), two
