@@ -354,7 +354,7 @@ __device__ __forceinline__ int64_t tile_point(const FastParams &P, int64_t tfi, 
 // enough to pay for the search.
 template <int METHOD>
 __device__ __forceinline__ bool volume_tiles(const FastParams &P) {
-  return METHOD != TFM && P.Nt * P.Nr >= VOLUME_TERMS;
+  return METHOD != TFM && (int64_t)P.Nt * P.Nr >= VOLUME_TERMS;
 }
 
 // The legs of one side of a method's term: a point element (TFM), a column or a

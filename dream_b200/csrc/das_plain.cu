@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(BD, MINB * 128 / BD) das_plain_tile_kernel(con
     constexpr int TF = plain_tile_f(M, BD), TS = plain_tile_s(M, BD);
     // patches of 8 x 4 points become 4 x 8 where a volume's lines are neighbours in two directions
     const uint32_t row =
-        !UNI && M != TFM && P.Nt * P.Nr >= VOLUME_TERMS ? volume_row(P.Ro, P.No, P.n_fast, P.n_slow) : 0;
+        !UNI && M != TFM && (int64_t)P.Nt * P.Nr >= VOLUME_TERMS ? volume_row(P.Ro, P.No, P.n_fast, P.n_slow) : 0;
     const int pf = TS % 8 == 0 && row ? 4 : plain_patch_f(M), wf = TF / pf;  // lanes and warps along the fast axis
     const int64_t f0 = (int64_t)blockIdx.x * TF, s0 = (P.no0 + blockIdx.y) * TS;
     const int64_t f = f0 + (warp % wf) * pf + lane % pf;
