@@ -1028,20 +1028,31 @@ __global__ void __launch_bounds__(256, 2) das_scatter_kernel(const FastParams P,
   const int64_t ostride = P.ycol_o > 0 ? P.ycol_o : n_in;
   const double Kf = (double)P.K;
   double *tab = legs + threadIdx.x;
-  const bool plain = T.usable && T.in_bounds && P.K < (int64_t(1) << 28);  // sample numbers of a chunk fit 32 bits
+  // Terms without a test: sample numbers of a chunk fit 32 bits, the tile's leg ranges lie inside the A-scan, and this
+  // point's own legs inside those ranges (a NaN point's are not, and the box of the tile's points does not show it).
+  const bool plain = T.usable && T.in_bounds && P.K < (int64_t(1) << 28);
   for (int o0 = 0; o0 < n_out; o0 += P.out_block) {
     const int on = min(P.out_block, n_out - o0);
-    for (int o = 0; o < on; o++) tab[o * blockDim.x] = outer(P, px, o0 + o);
+    bool outer_in = plain;
+    for (int o = 0; o < on; o++) {
+      const double l = outer(P, px, o0 + o);
+      outer_in = outer_in && leg_inside(l, P.Fs, T.be[o0 + o]);
+      tab[o * blockDim.x] = l;
+    }
     for (int i0 = i_lo; i0 < i_hi; i0 += SCATTER_JC) {
       const int jn = min(SCATTER_JC, i_hi - i0);
       double B[SCATTER_JC];
+      bool in = outer_in && jn == SCATTER_JC;
 #pragma unroll
-      for (int j = 0; j < SCATTER_JC; j++) B[j] = j < jn ? inner(P, px, i0 + j) : 0.0;
+      for (int j = 0; j < SCATTER_JC; j++) {
+        B[j] = j < jn ? inner(P, px, i0 + j) : 0.0;
+        in = in && leg_inside(B[j], P.Fs, T.be[n_out + (j < jn ? i0 + j : i0)]);
+      }
       for (int o = 0; o < on; o++) {
         const double a = tab[o * blockDim.x];
         const int64_t col = (o0 + o) * ostride + ycol_inner(P, i0);
         float *y = Ya + col * P.K;
-        if (plain && jn == SCATTER_JC) {
+        if (in) {
 #pragma unroll
           for (int j = 0; j < SCATTER_JC; j++) {
             const double p = __dmul_rn(__dadd_rn(a, B[j]), P.Fs);
