@@ -876,25 +876,37 @@ __device__ __forceinline__ void scatter_windows(const FastParams &P, const Scatt
   const Legs<METHOD, true> outer(P);
   const Legs<METHOD, false> inner(P);
   const double Fs = P.Fs, Kf = (double)K;
-  const bool aligned = (K & 3) == 0 && (reinterpret_cast<uintptr_t>(Ya) & 15) == 0;  // rows start on 16 bytes
+  const int64_t ostride = P.ycol_o > 0 ? P.ycol_o : n_in;  // columns per outer element
+  bool vectors = (K & 3) == 0 && (reinterpret_cast<uintptr_t>(Ya) & 15) == 0;  // rows start on 16 bytes
   double *tab = legs + tid;  // leg of outer element o0 + o: tab[o * nthr]
   // fixed-point scale of the tile: max |x| < 2^E, values scaled by 2^(22 - E)
   float mx = fabsf(xn_f);
   for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  uint32_t w_mx = 0;  // bits of the largest |weight|, NaN above all
+  if (WEIGHTED) {
+#pragma unroll 8
+    for (int64_t c = tid; c < n_out * ostride; c += nthr) w_mx = max(w_mx, __float_as_uint(__ldg(P.w + c)) & 0x7fffffffu);
+    w_mx = __reduce_max_sync(0xffffffffu, w_mx);
+  }
   __shared__ float s_mx[8];
-  if ((tid & 31) == 0) s_mx[tid >> 5] = mx;
+  __shared__ uint32_t s_w[8];
+  if ((tid & 31) == 0) s_mx[tid >> 5] = mx, s_w[tid >> 5] = w_mx;
   for (int e = tid; e < 2 * ROWS * WS; e += nthr) win[e] = 0;
   __syncthreads();
   mx = 0.0f;
-  for (int w = 0; w < (nthr >> 5); w++) mx = fmaxf(mx, s_mx[w]);
+  for (int w = 0; w < (nthr >> 5); w++) {
+    mx = fmaxf(mx, s_mx[w]);
+    w_mx = max(w_mx, s_w[w]);
+  }
   if (mx == 0.0f) return;  // nothing to add
   int E;
   frexpf(mx, &E);
   const float qscale = ldexpf(1.0f, 22 - E), iS = ldexpf(1.0f, E - 22);
   const int xn = __float2int_rn(xn_f * qscale);
+  // A row flushed in vectors adds 0 * (scale * weight) to its cells without a term: only where that is 0.
+  if (WEIGHTED) vectors = vectors && isfinite(iS * __uint_as_float(w_mx));
   // flush: a fixed group of nthr / ROWS threads per window row (q, j)
   const int tpr = nthr / ROWS, fr = tid / tpr, fq = tid - fr * tpr, fro = fr / JC, fri = fr % JC;
-  const int64_t ostride = P.ycol_o > 0 ? P.ycol_o : n_in;  // columns per outer element
   const int64_t ystep = SCATTER_NO * ostride * K;
   const uint32_t win_a = (uint32_t)__cvta_generic_to_shared(win);
   uint32_t buf = 0;  // byte offset of the batch's buffer
@@ -975,7 +987,7 @@ __device__ __forceinline__ void scatter_windows(const FastParams &P, const Scatt
         // samples kb + t of the row; its terms lie in the first ext_o + ext_i + 3 cells
         const int wr = flush ? be_o.y + be_r.y + 4 : 0;
         const int64_t kb = (int64_t)be_o.x + be_r.x;  // a multiple of 4
-        if (aligned && kb >= 0 && kb + ((wr + 3) & ~3) <= K) {
+        if (vectors && kb >= 0 && kb + ((wr + 3) & ~3) <= K) {
           int4 *wp = reinterpret_cast<int4 *>(reinterpret_cast<char *>(win) + buf) + (fr * WS >> 2) + fq;
           float *y = yrow + be_o.x + fq * 4;
           for (int t = fq * 4; t < wr; t += tpr * 4, wp += tpr, y += tpr * 4) {
