@@ -720,6 +720,8 @@ namespace {
 constexpr int SCATTER_JC = 8, SCATTER_NO = 2, SCATTER_ROWS = SCATTER_NO * SCATTER_JC;
 // Samples per window row; tiles of wider windows add every term with a global reduction.
 constexpr int SCATTER_WCAP = 192;
+// Smallest largest |x| of a tile of windows: its scale 2^(22 - E) and the inverse are normal FP32 numbers.
+constexpr float SCATTER_X_MIN = 0x1p-104f;
 
 // be of every element, then (16-byte aligned) the two window buffers, then the outer legs.
 __host__ __device__ constexpr size_t scatter_head_bytes(int n_out, int n_in) {
@@ -755,11 +757,13 @@ struct ScatterTile {
   bool low;                  // some term may lie before sample 0
   bool in_bounds;            // every term of the tile is in bounds
   int ext_outer, ext_inner;  // largest extents
+  float x_max;               // largest |x|, NaN above all
+  bool x_scales;             // the windows' fixed-point scale of x_max and its inverse are normal FP32 numbers
 };
 
-// Leg bounds of the tile; `scratch`: (blockDim.x / 32) * 8 doubles and as many ints.
-__device__ __forceinline__ void scatter_setup(const FastParams &P, const Pixel &px, unsigned char *smem, double *scratch,
-                                              int n_out, int n_in, int i_lo, int i_hi, ScatterTile &T) {
+// Leg bounds and value range of the tile; `scratch`: (blockDim.x / 32) * 8 doubles and as many ints.
+__device__ __forceinline__ void scatter_setup(const FastParams &P, const Pixel &px, float xn, unsigned char *smem,
+                                              double *scratch, int n_out, int n_in, int i_lo, int i_hi, ScatterTile &T) {
   const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
   T.be = reinterpret_cast<int2 *>(smem);
   double *red = scratch;
@@ -826,9 +830,10 @@ __device__ __forceinline__ void scatter_setup(const FastParams &P, const Pixel &
   hiA = __reduce_max_sync(0xffffffffu, hiA);
   loB = __reduce_min_sync(0xffffffffu, loB);
   hiB = __reduce_max_sync(0xffffffffu, hiB);
+  int x_mx = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(xn)));  // bits: in the values' order, NaN above all
   if (lane == 0) {
     int *s = stat + warp * 8;
-    s[0] = bad, s[1] = extA, s[2] = extB, s[3] = loA, s[4] = hiA, s[5] = loB, s[6] = hiB;
+    s[0] = bad, s[1] = extA, s[2] = extB, s[3] = loA, s[4] = hiA, s[5] = loB, s[6] = hiB, s[7] = x_mx;
   }
   __syncthreads();
   for (int w = 0; w < nwarps; w++) {
@@ -840,6 +845,7 @@ __device__ __forceinline__ void scatter_setup(const FastParams &P, const Pixel &
     hiA = max(hiA, s[4]);
     loB = min(loB, s[5]);
     hiB = max(hiB, s[6]);
+    x_mx = max(x_mx, s[7]);
   }
   __syncthreads();  // the scratch is read
   T.usable = !bad && loA <= hiA && loB <= hiB;
@@ -847,6 +853,8 @@ __device__ __forceinline__ void scatter_setup(const FastParams &P, const Pixel &
   T.in_bounds = !T.low && (int64_t)hiA + hiB + 2 < P.K;
   T.ext_outer = extA;
   T.ext_inner = extB;
+  T.x_max = __int_as_float(x_mx);
+  T.x_scales = T.x_max >= SCATTER_X_MIN && T.x_max < INFINITY;
 }
 
 // Whether a leg (ms) lies inside its window range (bases and extents leave a
@@ -879,28 +887,20 @@ __device__ __forceinline__ void scatter_windows(const FastParams &P, const Scatt
   const int64_t ostride = P.ycol_o > 0 ? P.ycol_o : n_in;  // columns per outer element
   bool vectors = (K & 3) == 0 && (reinterpret_cast<uintptr_t>(Ya) & 15) == 0;  // rows start on 16 bytes
   double *tab = legs + tid;  // leg of outer element o0 + o: tab[o * nthr]
-  // fixed-point scale of the tile: max |x| < 2^E, values scaled by 2^(22 - E)
-  float mx = fabsf(xn_f);
-  for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
   uint32_t w_mx = 0;  // bits of the largest |weight|, NaN above all
   if (WEIGHTED) {
 #pragma unroll 8
     for (int64_t c = tid; c < n_out * ostride; c += nthr) w_mx = max(w_mx, __float_as_uint(__ldg(P.w + c)) & 0x7fffffffu);
     w_mx = __reduce_max_sync(0xffffffffu, w_mx);
   }
-  __shared__ float s_mx[8];
   __shared__ uint32_t s_w[8];
-  if ((tid & 31) == 0) s_mx[tid >> 5] = mx, s_w[tid >> 5] = w_mx;
+  if ((tid & 31) == 0) s_w[tid >> 5] = w_mx;
   for (int e = tid; e < 2 * ROWS * WS; e += nthr) win[e] = 0;
   __syncthreads();
-  mx = 0.0f;
-  for (int w = 0; w < (nthr >> 5); w++) {
-    mx = fmaxf(mx, s_mx[w]);
-    w_mx = max(w_mx, s_w[w]);
-  }
-  if (mx == 0.0f) return;  // nothing to add
+  for (int w = 0; w < (nthr >> 5); w++) w_mx = max(w_mx, s_w[w]);
+  // fixed-point scale of the tile: max |x| < 2^E, values scaled by 2^(22 - E)
   int E;
-  frexpf(mx, &E);
+  frexpf(T.x_max, &E);
   const float qscale = ldexpf(1.0f, 22 - E), iS = ldexpf(1.0f, E - 22);
   const int xn = __float2int_rn(xn_f * qscale);
   // A row flushed in vectors adds 0 * (scale * weight) to its cells without a term: only where that is 0.
@@ -1026,14 +1026,16 @@ __global__ void __launch_bounds__(256, 2) das_scatter_kernel(const FastParams P,
   const int64_t no = tile_point(P, blockIdx.x, (int64_t)blockIdx.y + P.slow_tile0, row, active);
   Pixel px;
   pixel_of(P, no, px);
-  ScatterTile T;
-  scatter_setup(P, px, smem_raw, reinterpret_cast<double *>(win), n_out, n_in, i_lo, i_hi, T);
   const float xn = active ? __ldg(X + no) : 0.0f;
-  if (T.usable && T.ext_outer + T.ext_inner + 7 <= SCATTER_WCAP) {
-    scatter_windows<WEIGHTED, METHOD>(P, T, px, active, xn, Ya, win, legs, n_out, n_in, i_lo, i_hi);
+  ScatterTile T;
+  scatter_setup(P, px, xn, smem_raw, reinterpret_cast<double *>(win), n_out, n_in, i_lo, i_hi, T);
+  if (T.usable && T.ext_outer + T.ext_inner + 7 <= SCATTER_WCAP && (T.x_max == 0.0f || T.x_scales)) {
+    if (T.x_max > 0.0f)
+      scatter_windows<WEIGHTED, METHOD>(P, T, px, active, xn, Ya, win, legs, n_out, n_in, i_lo, i_hi);
     return;
   }
-  // windows wider than the shared-memory rows, or legs outside the integer range: every term added on its own
+  // windows wider than the shared-memory rows, legs outside the integer range, or values outside the windows'
+  // fixed-point range: every term added on its own
   if (!active) return;
   const Legs<METHOD, true> outer(P);
   const Legs<METHOD, false> inner(P);
