@@ -644,20 +644,13 @@ cudaError_t launch_batch(const FastParams *frames, const int4 *items, int n_item
   return cudaGetLastError();
 }
 
-// Sets the dynamic shared-memory limit; returns resident CTAs per SM (0 on error).
+// Raises the dynamic shared-memory limit where needed (never lowers it: an older
+// batch may need more); returns resident CTAs per SM (0 on error).
 int batch_prepare(size_t smem, bool bf16) {
+  auto kern = bf16 ? das_batch_kernel<__nv_bfloat16> : das_batch_kernel<float>;
+  if (ensure_smem(kern, smem) != cudaSuccess) return 0;
   int n = 0;
-  if (bf16) {
-    if (cudaFuncSetAttribute(das_batch_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem) != cudaSuccess)
-      return 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, das_batch_kernel<__nv_bfloat16>, 128, smem);
-  } else {
-    if (cudaFuncSetAttribute(das_batch_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, das_batch_kernel<float>, 128, smem);
-  }
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 128, smem);
   return n;
 }
 
