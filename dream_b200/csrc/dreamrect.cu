@@ -86,9 +86,12 @@ struct RectParams {
   const double *delay;
   int delay_multi;
   int full;               // every element live, windows [0, nt) in the output columns
+  int64_t *rest;          // points whose window one lane has no room for (in any order), and their number; rect_kernel
+  int64_t n_rest;         // takes these instead of all points when n_rest > 0
   double *H;
   unsigned long long *oob;        // out-of-bounds terms
   unsigned int *flags;            // RECT_MISS | RECT_LAST_OOB
+  unsigned long long *rest_count;
 };
 
 // The observation point as array element m sees it; `fast`: its sample
@@ -380,8 +383,9 @@ __global__ void __launch_bounds__(RECT_WARPS * 32, 4) rect_kernel(const RectPara
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double *stage = rect_dyn + warp * 32;
   double *win_sm = rect_dyn + (blockDim.x >> 5) * 32 + (int64_t)warp * P.win;
-  const int64_t n = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
-  if (n >= P.No) return;  // whole warps only: no block-wide barrier below
+  int64_t n = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
+  if (n >= (P.n_rest > 0 ? P.n_rest : P.No)) return;  // whole warps only: no block-wide barrier below
+  if (P.n_rest > 0) n = P.rest[n];
   double *out = P.H + n * P.nt;
   ElemView V;
   // union of the live elements' windows
@@ -522,10 +526,10 @@ __global__ void __launch_bounds__(32) rect_lane_kernel(const RectParams P) {
     w0 = max((int64_t)0, lo);
     w1 = max(w0, min(P.nt, hi));
   }
-  if (w1 - w0 > P.win) {  // not expected: the launch is repeated with the window in the output column
-    flags |= RECT_MISS;
-    w1 = w0;
-  }
+  // A point without trusted estimates (not a number, or very far away) has the window [0, nt). It is left to
+  // rect_kernel, and its lane adds nothing, whatever the warp computes for it.
+  const bool fits = w1 - w0 <= P.win;
+  if (!fits) w1 = w0;
   LaneSir S;
   S.trash = (unsigned int)__cvta_generic_to_shared(rect_dyn + lane);
   S.first = S.trash + 256u;
@@ -535,7 +539,7 @@ __global__ void __launch_bounds__(32) rect_lane_kernel(const RectParams P) {
   __syncwarp();
   if (!__any_sync(0xffffffffu, S.wn > 0)) {  // no term in bounds
     oob = E;
-  } else if (__all_sync(0xffffffffu, term_plain(P, V))) {
+  } else if (__all_sync(0xffffffffu, term_plain(P, V) || !fits)) {
     const double c0 = __fma_rn(-V.dl, P.inv_dt, RECT_MAGIC);
     int q_min = INT_MAX, q_max = INT_MIN;
     int iy = 0, left = P.nx;  // row and terms left in it
@@ -624,7 +628,8 @@ __global__ void __launch_bounds__(32) rect_lane_kernel(const RectParams P) {
     oob = E - S.hits;
   }
   if (oob) flags |= RECT_LAST_OOB;
-  if (!active) {
+  if (active && !fits) P.rest[atomicAdd(P.rest_count, 1ull)] = first + lane;
+  if (!active || !fits) {
     oob = 0;
     flags = 0;
   }
@@ -665,8 +670,9 @@ int rect_centres(double a, double b, double dx, double dy, std::vector<double> &
 struct RectBuffers {
   std::mutex mu;
   double *centres = nullptr, *Ro = nullptr, *delay = nullptr, *H = nullptr, *elems = nullptr;
-  size_t cap_c = 0, cap_ro = 0, cap_d = 0, cap_h = 0, cap_e = 0;
-  unsigned long long *ctr = nullptr;  // [0] out-of-bounds terms, [1] RECT_* flags (low word)
+  double *rest = nullptr;  // point numbers (RectParams::rest)
+  size_t cap_c = 0, cap_ro = 0, cap_d = 0, cap_h = 0, cap_e = 0, cap_r = 0;
+  unsigned long long *ctr = nullptr;  // [0] out-of-bounds terms, [1] RECT_* flags (low word), [2] points in rest
   cudaStream_t st = nullptr;
 };
 
@@ -854,7 +860,7 @@ int rect_device(RectBuffers &rb, const double *dRo, int64_t No, double a, double
   }
   if (dRo == nullptr || ddelay == nullptr || dH == nullptr) return set_last_error(DREAM_ERR_ARGUMENT, "NULL pointer");
   cudaError_t e = cudaSuccess;
-  if (rb.ctr == nullptr && (e = cudaMalloc(&rb.ctr, 2 * sizeof(unsigned long long))) != cudaSuccess)
+  if (rb.ctr == nullptr && (e = cudaMalloc(&rb.ctr, 3 * sizeof(unsigned long long))) != cudaSuccess)
     return set_last_error(DREAM_ERR_ALLOC, cudaGetErrorString(e));
   if (terms == 0) {  // no surface element: the SIRs are zero
     e = cudaMemsetAsync(dH, 0, (size_t)No * nt * 8, st);
@@ -895,7 +901,9 @@ int rect_device(RectBuffers &rb, const double *dRo, int64_t No, double a, double
   P.H = dH;
   P.oob = rb.ctr;
   P.flags = reinterpret_cast<unsigned int *>(rb.ctr + 1);
-  unsigned long long h_ctr[2] = {0, 0};
+  P.rest_count = rb.ctr + 2;
+  P.n_rest = 0;
+  unsigned long long h_ctr[3] = {0, 0, 0};
   const auto kernel = A.single ? rect_kernel<false> : rect_kernel<true>;
   if (e == cudaSuccess) e = ensure_smem(kernel, RECT_SMEM_MAX);
   // dreamrect: one point per lane where that is the faster form. With c windows on an SM a round takes about 1 + c/50
@@ -912,6 +920,8 @@ int rect_device(RectBuffers &rb, const double *dRo, int64_t No, double a, double
     lanes = (double)rounds * (1.0 + 0.02 * c) * 11100.0 < (double)No;
   }
   if (lanes && e == cudaSuccess) e = ensure_smem(rect_lane_kernel, RECT_SMEM_MAX);
+  if (lanes && (r = grow(rb.rest, rb.cap_r, (size_t)No * sizeof(int64_t)))) return r;
+  P.rest = reinterpret_cast<int64_t *>(rb.rest);
   // Steps that end with the rows where the lanes this leaves idle cost less than the steps that straddle two rows (and
   // whose equal samples are then no neighbours): 30-element rows of arrays 10.1 against 14.4 ms, 200-element rows of
   // one element 38.0 against 36.4, 8-element rows 0.77 against 0.30 (IEEE root and 64-bit samples in all of these).
@@ -926,19 +936,29 @@ int rect_device(RectBuffers &rb, const double *dRo, int64_t No, double a, double
     }
     P.win = win;
     P.full = full;
-    const unsigned grid = (unsigned)((No + warps - 1) / warps);
+    const size_t smem = (size_t)warps * (win + 32) * sizeof(double);
+    const auto read_counters = [&]() {
+      cudaError_t c = cudaGetLastError();
+      if (c == cudaSuccess) c = cudaMemcpyAsync(h_ctr, rb.ctr, sizeof(h_ctr), cudaMemcpyDeviceToHost, st);
+      return c == cudaSuccess ? cudaStreamSynchronize(st) : c;
+    };
     e = cudaMemsetAsync(rb.ctr, 0, sizeof(h_ctr), st);
-    if (e == cudaSuccess) {
-      if (lanes && !full) {
-        P.win = lane_win;
-        rect_lane_kernel<<<(unsigned)((No + 31) / 32), 32, lane_smem, st>>>(P);
-      } else {
-        kernel<<<grid, warps * 32, (size_t)warps * (win + 32) * sizeof(double), st>>>(P);
+    if (e != cudaSuccess) break;
+    if (lanes && !full) {
+      P.win = lane_win;
+      rect_lane_kernel<<<(unsigned)((No + 31) / 32), 32, lane_smem, st>>>(P);
+      e = read_counters();
+      if (e == cudaSuccess && h_ctr[2] > 0 && !(h_ctr[1] & RECT_MISS)) {
+        P.win = win;
+        P.n_rest = (int64_t)h_ctr[2];
+        kernel<<<(unsigned)((P.n_rest + warps - 1) / warps), warps * 32, smem, st>>>(P);
+        P.n_rest = 0;
+        e = read_counters();
       }
+    } else {
+      kernel<<<(unsigned)((No + warps - 1) / warps), warps * 32, smem, st>>>(P);
+      e = read_counters();
     }
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_ctr, rb.ctr, sizeof(h_ctr), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (!(h_ctr[1] & RECT_MISS)) break;  // every term fell in its point's window
   }
   if (e != cudaSuccess) return set_last_error(DREAM_ERR_CUDA, std::string(fn) + ": " + cudaGetErrorString(e));
