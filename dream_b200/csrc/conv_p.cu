@@ -31,7 +31,12 @@
 //
 // '+=' / '-=' add into existing values; out-of-column terms then contribute
 // the exact neutral element (-0 for +=, +0 for -=), so a stored -0 stays -0
-// exactly as in the reference, which never visits those terms.
+// exactly as in the reference, which never visits those terms. For '=' their
+// products are zeros, which leave a sum that starts from +0 as it is, unless a
+// sample of B is infinite or NaN. That product is NaN, and so is the sum, so a
+// lane whose sums are not all finite forms them again from the terms inside the
+// column. (A test in the trips at a column's ends: 4000 columns of 300 * 300 0.168
+// against 0.084 ms; a vote on B with both forms of a trip 0.089.)
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -88,6 +93,20 @@ __device__ __forceinline__ void conv_trip(double (&acc)[R], double (&X)[conv_p(R
       acc[r] = conv_acc<MODE>(acc[r], prod);
     }
     X[u] = xp[u + CP];
+  }
+}
+
+// Outputs k = k0 .. k0 + R - 1 of a '=' tile from its staged samples, only the terms inside the column; xp: the
+// lane's first A sample. Out of line: the trips lose no registers to it.
+template <int R>
+__device__ __noinline__ void conv_inside(const double *xp, const double *ys, int64_t M, int64_t L, int64_t k0,
+                                         int64_t NY, double *z) {
+  for (int r = 0; r < R && k0 + r < NY; r++) {
+    const int64_t k = k0 + r;
+    const int s0 = (int)std::max<int64_t>(0, L - 1 - k), s1 = (int)std::min<int64_t>(L - 1, M - 1 - k + L - 1);
+    double acc = 0.0;
+    for (int s = s0; s <= s1; s++) acc = __dadd_rn(acc, __dmul_rn(xp[r + s], ys[s]));
+    z[k] = acc;
   }
 }
 
@@ -158,6 +177,12 @@ __global__ void __launch_bounds__(CONV_WARPS * 32) conv_p_kernel(const double *_
       for (int r = 0; r < R; r++) {
         const int64_t k = k_cta + q0 + r;
         if (k < NY) z[k] = acc[r];
+      }
+      if (MODE == 0) {
+        int top = 0;  // high word of the largest |sum|, infinity and NaN above all
+#pragma unroll
+        for (int r = 0; r < R; r++) top = max(top, __double2hiint(acc[r]) & 0x7fffffff);
+        if (top >= 0x7ff00000) conv_inside<R>(xs + q0, ys, M, L, k_cta + q0, NY, z);
       }
     }
   }
