@@ -503,24 +503,26 @@ int launch_fast_plan(dream_das_plan *p, const void *dY, const void *dRo, const v
   const int64_t slow_tiles = (F.n_slow + F.tile_s - 1) / F.tile_s;
   const int64_t chunk = slow_tile_chunk(F, tpp);
   // L2 blocking: A-scans larger than the budget are beamformed in passes over
-  // ranges of inner elements (multiples of 16), each
+  // ranges of inner elements (multiples of 8), each
   // pass adding its terms into the image, so the A-scans of one pass stay in
   // L2 while every image point gathers from them.
   const int n_in = (method == DREAM_DAS_RCA_ROWTX) ? F.Nt : F.Nr;
   if (!apply_shard(p, F)) return 0;  // Y holds the columns of inner elements [shard_lo, shard_hi) only
   const int64_t col_bytes = (int64_t)n_out * p->K * (bf16 ? 2 : 4);  // A-scans of one inner element
   const int64_t y_bytes = col_bytes * n_in;
-  // automatic: even passes of at most 136 MB, a little more than the 126 MB L2,
-  // widths multiples of 16 columns (RCA 128x128, K 4096, 128x128x256 points: FP32
+  // automatic: passes of about 136 MB, a little more than the 126 MB L2 (RCA
+  // 128x128, K 4096, 128x128x256 points: FP32
   // 268 MB in two passes 25.6 ms, in three 26.5, in five 27.5; one pass 25.1, but
   // 3.8 against 3.6 for 64x64x128 points, which lie further apart; BF16 134 MB in
   // one pass 11.6, in two 11.9: a pass sets up its legs again)
   const int64_t budget = p->l2_block > 0 ? p->l2_block : (int64_t(136) << 20);
   int pass_w = n_in;
   if (in_hi == 0 && p->l2_block >= 0 && y_bytes > budget) {
-    const int64_t n_pass = (y_bytes + budget - 1) / budget;
-    pass_w = (int)std::max<int64_t>(16, ((n_in + n_pass - 1) / n_pass + 15) / 16 * 16);
-    pass_w = std::min(pass_w, n_in);
+    // As even as multiples of 8 allow. A caller's budget bounds every pass; the automatic one sets their number, and a
+    // width may round up past it (132 inner elements, 277 MB: two passes 12.4 ms, three 12.7).
+    const int64_t fits = std::max<int64_t>(8, budget / col_bytes / 8 * 8);
+    const int64_t n_pass = p->l2_block > 0 ? (n_in + fits - 1) / fits : (y_bytes + budget - 1) / budget;
+    pass_w = (int)std::min<int64_t>(n_in, ((n_in + n_pass - 1) / n_pass + 7) / 8 * 8);
   }
   const int lo0 = F.in_lo, hi0 = F.in_hi > 0 ? F.in_hi : n_in;
   for (int i0 = lo0; i0 < hi0; i0 += pass_w) {

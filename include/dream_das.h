@@ -257,10 +257,11 @@ int dream_das_set_inner_shard(dream_das_plan *plan, int64_t lo, int64_t hi);
  * L2 blocking of the F32_STORE / BF16_STORE kernels (TFM, RCA; no counterpart
  * in the reference, whose CPU loops have no such cache to fit). A-scans larger
  * than the budget are beamformed in passes over ranges of inner elements (a
- * multiple of 16 each) whose A-scans take at most `bytes`, each pass adding
- * into the image: the pass's samples stay in L2 while every image point
- * gathers from them. 0 = automatic (even passes of at most 136 MB),
- * < 0 = never split. The image changes only by FP32 rounding.
+ * multiple of 8 each, the last one's rest excepted) whose A-scans take at most
+ * `bytes` (or 8 inner elements, where those take more), each pass adding into
+ * the image: the pass's samples stay in L2 while every image point gathers from
+ * them. 0 = automatic (even passes of about 136 MB), < 0 = never
+ * split. The image changes only by FP32 rounding.
  */
 int dream_das_set_l2_block(dream_das_plan *plan, int64_t bytes);
 
