@@ -24,7 +24,8 @@
 // elements' windows sits in shared memory (sized on the host by the
 // diameter of the array and the spread of its delays, up to 8 warps per
 // CTA); longer windows are accumulated in the output column itself. The warp
-// takes 32 consecutive terms of one live element per step: lanes that hit
+// takes 32 consecutive terms of one live element per step (of several, where
+// elements have few: packed_terms): lanes that hit
 // the same sample are grouped (__match_any_sync) and the lowest lane of each
 // group adds the group's amplitudes in lane order (as many shuffle steps as
 // the largest group has members), so every sample receives its terms in the
@@ -308,11 +309,12 @@ __device__ __forceinline__ void term_step(const RectParams &P, const ElemView &V
 
 // The same step for an element that is term_plain, at a surface element whose
 // centre differs by rx from the point in x and by ry2 squared in y; c0 as for
-// rect_number. hits counts the terms added (the others are out of bounds).
+// rect_number. hits counts the terms added (the others are out of bounds; `last`:
+// flagged as such, a term of the array's last element).
 template <bool SKIP>
 __device__ __forceinline__ void plain_step(const RectParams &P, const ElemView &V, double c0, bool valid, double rx,
                                            double ry2, int lane, int w0, int wn, double *h, double *stage,
-                                           unsigned int &hits, unsigned int &flags) {
+                                           unsigned int &hits, unsigned int &flags, bool last = false) {
   double rh;
   const double r = rect_root(__dadd_rn(__dadd_rn(__dmul_rn(rx, rx), ry2), V.rz2), rh);
   double ai = SKIP ? 0.0 : rect_amplitude(P, V.w, r, rh);
@@ -322,6 +324,7 @@ __device__ __forceinline__ void plain_step(const RectParams &P, const ElemView &
   const unsigned int slot = (unsigned int)(it - w0);
   const bool in = valid && slot < (unsigned int)wn;
   hits += in ? 1u : 0u;
+  if (last && valid && !in) flags |= RECT_LAST_OOB;
   if (valid && !in && (unsigned int)it < (unsigned int)P.nt) flags |= RECT_MISS;  // not expected
   if (SKIP) {
     if (!__any_sync(0xffffffffu, in)) return;  // no term of this step lands in the SIR
@@ -376,9 +379,51 @@ __device__ __forceinline__ void element_terms(const RectParams &P, const ElemVie
   }
 }
 
-// ARR = false: dreamrect (one element at the origin, P.M == 1), ARR = true: arrays.
-template <bool ARR>
-__global__ void __launch_bounds__(RECT_WARPS * 32, 4) rect_kernel(const RectParams P) {
+// Terms of the live elements L (bits) among elements m0 .. m0 + 31, 32 consecutive
+// ones per step whatever element they belong to; `plain`: all are term_plain.
+__device__ __forceinline__ void packed_terms(const RectParams &P, int64_t m0, int64_t n, unsigned int L, bool plain,
+                                             int lane, int64_t w0, int64_t w1, double *h, double *stage,
+                                             unsigned long long &oob, unsigned int &flags) {
+  const int E = P.nx * P.ny, total = __popc(L) * E;
+  // this lane's term: its live element (the lowest bit still set in L) and surface element (ix, iy)
+  int iy = lane % E / P.nx, ix = lane % E - iy * P.nx;
+  for (int j = lane / E; j > 0; j--) L &= L - 1u;
+  ElemView V;
+  double c0 = 0.0;
+  bool last = false;
+  auto view = [&]() {  // of the last element where none is left (never added)
+    const int64_t m = L ? m0 + __ffs(L) - 1 : P.M - 1;
+    elem_view(P, m, n, V);
+    c0 = __fma_rn(-V.dl, P.inv_dt, RECT_MAGIC);
+    last = m == P.M - 1;
+  };
+  view();
+  unsigned int hits = 0;
+  for (int g0 = 0;;) {
+    const bool valid = g0 + lane < total;
+    if (plain) {
+      const double rx = __dsub_rn(V.xo, __ldg(P.xs + ix)), ry = __dsub_rn(V.yo, __ldg(P.ys + iy));
+      plain_step<true>(P, V, c0, valid, rx, __dmul_rn(ry, ry), lane, (int)w0, (int)(w1 - w0), h, stage, hits, flags, last);
+    } else {
+      term_step<true>(P, V, valid, ix, iy, lane, w0, w1, h, stage, oob, flags, last);
+    }
+    if ((g0 += 32) >= total) break;
+    bool next = false;
+    for (ix += 32; ix >= P.nx; ix -= P.nx)
+      if (++iy == P.ny) {
+        iy = 0;
+        L &= L - 1u;
+        next = true;
+      }
+    if (next) view();
+  }
+  if (plain) oob += (lane == 0 ? (unsigned long long)total : 0ull) - hits;  // summed over the warp at the end
+}
+
+// ARR = false: dreamrect (one element at the origin, P.M == 1), ARR = true: arrays;
+// PACK: their live elements' terms side by side. MINB: blocks per SM.
+template <bool ARR, bool PACK, int MINB = 4>
+__global__ void __launch_bounds__(RECT_WARPS * 32, MINB) rect_kernel(const RectParams P) {
   extern __shared__ __align__(16) double rect_dyn[];  // [warps][32] staged amplitudes, then [warps][P.win]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double *stage = rect_dyn + warp * 32;
@@ -447,7 +492,13 @@ __global__ void __launch_bounds__(RECT_WARPS * 32, 4) rect_kernel(const RectPara
           if (c0 + lane == P.M - 1) flags |= RECT_LAST_OOB;
         }
       }
-      for (unsigned int L = __ballot_sync(0xffffffffu, live); L; L &= L - 1u) {
+      unsigned int L = __ballot_sync(0xffffffffu, live);
+      if (PACK) {
+        const bool plain = __all_sync(0xffffffffu, !live || term_plain(P, V));
+        if (L) packed_terms(P, c0, n, L, plain, lane, w0, w1, h, stage, oob, flags);
+        continue;
+      }
+      for (; L; L &= L - 1u) {
         const int64_t m = c0 + __ffs(L) - 1;
         elem_view(P, m, n, V);
         element_terms<true>(P, V, lane, w0, w1, h, stage, oob, flags, m == P.M - 1);
@@ -904,7 +955,25 @@ int rect_device(RectBuffers &rb, const double *dRo, int64_t No, double a, double
   P.rest_count = rb.ctr + 2;
   P.n_rest = 0;
   unsigned long long h_ctr[3] = {0, 0, 0};
-  const auto kernel = A.single ? rect_kernel<false> : rect_kernel<true>;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // Steps that end with the rows where the lanes this leaves idle cost less than the steps that straddle two rows (and
+  // whose equal samples are then no neighbours): 30-element rows of arrays 10.1 against 14.4 ms, 200-element rows of
+  // one element 38.0 against 36.4, 8-element rows 0.77 against 0.30 (IEEE root and 64-bit samples in all of these).
+  P.row_steps = nx >= 20 && (nx % 32 == 0 || nx % 32 > 10);
+  // Arrays without such rows: steps that run on from one live element to the next, where a last step of its own would
+  // leave a fifth of an element's lanes idle (441 elements, 60000 points, nt = 400, of 1 surface element each 0.86
+  // against 12.5 ms, of 4 2.0 against 11.0; of 64 they cost 2 % more). They keep a view per lane, which 64 registers
+  // do not hold without spilling: less than a wave of blocks takes 80 (81 elements of 36, 500 points 0.19 ms, 0.23 with
+  // 64, 0.27 by element; of 100 0.34 against 0.42 by element; 60000 points 0.83 with 80, 0.76 with 64).
+  const uint64_t E = (uint64_t)nx * ny;
+  const bool small = (No + RECT_WARPS - 1) / RECT_WARPS <= 4 * (int64_t)sms;
+  const bool pack = !P.row_steps && E <= 1024 && (small || (E + 31) / 32 * 32 * 5 > E * 6);
+  const auto kernel = A.single ? rect_kernel<false, false>
+                      : !pack  ? rect_kernel<true, false>
+                      : small  ? rect_kernel<true, true, 3>
+                               : rect_kernel<true, true>;
   if (e == cudaSuccess) e = ensure_smem(kernel, RECT_SMEM_MAX);
   // dreamrect: one point per lane where that is the faster form. With c windows on an SM a round takes about 1 + c/50
   // times a lone warp's 71 ns per term; one warp per point takes 6.4 ps per term and point (both on the 60000-element
@@ -912,9 +981,6 @@ int rect_device(RectBuffers &rb, const double *dRo, int64_t No, double a, double
   const int64_t lane_win = A.single ? window_bound(el, a, b, dt, cp, nt) : 0, lane_smem = (lane_win + 1) * 32 * 8;
   bool lanes = false;
   if (A.single && nt <= INT32_MAX && lane_smem <= RECT_SMEM_MAX) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t c = std::min<int64_t>(16, (227 * 1024) / (lane_smem + 1024));
     const int64_t rounds = (No + 32 * c * sms - 1) / (32 * c * sms);
     lanes = (double)rounds * (1.0 + 0.02 * c) * 11100.0 < (double)No;
@@ -922,10 +988,6 @@ int rect_device(RectBuffers &rb, const double *dRo, int64_t No, double a, double
   if (lanes && e == cudaSuccess) e = ensure_smem(rect_lane_kernel, RECT_SMEM_MAX);
   if (lanes && (r = grow(rb.rest, rb.cap_r, (size_t)No * sizeof(int64_t)))) return r;
   P.rest = reinterpret_cast<int64_t *>(rb.rest);
-  // Steps that end with the rows where the lanes this leaves idle cost less than the steps that straddle two rows (and
-  // whose equal samples are then no neighbours): 30-element rows of arrays 10.1 against 14.4 ms, 200-element rows of
-  // one element 38.0 against 36.4, 8-element rows 0.77 against 0.30 (IEEE root and 64-bit samples in all of these).
-  P.row_steps = nx >= 20 && (nx % 32 == 0 || nx % 32 > 10);
   for (int full = 0; full < 2 && e == cudaSuccess; full++) {
     int64_t win = full ? 0 : window_bound(el, a, b, dt, cp, nt);
     int warps = RECT_WARPS;
