@@ -413,8 +413,10 @@ __global__ void __launch_bounds__(BD, MINB * 128 / BD) das_plain_tile_kernel(con
   for (int o = 0; o < n_out; o++) {
     const T lo = pt.outer_leg(P, o);
     // Rounded sums and products are monotone, so every time of this outer
-    // element lies between those of the shortest and the longest inner leg.
-    const bool in = fin && A::mul(A::add(lo, mn), P.Fs) >= (T)0 && A::mul(A::add(lo, mx), P.Fs) < P.Kf;
+    // element lies between those of the shortest and the longest inner leg: all in
+    // bounds, all out of bounds, or tested one by one.
+    const T first_p = A::mul(A::add(lo, mn), P.Fs), last_p = A::mul(A::add(lo, mx), P.Fs);
+    const bool in = fin && first_p >= (T)0 && last_p < P.Kf;
     if (!BIGK && !IDX && __all_sync(0xffffffffu, in)) {
       int i = 0;
       for (; i + 2 * U <= n_in; i += 2 * U) {
@@ -429,6 +431,8 @@ __global__ void __launch_bounds__(BD, MINB * 128 / BD) das_plain_tile_kernel(con
         gather(lo, i + U, yb, false);
         accumulate(ya);
       }
+    } else if (!IDX && __all_sync(0xffffffffu, fin && (first_p >= P.Kf || last_p <= (T)-1))) {
+      oob += n_in;
     } else {
       for (int i = 0; i < n_in; i += 2 * U) {
         gather_tested(lo, i, ya);

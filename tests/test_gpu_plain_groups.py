@@ -1,5 +1,7 @@
 """The plain TFM / RCA kernels where terms are tested one by one: inner elements too
-many for the leg table, around the groups of eight. Images equal the oracle's bit for bit, out-of-bounds counts are the oracle's,
+many for the leg table, around the groups of eight; outer elements all of whose
+terms lie past the A-scan's end or before its start beside others that straddle
+them. Images equal the oracle's bit for bit, out-of-bounds counts are the oracle's,
 and so is the index table."""
 import ctypes
 
@@ -53,3 +55,11 @@ def _run(method, n_out, n_in, K, delay, dtype, seed):
 @pytest.mark.parametrize("K,delay", [(200, 0.1), (400, -3.0)])
 def test_without_a_leg_table(n_in, dtype, K, delay):
     _run("tfm", 2, n_in, K, delay, dtype, n_in)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("method", ["tfm", "rca_coltx", "rca_rowtx"])
+@pytest.mark.parametrize("K,delay", [(90, 0.0), (250, 0.0), (300, -12.0), (300, -40.0), (300, 1000.0)])
+def test_elements_out_of_bounds(method, K, delay, dtype):
+    out, all_terms = _run(method, 9, 19 if method == "tfm" else 13, K, delay, dtype, K)  # RCAs: edges inside Gr
+    assert 0 < out < all_terms or abs(delay) >= 40.0
