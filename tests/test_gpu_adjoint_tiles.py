@@ -1,8 +1,9 @@
-"""Tiles of the operator's adjoint on frames whose last tiles are partly filled in
-either direction; points without lines (none found, or one point per line), on
-frames below and above a tile per SM. Whole-number images make the adjoint exact: a
-point taken twice, never or at another's place shows. Points in rows along x have to
-stay within five times the same points in lines (one point per line would fill a
+"""Tiles of the operator's adjoint on frames whose last tiles are partly filled in either direction; points without lines (none
+found, or one point per line), on frames below and above a tile per SM; few outer
+elements. Whole-number images make the adjoint exact: a point taken twice, never or
+at another's place shows. The automatic tile has to keep up with a caller's: within
+one and a half times the better of two fixed tiles, and points in rows along x
+within five times the same points in lines (one point per line would fill a
 sixteenth of a tile's lanes)."""
 import numpy as np
 import pytest
@@ -62,6 +63,21 @@ def _ms(op, x):
         torch.cuda.synchronize()
         best = min(best, e0.elapsed_time(e1))
     return best
+
+
+@pytest.mark.parametrize("n_out,n_in,lines,depth,half,z_hi", [(37, 53, 301, 203, 20.0, 37.0), (2, 801, 48, 64, 15.0, 27.0), (8, 300, 48, 64, 15.0, 27.0)])
+def test_automatic_tile_keeps_up(n_out, n_in, lines, depth, half, z_hi):
+    from dream_b200 import _lib
+    from dream_b200.autograd import DASOperator
+    Gt, Gr = synth.linear_array(n_out, 0.5), synth.linear_array(n_in, 0.5)
+    op = DASOperator(Gt, Gr, synth.grid_xz(lines, depth, (-half, half), (2.0, z_hi)), DT, np.zeros((1, 1)), CP, "tfm", 1777)
+    x = torch.randn(op.No, device="cuda")
+    auto = _ms(op, x)
+    fixed = []
+    for tile in ((8, 32), (16, 16)):
+        _lib.check(_lib.load().dream_das_set_tile(op.plan.handle, *tile))
+        fixed.append(_ms(op, x))
+    assert auto <= 1.5 * min(fixed), (auto, fixed)
 
 
 def test_rows_along_x():
