@@ -352,31 +352,32 @@ int zero_length_ascans(dream_das_plan *p, void *dIm, unsigned long long *doob, c
   return 0;
 }
 
-// Tile of the operator's adjoint: the user's, or on a hinted TFM grid 16 x 16
-// points (64x64 elements, 512x512 points 0.80 ms, 37x53 elements 0.35; 8 x 32
-// points 0.79 and 0.46), on an RCA volume 8 x 16, whose windows grow fastest with
-// the tile (128x128 elements, 128x128x256 points 54.7 ms; in tiles along one row
-// of lines 61.4, 8 x 8 93.9, 16 x 8 81), on both 8 x 8 where that would leave SMs
-// without a tile (64x64 elements, 150x125 points 0.25 against 0.49 ms), or 8 x 16
-// if there are few outer elements, whose terms then cost less than the inner legs
-// (2x801 elements, 48x64 points 0.21 against 0.57 ms, 8x300 0.23 against 0.43, 8x64
-// 0.043 against 0.052). Points
-// without lines (no hint, or one point per line): 256 consecutive ones, or 32
-// where that would leave SMs without a tile (64x9 elements, 65536 points in rows
-// along x 0.11 ms, as lines of one point in 8 x 32 tiles 1.2, 16 x 16 2.5; 33x33,
-// 3072 points 0.056 against 0.165 with 256).
+// Tile of the operator's adjoint: the user's, or on a TFM grid of lines 16 x 16 or
+// 8 x 32 points by their spacing (square_tile), on an RCA volume 8 x 16, whose
+// windows grow fastest with the tile (128x128 elements, 128x128x256 points 54.7
+// ms; in tiles along one row of lines 61.4, 8 x 8 93.9, 16 x 8 81), on both 8 x 8
+// where that would leave SMs without a tile (64x64 elements, 150x125 points 0.25
+// against 0.49 ms), or 8 x 16 if there are few outer elements, whose terms then
+// cost less than the inner legs (2x801 elements, 48x64 points 0.21 against 0.57 ms,
+// 8x300 0.23 against 0.43, 8x64 0.043 against 0.052). Points without lines (no
+// hint, or one point per line): 256 consecutive ones, or 32 where that would leave
+// SMs without a tile (64x9 elements, 65536 points in rows along x 0.11 ms, as lines
+// of one point in 8 x 32 tiles 1.2, 16 x 16 2.5; 33x33, 3072 points 0.056 against
+// 0.165 with 256).
 void scatter_tile(const dream_das_plan *p, FastParams &F) {
   const int n_out = (F.method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt, n_in = (F.method == DREAM_DAS_RCA_ROWTX) ? F.Nt : F.Nr;
   F.wf = p->n_fast > 0 ? 8 : 32;
+  F.square = 0;
   if (p->tile_f > 0) {
     F.tile_f = p->tile_f;
     F.tile_s = p->tile_s;
   } else if (p->n_fast > 1) {
-    F.tile_f = F.method == DREAM_DAS_TFM ? 16 : 8;
-    F.tile_s = 16;
+    F.square = F.method == DREAM_DAS_TFM;
+    F.tile_f = 8;
+    F.tile_s = F.square ? 32 : 16;
     if (p->No < (int64_t)p->sm_count * F.tile_f * F.tile_s) {
-      F.tile_f = 8;
       F.tile_s = n_in >= 16 * n_out ? 16 : 8;
+      F.square = 0;
     }
   } else {
     F.n_fast = p->No;

@@ -336,18 +336,19 @@ struct LegBounds {
   __device__ __forceinline__ double max_leg() const { return __hiloint2double(word(hi), hi < 0 ? 0 : -1); }
 };
 
-// The image point of this thread (inactive lanes repeat the tile's first point);
-// lines in the order of volume_line.
-__device__ __forceinline__ int64_t tile_point(const FastParams &P, int64_t tfi, int64_t tsi, uint32_t row, bool &active) {
+// The image point of this thread (inactive lanes repeat the tile's first point)
+// in tile (tfi, tsi) of tile_f x tile_s points; lines in the order of volume_line.
+__device__ __forceinline__ int64_t tile_point(const FastParams &P, int tile_f, int tile_s, int64_t tfi, int64_t tsi,
+                                              uint32_t row, bool &active) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int lf = lane % P.wf, ls = lane / P.wf;
-  const int warps_f = P.tile_f / P.wf;
+  const int warps_f = tile_f / P.wf;
   const int wfi = warp % warps_f, wsi = warp / warps_f;
-  const int64_t f = tfi * P.tile_f + wfi * P.wf + lf;
-  const int64_t s = tsi * P.tile_s + wsi * (32 / P.wf) + ls;
+  const int64_t f = tfi * tile_f + wfi * P.wf + lf;
+  const int64_t s = tsi * tile_s + wsi * (32 / P.wf) + ls;
   active = f < P.n_fast && s < P.n_slow;
   return active ? volume_line(s, row, P.n_slow) * P.n_fast + f
-                : volume_line(tsi * P.tile_s, row, P.n_slow) * P.n_fast + tfi * P.tile_f;
+                : volume_line(tsi * tile_s, row, P.n_slow) * P.n_fast + tfi * tile_f;
 }
 
 // Whether a block looks for rows of lines: RCAs, which image volumes, with terms
@@ -409,7 +410,7 @@ __device__ __forceinline__ void gather_tile(const FastParams &P, int64_t tfi, in
     if (threadIdx.x == 0) s_row = row;
     __syncthreads();
   }
-  auto point = [&]() { return tile_point(P, tfi, tsi, METHOD != TFM ? *(volatile uint32_t *)&s_row : 0, active); };
+  auto point = [&]() { return tile_point(P, P.tile_f, P.tile_s, tfi, tsi, METHOD != TFM ? *(volatile uint32_t *)&s_row : 0, active); };
   Pixel px;
   pixel_of(P, point(), px);
   // 2^52 + j * K, read from shared memory: as uniform values each use would move them to a register first
@@ -1006,6 +1007,20 @@ __device__ __forceinline__ void scatter_windows(const FastParams &P, const Scatt
   }
 }
 
+// Whether a TFM grid's 256-point tiles are 16 x 16 rather than 8 deep and 32 wide.
+// A leg spans at most the tile's diagonal, and windows beyond their capacity cost
+// two to three times as much: the shorter diagonal, 16 x 16 where lines are further
+// apart than half the spacing in depth. 64x64 elements, 1024 lines 0.03 mm apart of
+// 40 points 0.64 mm apart: 8 x 32 0.30 ms, 16 x 16 0.82; 37x53 elements, 301 lines
+// of 203 points 0.13 and 0.18 mm apart 0.46 and 0.33; 512x512 points 0.79 and 0.82.
+// The first points decide, alike in every block.
+__device__ __forceinline__ bool square_tile(const FastParams &P) {
+  const double *R = P.Ro + (P.n_slow > 1 ? P.n_fast : 0);
+  const double x = R[0] - P.Ro[0], y = R[P.No] - P.Ro[P.No], z = R[2 * P.No] - P.Ro[2 * P.No];
+  const double d = P.Ro[2 * P.No + 1] - P.Ro[2 * P.No];
+  return !(d * d > 4.0 * (x * x + y * y + z * z));
+}
+
 template <bool WEIGHTED, int METHOD>
 __global__ void __launch_bounds__(256, 2) das_scatter_kernel(const FastParams P, const float *__restrict__ X,
                                                              float *__restrict__ Ya) {
@@ -1016,7 +1031,18 @@ __global__ void __launch_bounds__(256, 2) das_scatter_kernel(const FastParams P,
   double *legs = reinterpret_cast<double *>(smem_raw + scatter_head_bytes(n_out, n_in) + SCATTER_WIN_BYTES);
   bool active;
   const uint32_t row = volume_tiles<METHOD>(P) ? volume_row(P.Ro, P.No, P.n_fast, P.n_slow) : 0;
-  const int64_t no = tile_point(P, blockIdx.x, (int64_t)blockIdx.y + P.slow_tile0, row, active);
+  int tile_f = P.tile_f, tile_s = P.tile_s;
+  int64_t tfi = blockIdx.x, tsi = (int64_t)blockIdx.y + P.slow_tile0;
+  if (METHOD == TFM && P.square) {  // a launch row holds 32 lines: the blocks of one row of 8 x 32, or two of 16 x 16
+    if (square_tile(P)) {
+      const int64_t cols = (P.n_fast + 15) / 16, lower = tfi >= cols;
+      tile_f = tile_s = 16;
+      tsi = 2 * tsi + lower;
+      tfi -= lower * cols;
+    }
+    if (tfi * tile_f >= P.n_fast || tsi * tile_s >= P.n_slow) return;
+  }
+  const int64_t no = tile_point(P, tile_f, tile_s, tfi, tsi, row, active);
   Pixel px;
   pixel_of(P, no, px);
   const float xn = active ? __ldg(X + no) : 0.0f;
@@ -1101,7 +1127,7 @@ cudaError_t launch_scatter(const FastParams &P0, const float *X, float *Ya, cuda
 #undef SCATTER_KERNEL
   cudaError_t e = ensure_smem(kern, smem);
   if (e != cudaSuccess) return e;
-  const int64_t gx = (P.n_fast + P.tile_f - 1) / P.tile_f;
+  const int64_t gx = P.square ? (P.n_fast + 15) / 16 * 2 : (P.n_fast + P.tile_f - 1) / P.tile_f;  // square: of either tile
   const int64_t gy = P.slow_tile1 - P.slow_tile0;
   if (gx <= 0 || gy <= 0) return cudaSuccess;
   kern<<<dim3((unsigned)gx, (unsigned)gy), nthr, smem, st>>>(P, X, Ya);

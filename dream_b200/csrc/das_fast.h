@@ -25,6 +25,7 @@ struct FastParams {
   // image tiling: point n = s*n_fast + f
   int64_t n_fast, n_slow;
   int tile_f, tile_s, wf;  // tile extents; warp lanes along the fast axis
+  int square;              // adjoint: 8 x 32-point tiles become 16 x 16 where the grid's spacing asks for it
   int out_block;           // outer elements whose legs are tabled at a time
   int64_t slow_tile0, slow_tile1;  // slow-tile range of this launch
   int64_t no0, no1;                // point range (SAFT launches)

@@ -228,9 +228,10 @@ int dream_das_detect_grid(dream_das_plan *plan, const void *dRo, int64_t *n_fast
  * is a multiple of 8 and tile_s of 4, without one tile_s must be 1).
  * (0, 0) restores the automatic choice. Used by the autotuner. Automatic,
  * on a hinted grid: 8 x 16 points for the gathers; for the operator's adjoint 16 x
- * 16 on TFM frames and 8 x 16 on RCA volumes, or fewer points where that would
- * leave SMs without a tile; 128 consecutive points (the adjoint: 256, or 32 on small frames,
- * on lines of one point too) without a hint.
+ * 16 or 8 x 32 on TFM frames, by the grid's spacing, and 8 x 16 on RCA volumes, or
+ * fewer points where that would leave SMs without a tile; 128 consecutive points
+ * (the adjoint: 256, or 32 on small frames, on lines of one point too) without a
+ * hint.
  */
 int dream_das_set_tile(dream_das_plan *plan, int tile_f, int tile_s);
 int dream_das_get_tile(const dream_das_plan *plan, int *tile_f, int *tile_s);

@@ -1,4 +1,5 @@
-"""Tiles of the operator's adjoint on frames whose last tiles are partly filled in either direction; points without lines (none
+"""Tiles of the operator's adjoint: square or long by the grid's spacing, on frames
+whose last tiles are partly filled in either direction; points without lines (none
 found, or one point per line), on frames below and above a tile per SM; few outer
 elements. Whole-number images make the adjoint exact: a point taken twice, never or
 at another's place shows. The automatic tile has to keep up with a caller's: within
@@ -65,7 +66,8 @@ def _ms(op, x):
     return best
 
 
-@pytest.mark.parametrize("n_out,n_in,lines,depth,half,z_hi", [(37, 53, 301, 203, 20.0, 37.0), (2, 801, 48, 64, 15.0, 27.0), (8, 300, 48, 64, 15.0, 27.0)])
+@pytest.mark.parametrize("n_out,n_in,lines,depth,half,z_hi", [(64, 64, 1024, 40, 15.0, 27.0), (37, 53, 301, 203, 20.0, 37.0),
+                                                              (2, 801, 48, 64, 15.0, 27.0), (8, 300, 48, 64, 15.0, 27.0)])
 def test_automatic_tile_keeps_up(n_out, n_in, lines, depth, half, z_hi):
     from dream_b200 import _lib
     from dream_b200.autograd import DASOperator
