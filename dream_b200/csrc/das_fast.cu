@@ -751,17 +751,19 @@ struct ScatterTile {
   bool low;                  // some term may lie before sample 0
   bool in_bounds;            // every term of the tile is in bounds
   int ext_outer, ext_inner;  // largest extents
-  float x_max;               // largest |x|, NaN above all
+  float x_max, w_max;        // largest |x| and |weight|, NaN above all
   bool x_scales;             // the windows' fixed-point scale of x_max and its inverse are normal FP32 numbers
 };
 
-// Leg bounds and value range of the tile; `scratch`: (blockDim.x / 32) * 8 doubles and as many ints.
-__device__ __forceinline__ void scatter_setup(const FastParams &P, const Pixel &px, float xn, unsigned char *smem,
+// Leg bounds and value range of the tile; `scratch`: (blockDim.x / 32) * 8 doubles and 9 ints.
+template <bool WEIGHTED>
+__device__ __forceinline__ void scatter_setup(const FastParams &P, const Pixel &px, float xn, int w_mx, unsigned char *smem,
                                               double *scratch, int n_out, int n_in, int i_lo, int i_hi, ScatterTile &T) {
   const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
   T.be = reinterpret_cast<int2 *>(smem);
   double *red = scratch;
   int *stat = reinterpret_cast<int *>(red + nwarps * 8);
+  constexpr int STAT = WEIGHTED ? 9 : 8;
   {
     double mn[4] = {px.xo, px.yo, px.zo, px.delay_ms}, mx[4] = {px.xo, px.yo, px.zo, px.delay_ms};
 #pragma unroll
@@ -825,13 +827,15 @@ __device__ __forceinline__ void scatter_setup(const FastParams &P, const Pixel &
   loB = __reduce_min_sync(0xffffffffu, loB);
   hiB = __reduce_max_sync(0xffffffffu, hiB);
   int x_mx = __reduce_max_sync(0xffffffffu, __float_as_int(fabsf(xn)));  // bits: in the values' order, NaN above all
+  if (WEIGHTED) w_mx = __reduce_max_sync(0xffffffffu, w_mx);
   if (lane == 0) {
-    int *s = stat + warp * 8;
+    int *s = stat + warp * STAT;
     s[0] = bad, s[1] = extA, s[2] = extB, s[3] = loA, s[4] = hiA, s[5] = loB, s[6] = hiB, s[7] = x_mx;
+    if (WEIGHTED) s[8] = w_mx;
   }
   __syncthreads();
   for (int w = 0; w < nwarps; w++) {
-    const int *s = stat + w * 8;
+    const int *s = stat + w * STAT;
     bad |= s[0];
     extA = max(extA, s[1]);
     extB = max(extB, s[2]);
@@ -840,6 +844,7 @@ __device__ __forceinline__ void scatter_setup(const FastParams &P, const Pixel &
     loB = min(loB, s[5]);
     hiB = max(hiB, s[6]);
     x_mx = max(x_mx, s[7]);
+    if (WEIGHTED) w_mx = max(w_mx, s[8]);
   }
   __syncthreads();  // the scratch is read
   T.usable = !bad && loA <= hiA && loB <= hiB;
@@ -848,6 +853,7 @@ __device__ __forceinline__ void scatter_setup(const FastParams &P, const Pixel &
   T.ext_outer = extA;
   T.ext_inner = extB;
   T.x_max = __int_as_float(x_mx);
+  T.w_max = __int_as_float(w_mx);
   T.x_scales = T.x_max >= SCATTER_X_MIN && T.x_max < INFINITY;
 }
 
@@ -878,29 +884,20 @@ __device__ __forceinline__ void scatter_windows(const FastParams &P, const Scatt
   const Legs<METHOD, true> outer(P);
   const Legs<METHOD, false> inner(P);
   const double Fs = P.Fs, Kf = (double)K;
-  const int64_t ostride = P.ycol_o > 0 ? P.ycol_o : n_in;  // columns per outer element
   bool vectors = (K & 3) == 0 && (reinterpret_cast<uintptr_t>(Ya) & 15) == 0;  // rows start on 16 bytes
   double *tab = legs + tid;  // leg of outer element o0 + o: tab[o * nthr]
-  uint32_t w_mx = 0;  // bits of the largest |weight|, NaN above all
-  if (WEIGHTED) {
-#pragma unroll 8
-    for (int64_t c = tid; c < n_out * ostride; c += nthr) w_mx = max(w_mx, __float_as_uint(__ldg(P.w + c)) & 0x7fffffffu);
-    w_mx = __reduce_max_sync(0xffffffffu, w_mx);
-  }
-  __shared__ uint32_t s_w[8];
-  if ((tid & 31) == 0) s_w[tid >> 5] = w_mx;
   for (int e = tid; e < 2 * ROWS * WS; e += nthr) win[e] = 0;
   __syncthreads();
-  for (int w = 0; w < (nthr >> 5); w++) w_mx = max(w_mx, s_w[w]);
   // fixed-point scale of the tile: max |x| < 2^E, values scaled by 2^(22 - E)
   int E;
   frexpf(T.x_max, &E);
   const float qscale = ldexpf(1.0f, 22 - E), iS = ldexpf(1.0f, E - 22);
   const int xn = __float2int_rn(xn_f * qscale);
   // A row flushed in vectors adds 0 * (scale * weight) to its cells without a term: only where that is 0.
-  if (WEIGHTED) vectors = vectors && isfinite(iS * __uint_as_float(w_mx));
+  if (WEIGHTED) vectors = vectors && isfinite(iS * T.w_max);
   // flush: a fixed group of nthr / ROWS threads per window row (q, j)
   const int tpr = nthr / ROWS, fr = tid / tpr, fq = tid - fr * tpr, fro = fr / JC, fri = fr % JC;
+  const int64_t ostride = P.ycol_o > 0 ? P.ycol_o : n_in;  // columns per outer element
   const int64_t ystep = SCATTER_NO * ostride * K;
   const uint32_t win_a = (uint32_t)__cvta_generic_to_shared(win);
   uint32_t buf = 0;  // byte offset of the batch's buffer
@@ -1029,6 +1026,12 @@ __global__ void __launch_bounds__(256, 2) das_scatter_kernel(const FastParams P,
   const int i_lo = P.in_lo, i_hi = P.in_hi > 0 ? P.in_hi : n_in;
   int *win = reinterpret_cast<int *>(smem_raw + scatter_head_bytes(n_out, n_in));
   double *legs = reinterpret_cast<double *>(smem_raw + scatter_head_bytes(n_out, n_in) + SCATTER_WIN_BYTES);
+  int w_mx = 0;  // bits of the largest |weight| that this thread reads; here, beside the reads that place the tile
+  if (WEIGHTED) {
+    const int64_t columns = n_out * (int64_t)(P.ycol_o > 0 ? P.ycol_o : n_in);
+#pragma unroll 8
+    for (int64_t c = threadIdx.x; c < columns; c += blockDim.x) w_mx = max(w_mx, __float_as_int(fabsf(__ldg(P.w + c))));
+  }
   bool active;
   const uint32_t row = volume_tiles<METHOD>(P) ? volume_row(P.Ro, P.No, P.n_fast, P.n_slow) : 0;
   int tile_f = P.tile_f, tile_s = P.tile_s;
@@ -1047,7 +1050,7 @@ __global__ void __launch_bounds__(256, 2) das_scatter_kernel(const FastParams P,
   pixel_of(P, no, px);
   const float xn = active ? __ldg(X + no) : 0.0f;
   ScatterTile T;
-  scatter_setup(P, px, xn, smem_raw, reinterpret_cast<double *>(win), n_out, n_in, i_lo, i_hi, T);
+  scatter_setup<WEIGHTED>(P, px, xn, w_mx, smem_raw, reinterpret_cast<double *>(win), n_out, n_in, i_lo, i_hi, T);
   if (T.usable && T.ext_outer + T.ext_inner + 7 <= SCATTER_WCAP && (T.x_max == 0.0f || T.x_scales)) {
     if (T.x_max > 0.0f)
       scatter_windows<WEIGHTED, METHOD>(P, T, px, active, xn, Ya, win, legs, n_out, n_in, i_lo, i_hi);
