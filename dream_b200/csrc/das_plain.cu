@@ -380,25 +380,37 @@ __global__ void __launch_bounds__(BD, MINB * 128 / BD) das_plain_tile_kernel(con
       if (full || i + u < n_in) y[u] = load_at(P, yb, k[u]);
     }
   };
-  auto gather_tested = [&](T lo, int i, T(&y)[U]) {
-    T li[U];
-    legs(i, li);
+  // the terms of one outer element, tested one by one, G at a time; a group without a
+  // term in bounds for any point of the warp is skipped
+  auto add_tested = [&](T lo) {
+    constexpr int G = 8;
+    for (int i = 0; i < n_in; i += G) {
+      T p[G], y[G];
+      uint32_t in = 0;
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      y[u] = (T)0;
-      if (i + u < n_in) {
-        const T p = A::mul(A::add(lo, li[u]), P.Fs);
-        const bool v = p > (T)-1 && p < P.Kf;
+      for (int u = 0; u < G; u++) {
+        p[u] = A::mul(A::add(lo, tab[(i / V + u / V) * V * BD + tid * V + u % V]), P.Fs);
+        if (i + u < n_in && p[u] > (T)-1 && p[u] < P.Kf) in |= 1u << u;
+      }
+      oob += min(G, n_in - i) - __popc(in);
+      if (!IDX && !__any_sync(0xffffffffu, in)) continue;
+#pragma unroll
+      for (int u = 0; u < G; u++) {
+        const bool v = in >> u & 1;
+        y[u] = (T)0;
         if constexpr (IDX) {
-          if (active) *idx = v ? (int64_t)to_index<T, BIGK>(p) : -1;
-          idx += P.No;
+          if (i + u < n_in) {
+            if (active) *idx = v ? (int64_t)to_index<T, BIGK>(p[u]) : -1;
+            idx += P.No;
+          }
         } else if (v) {
-          const int k = to_index<T, BIGK>(p);
+          const int k = to_index<T, BIGK>(p[u]);
           y[u] = BIGK ? load_y(P, ycol + (int64_t)(i + u) * P.K, k)
                       : load_at(P, ycol + (int64_t)i * P.K, (uint32_t)u * (uint32_t)P.K + (uint32_t)k);
         }
-        oob += v ? 0 : 1;
       }
+#pragma unroll
+      for (int u = 0; u < G; u++) im = A::add(im, y[u]);
     }
   };
   auto accumulate = [&](const T(&y)[U]) {
@@ -434,12 +446,10 @@ __global__ void __launch_bounds__(BD, MINB * 128 / BD) das_plain_tile_kernel(con
     } else if (!IDX && __all_sync(0xffffffffu, fin && (first_p >= P.Kf || last_p <= (T)-1))) {
       oob += n_in;
     } else {
-      for (int i = 0; i < n_in; i += 2 * U) {
-        gather_tested(lo, i, ya);
-        accumulate(yb);
-        gather_tested(lo, i + U, yb);
-        accumulate(ya);
-      }
+      accumulate(yb);
+#pragma unroll
+      for (int u = 0; u < U; u++) yb[u] = (T)0;
+      add_tested(lo);
     }
     ycol += (int64_t)n_in * P.K;
   }
