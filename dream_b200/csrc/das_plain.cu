@@ -316,6 +316,11 @@ __global__ void __launch_bounds__(BD, MINB * 128 / BD) das_plain_tile_kernel(con
   using A = Ar<T>;
   constexpr int U = MINB == 4 ? PLAIN_U / 2 : PLAIN_U;  // 16 FP64 samples, twice, do not fit 128 registers
   constexpr int V = 16 / sizeof(T);  // legs per 16-byte table read
+  // Blocks that a long leg table cuts to one or two warps have too few to hide a test per term: outer elements wholly
+  // out of bounds are skipped, the others tested in a loop of their own (64x300 elements, 200x200 points, FP64, K = 300
+  // 0.82 against 5.10 ms, K = 1500 6.87 against 7.15). Whole blocks keep the pipelined groups: with both forms they are
+  // up to 16 % slower in bounds (RCA 64x64, FP32 0.256 and 0.297 ms).
+  constexpr bool FEW = BD < 128;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *tab = reinterpret_cast<T *>(smem_raw);  // leg i of thread t: tab[(i / V) * V * BD + t * V + i % V]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -380,8 +385,29 @@ __global__ void __launch_bounds__(BD, MINB * 128 / BD) das_plain_tile_kernel(con
       if (full || i + u < n_in) y[u] = load_at(P, yb, k[u]);
     }
   };
-  // the terms of one outer element, tested one by one, G at a time; a group without a
-  // term in bounds for any point of the warp is skipped
+  auto gather_tested = [&](T lo, int i, T(&y)[U]) {
+    T li[U];
+    legs(i, li);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      y[u] = (T)0;
+      if (i + u < n_in) {
+        const T p = A::mul(A::add(lo, li[u]), P.Fs);
+        const bool v = p > (T)-1 && p < P.Kf;
+        if constexpr (IDX) {
+          if (active) *idx = v ? (int64_t)to_index<T, BIGK>(p) : -1;
+          idx += P.No;
+        } else if (v) {
+          const int k = to_index<T, BIGK>(p);
+          y[u] = BIGK ? load_y(P, ycol + (int64_t)(i + u) * P.K, k)
+                      : load_at(P, ycol + (int64_t)i * P.K, (uint32_t)u * (uint32_t)P.K + (uint32_t)k);
+        }
+        oob += v ? 0 : 1;
+      }
+    }
+  };
+  // FEW warps: the terms of one outer element, tested one by one, G at a time; a group
+  // without a term in bounds for any point of the warp is skipped
   auto add_tested = [&](T lo) {
     constexpr int G = 8;
     for (int i = 0; i < n_in; i += G) {
@@ -425,8 +451,7 @@ __global__ void __launch_bounds__(BD, MINB * 128 / BD) das_plain_tile_kernel(con
   for (int o = 0; o < n_out; o++) {
     const T lo = pt.outer_leg(P, o);
     // Rounded sums and products are monotone, so every time of this outer
-    // element lies between those of the shortest and the longest inner leg: all in
-    // bounds, all out of bounds, or tested one by one.
+    // element lies between those of the shortest and the longest inner leg.
     const T first_p = A::mul(A::add(lo, mn), P.Fs), last_p = A::mul(A::add(lo, mx), P.Fs);
     const bool in = fin && first_p >= (T)0 && last_p < P.Kf;
     if (!BIGK && !IDX && __all_sync(0xffffffffu, in)) {
@@ -443,13 +468,20 @@ __global__ void __launch_bounds__(BD, MINB * 128 / BD) das_plain_tile_kernel(con
         gather(lo, i + U, yb, false);
         accumulate(ya);
       }
-    } else if (!IDX && __all_sync(0xffffffffu, fin && (first_p >= P.Kf || last_p <= (T)-1))) {
+    } else if (FEW && !IDX && __all_sync(0xffffffffu, fin && (first_p >= P.Kf || last_p <= (T)-1))) {
       oob += n_in;
-    } else {
+    } else if (FEW) {
       accumulate(yb);
 #pragma unroll
       for (int u = 0; u < U; u++) yb[u] = (T)0;
       add_tested(lo);
+    } else {
+      for (int i = 0; i < n_in; i += 2 * U) {
+        gather_tested(lo, i, ya);
+        accumulate(yb);
+        gather_tested(lo, i + U, yb);
+        accumulate(ya);
+      }
     }
     ycol += (int64_t)n_in * P.K;
   }
