@@ -359,7 +359,8 @@ int zero_length_ascans(dream_das_plan *p, void *dIm, unsigned long long *doob, c
 // where that would leave SMs without a tile (64x64 elements, 150x125 points 0.25
 // against 0.49 ms), or 8 x 16 if there are few outer elements, whose terms then
 // cost less than the inner legs (2x801 elements, 48x64 points 0.21 against 0.57 ms,
-// 8x300 0.23 against 0.43, 8x64 0.043 against 0.052). Points without lines (no
+// 8x300 0.23 against 0.43; 32x32 on 100x100 points 0.097 against 0.085 with 8 x 8).
+// Points without lines (no
 // hint, or one point per line): 256 consecutive ones, or 32 where that would leave
 // SMs without a tile (64x9 elements, 65536 points in rows along x 0.11 ms, as lines
 // of one point in 8 x 32 tiles 1.2, 16 x 16 2.5; 33x33, 3072 points 0.056 against
@@ -528,7 +529,8 @@ int launch_fast_plan(dream_das_plan *p, const void *dY, const void *dRo, const v
   // 128x128, K 4096, 128x128x256 points: FP32
   // 268 MB in two passes 25.6 ms, in three 26.5, in five 27.5; one pass 25.1, but
   // 3.8 against 3.6 for 64x64x128 points, which lie further apart; BF16 134 MB in
-  // one pass 11.6, in two 11.9: a pass sets up its legs again)
+  // one pass 26.1, in two 26.9: a pass sets up its legs again; FP32 143 - 398 MB
+  // on 96x96x200 points 6.6 - 18.0 ms, without a jump where a pass is added)
   const int64_t budget = p->l2_block > 0 ? p->l2_block : (int64_t(136) << 20);
   int pass_w = n_in;
   if (in_hi == 0 && p->l2_block >= 0 && y_bytes > budget) {

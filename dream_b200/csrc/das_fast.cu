@@ -216,11 +216,11 @@ __device__ __forceinline__ void leg_range(const FastParams &P, const TileBox &B,
 // the shortest and the longest legs decide exactly whether every term of the
 // chunk is in bounds.
 //
-// Bound (64x64 elements, K = 3000, 512x512 points, FP32 storage): 0.42 ms at 10
-// instructions per term and 0.71 of the issue slots; 6.5 of them are the three
+// Bound (64x64 elements, K = 3000, 512x512 points, FP32 storage): 0.42 ms at 9.3
+// instructions per 32 terms and 0.67 of the issue slots; 6.5 of them are the three
 // FP64 operations, the 64-bit address, the load and half a packed add, about 2.5
-// the legs. The FP64 pipe is at 0.54 (its own limit for the terms alone would be
-// 0.17 ms), the L1 data pipe at 0.46. Fixed-point legs with an ambiguity test
+// the legs. The FP64 pipe is at 0.52 (its own limit for the terms alone would be
+// 0.17 ms), the L1 data pipe at 0.43. Fixed-point legs with an ambiguity test
 // and an FP64 fallback, the form this replaces, took 0.505 ms there, 0.069
 // against 0.037 for 32x32 elements and 256x256 points (no per-tile set-up with
 // block barriers here), 38.0 against 25.6 for the 128x128-element RCA volume.
@@ -697,14 +697,14 @@ cudaError_t convert_f32_to_bf16(const float *x, void *y, int64_t n, cudaStream_t
 // buffers alternate, so one block barrier per batch suffices (between its adds
 // and its flush).
 //
-// Bound: instruction issue (0.54 of the slots; 13.7 instructions per 32 terms, of
+// Bound: instruction issue (0.59 of the slots; 15.5 instructions per 32 terms, of
 // which the index chain, the cell's address and the shared addition are 5, the
 // legs of two blocks of outer elements about 2) and the shared-memory / L1 data
-// pipe (0.73: a warp's additions to one cell take a wavefront each, 2.7 per
+// pipe (0.72: a warp's additions to one cell take a wavefront each, 2.7 per
 // instruction with 8 x 4 points per warp). 64x64 elements, K = 3000, 512x512
-// points: 0.80 ms, weighted 0.89; with fixed-point legs, an ambiguity test and
-// batches of one outer x 16 inner elements 0.83 and 0.99 (37x53 elements 0.35
-// against 0.48, 32x32 and 256x256 points 0.077 against 0.098). The adds carry no
+// points: 0.82 ms, weighted 0.85; with fixed-point legs, an ambiguity test and
+// batches of one outer x 16 inner elements 0.83 and 0.99 (37x53 elements 0.33
+// against 0.55, 32x32 and 256x256 points 0.077 against 0.085). The adds carry no
 // guard and the flush no test for zeros: either costs a branch per term (1.2 and
 // 0.97 ms).
 // ===========================================================================

@@ -296,7 +296,7 @@ struct ColStep<float> {
 // ms in FP64 and 0.98 in FP32). FP64: 0.69 ms, 0.77 of the shared-memory / L1
 // data pipe (2 wavefronts per term for the leg, 2.3 for the 8-byte sample),
 // the FP64 pipe (two-leg add, scale, truncation, accumulate) at 0.42. FP32:
-// 0.36 ms, 8.6 instructions per term, 0.73 of the issue slots. What got it there:
+// 0.36 ms, 8.6 instructions per 32 terms, 0.74 of the issue slots. What got it there:
 //  - no test per term. The shortest and the longest inner leg bound every time
 //    of an outer element exactly (rounded sums and products are monotone), so
 //    one vote per outer element shows that all its terms are in bounds.
@@ -316,11 +316,11 @@ __global__ void __launch_bounds__(BD, MINB * 128 / BD) das_plain_tile_kernel(con
   using A = Ar<T>;
   constexpr int U = MINB == 4 ? PLAIN_U / 2 : PLAIN_U;  // 16 FP64 samples, twice, do not fit 128 registers
   constexpr int V = 16 / sizeof(T);  // legs per 16-byte table read
-  // Blocks that a long leg table cuts to one or two warps have too few to hide a test per term: outer elements wholly
+  // Blocks that a long leg table cuts to one warp have too few to hide a test per term: outer elements wholly
   // out of bounds are skipped, the others tested in a loop of their own (64x300 elements, 200x200 points, FP64, K = 300
-  // 0.82 against 5.10 ms, K = 1500 6.87 against 7.15). Whole blocks keep the pipelined groups: with both forms they are
+  // 0.82 against 5.10 ms, K = 1500 6.87 against 7.15). Larger blocks keep the pipelined groups: with both forms they are
   // up to 16 % slower in bounds (RCA 64x64, FP32 0.256 and 0.297 ms).
-  constexpr bool FEW = BD < 128;
+  constexpr bool FEW = BD == 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *tab = reinterpret_cast<T *>(smem_raw);  // leg i of thread t: tab[(i / V) * V * BD + t * V + i % V]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

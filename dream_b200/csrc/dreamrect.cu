@@ -152,7 +152,8 @@ __device__ __forceinline__ bool elem_window(const RectParams &P, const ElemView 
 // residual (P. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", 1990; "IA-64 and Elementary Functions", 2000). They
 // differed from the IEEE operations in none of 1.2e10 samples, half of them next
-// to rounding boundaries. term_plain tells where they hold.
+// to rounding boundaries; the tests repeat 4.9e6 such samples through SIRs of a
+// single amplitude. term_plain tells where they hold.
 // ---------------------------------------------------------------------------
 
 constexpr int RECT_FB = 14;                          // fraction bits of the sample number in the low mantissa word
@@ -263,7 +264,7 @@ __device__ __forceinline__ void ordered_adds(bool in, Key key, double ai, double
 // every group is a run of consecutive lanes (the common case: along a row
 // the sample index changes monotonically on either side of the point's
 // projection) the leaders read their run from the warp's 32 staged
-// amplitudes, four per trip; otherwise they walk their member masks.
+// amplitudes, eight per trip; otherwise they walk their member masks.
 // SKIP: steps with no term in the SIR skip the amplitudes and the sums (arrays,
 // whose live elements still place most terms outside short windows); without
 // it the amplitude divisions overlap the index computation.
