@@ -364,21 +364,21 @@ int zero_length_ascans(dream_das_plan *p, void *dIm, unsigned long long *doob, c
 // hint, or one point per line): 256 consecutive ones, or 32 where that would leave
 // SMs without a tile (64x9 elements, 65536 points in rows along x 0.11 ms, as lines
 // of one point in 8 x 32 tiles 1.2, 16 x 16 2.5; 33x33, 3072 points 0.056 against
-// 0.165 with 256).
-void scatter_tile(const dream_das_plan *p, FastParams &F) {
+// 0.165 with 256). Returns whether 8 x 32 tiles may become 16 x 16.
+bool scatter_tile(const dream_das_plan *p, FastParams &F) {
   const int n_out = (F.method == DREAM_DAS_RCA_ROWTX) ? F.Nr : F.Nt, n_in = (F.method == DREAM_DAS_RCA_ROWTX) ? F.Nt : F.Nr;
   F.wf = p->n_fast > 0 ? 8 : 32;
-  F.square = 0;
+  bool square = false;
   if (p->tile_f > 0) {
     F.tile_f = p->tile_f;
     F.tile_s = p->tile_s;
   } else if (p->n_fast > 1) {
-    F.square = F.method == DREAM_DAS_TFM;
+    square = F.method == DREAM_DAS_TFM;
     F.tile_f = 8;
-    F.tile_s = F.square ? 32 : 16;
+    F.tile_s = square ? 32 : 16;
     if (p->No < (int64_t)p->sm_count * F.tile_f * F.tile_s) {
       F.tile_s = n_in >= 16 * n_out ? 16 : 8;
-      F.square = 0;
+      square = false;
     }
   } else {
     F.n_fast = p->No;
@@ -387,6 +387,7 @@ void scatter_tile(const dream_das_plan *p, FastParams &F) {
     F.tile_s = 1;
     F.wf = 32;
   }
+  return square;
 }
 
 // Tile of the gathers: the user's, or 128 points, 8 x 16 on a hinted grid (64 and
@@ -843,14 +844,14 @@ static int op_scatter(dream_das_plan *p, const float *X, const float *dW, float 
   F.w = dW;
   int r = grid_params(p, F);
   if (r) return r;
-  scatter_tile(p, F);
+  const bool square = scatter_tile(p, F);
   if (!apply_shard(p, F)) return 0;
   const int64_t slow_tiles = (F.n_slow + F.tile_s - 1) / F.tile_s;
   const int64_t chunk = slow_tile_chunk(F, terms_per_pixel(p));
   for (int64_t t0 = 0; t0 < slow_tiles; t0 += chunk) {
     F.slow_tile0 = t0;
     F.slow_tile1 = std::min(slow_tiles, t0 + chunk);
-    CU(launch_scatter(F, X, Ya, st));
+    CU(launch_scatter(F, square, X, Ya, st));
     p->launches++;
   }
   return 0;

@@ -337,18 +337,20 @@ struct LegBounds {
 };
 
 // The image point of this thread (inactive lanes repeat the tile's first point)
-// in tile (tfi, tsi) of tile_f x tile_s points; lines in the order of volume_line.
-__device__ __forceinline__ int64_t tile_point(const FastParams &P, int tile_f, int tile_s, int64_t tfi, int64_t tsi,
-                                              uint32_t row, bool &active) {
+// in tile (tfi, tsi) of T.tile_f x T.tile_s points (P's own, for the gathers); lines
+// in the order of volume_line.
+template <class Tile>
+__device__ __forceinline__ int64_t tile_point(const FastParams &P, const Tile &T, int64_t tfi, int64_t tsi, uint32_t row,
+                                              bool &active) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int lf = lane % P.wf, ls = lane / P.wf;
-  const int warps_f = tile_f / P.wf;
+  const int warps_f = T.tile_f / P.wf;
   const int wfi = warp % warps_f, wsi = warp / warps_f;
-  const int64_t f = tfi * tile_f + wfi * P.wf + lf;
-  const int64_t s = tsi * tile_s + wsi * (32 / P.wf) + ls;
+  const int64_t f = tfi * T.tile_f + wfi * P.wf + lf;
+  const int64_t s = tsi * T.tile_s + wsi * (32 / P.wf) + ls;
   active = f < P.n_fast && s < P.n_slow;
   return active ? volume_line(s, row, P.n_slow) * P.n_fast + f
-                : volume_line(tsi * tile_s, row, P.n_slow) * P.n_fast + tfi * tile_f;
+                : volume_line(tsi * T.tile_s, row, P.n_slow) * P.n_fast + tfi * T.tile_f;
 }
 
 // Whether a block looks for rows of lines: RCAs, which image volumes, with terms
@@ -410,7 +412,7 @@ __device__ __forceinline__ void gather_tile(const FastParams &P, int64_t tfi, in
     if (threadIdx.x == 0) s_row = row;
     __syncthreads();
   }
-  auto point = [&]() { return tile_point(P, P.tile_f, P.tile_s, tfi, tsi, METHOD != TFM ? *(volatile uint32_t *)&s_row : 0, active); };
+  auto point = [&]() { return tile_point(P, P, tfi, tsi, METHOD != TFM ? *(volatile uint32_t *)&s_row : 0, active); };
   Pixel px;
   pixel_of(P, point(), px);
   // 2^52 + j * K, read from shared memory: as uniform values each use would move them to a register first
@@ -1004,6 +1006,10 @@ __device__ __forceinline__ void scatter_windows(const FastParams &P, const Scatt
   }
 }
 
+struct TileShape {
+  int tile_f, tile_s;
+};
+
 // Whether a TFM grid's 256-point tiles are 16 x 16 rather than 8 deep and 32 wide.
 // A leg spans at most the tile's diagonal, and windows beyond their capacity cost
 // two to three times as much: the shorter diagonal, 16 x 16 where lines are further
@@ -1019,8 +1025,8 @@ __device__ __forceinline__ bool square_tile(const FastParams &P) {
 }
 
 template <bool WEIGHTED, int METHOD>
-__global__ void __launch_bounds__(256, 2) das_scatter_kernel(const FastParams P, const float *__restrict__ X,
-                                                             float *__restrict__ Ya) {
+__global__ void __launch_bounds__(256, 2) das_scatter_kernel(const FastParams P, bool square,
+                                                             const float *__restrict__ X, float *__restrict__ Ya) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int n_out = METHOD == RCA_ROWTX ? P.Nr : P.Nt, n_in = METHOD == RCA_ROWTX ? P.Nt : P.Nr;
   const int i_lo = P.in_lo, i_hi = P.in_hi > 0 ? P.in_hi : n_in;
@@ -1034,18 +1040,18 @@ __global__ void __launch_bounds__(256, 2) das_scatter_kernel(const FastParams P,
   }
   bool active;
   const uint32_t row = volume_tiles<METHOD>(P) ? volume_row(P.Ro, P.No, P.n_fast, P.n_slow) : 0;
-  int tile_f = P.tile_f, tile_s = P.tile_s;
+  TileShape tile = {P.tile_f, P.tile_s};
   int64_t tfi = blockIdx.x, tsi = (int64_t)blockIdx.y + P.slow_tile0;
-  if (METHOD == TFM && P.square) {  // a launch row holds 32 lines: the blocks of one row of 8 x 32, or two of 16 x 16
+  if (METHOD == TFM && square) {  // a launch row holds 32 lines: the blocks of one row of 8 x 32, or two of 16 x 16
     if (square_tile(P)) {
       const int64_t cols = (P.n_fast + 15) / 16, lower = tfi >= cols;
-      tile_f = tile_s = 16;
+      tile.tile_f = tile.tile_s = 16;
       tsi = 2 * tsi + lower;
       tfi -= lower * cols;
     }
-    if (tfi * tile_f >= P.n_fast || tsi * tile_s >= P.n_slow) return;
+    if (tfi * tile.tile_f >= P.n_fast || tsi * tile.tile_s >= P.n_slow) return;
   }
-  const int64_t no = tile_point(P, tile_f, tile_s, tfi, tsi, row, active);
+  const int64_t no = tile_point(P, tile, tfi, tsi, row, active);
   Pixel px;
   pixel_of(P, no, px);
   const float xn = active ? __ldg(X + no) : 0.0f;
@@ -1111,7 +1117,7 @@ __global__ void __launch_bounds__(256, 2) das_scatter_kernel(const FastParams P,
 }  // namespace
 
 // Tile scatter over the slow-tile range of P (P.w optional). Ya is not zeroed here.
-cudaError_t launch_scatter(const FastParams &P0, const float *X, float *Ya, cudaStream_t st) {
+cudaError_t launch_scatter(const FastParams &P0, bool square, const float *X, float *Ya, cudaStream_t st) {
   FastParams P = P0;
   const int nthr = P.tile_f * P.tile_s;
   const int n_out = P.method == RCA_ROWTX ? P.Nr : P.Nt, n_in = P.method == RCA_ROWTX ? P.Nt : P.Nr;
@@ -1130,10 +1136,10 @@ cudaError_t launch_scatter(const FastParams &P0, const float *X, float *Ya, cuda
 #undef SCATTER_KERNEL
   cudaError_t e = ensure_smem(kern, smem);
   if (e != cudaSuccess) return e;
-  const int64_t gx = P.square ? (P.n_fast + 15) / 16 * 2 : (P.n_fast + P.tile_f - 1) / P.tile_f;  // square: of either tile
+  const int64_t gx = square ? (P.n_fast + 15) / 16 * 2 : (P.n_fast + P.tile_f - 1) / P.tile_f;  // square: of either tile
   const int64_t gy = P.slow_tile1 - P.slow_tile0;
   if (gx <= 0 || gy <= 0) return cudaSuccess;
-  kern<<<dim3((unsigned)gx, (unsigned)gy), nthr, smem, st>>>(P, X, Ya);
+  kern<<<dim3((unsigned)gx, (unsigned)gy), nthr, smem, st>>>(P, square, X, Ya);
   return cudaGetLastError();
 }
 

@@ -25,7 +25,6 @@ struct FastParams {
   // image tiling: point n = s*n_fast + f
   int64_t n_fast, n_slow;
   int tile_f, tile_s, wf;  // tile extents; warp lanes along the fast axis
-  int square;              // adjoint: 8 x 32-point tiles become 16 x 16 where the grid's spacing asks for it
   int out_block;           // outer elements whose legs are tabled at a time
   int64_t slow_tile0, slow_tile1;  // slow-tile range of this launch
   int64_t no0, no1;                // point range (SAFT launches)
@@ -66,8 +65,9 @@ inline bool too_many_elements(int n_out, int n_in, int nthr) {
 size_t gather_smem_bytes(const FastParams &P, int nthr);  // leg table of the gather (P.out_block)
 cudaError_t launch_fast(const FastParams &P, bool bf16, cudaStream_t st);
 // Adjoint on the forward's tiles: Ya[k(n,c), c] += w[c] * X[n] (FP32 A-scans;
-// P.w may be NULL). Adds into Ya, which the caller zeroes first.
-cudaError_t launch_scatter(const FastParams &P, const float *X, float *Ya, cudaStream_t st);
+// P.w may be NULL). Adds into Ya, which the caller zeroes first. square: 8 x 32-point
+// tiles of a TFM grid become 16 x 16 where its spacing asks for it.
+cudaError_t launch_scatter(const FastParams &P, bool square, const float *X, float *Ya, cudaStream_t st);
 // Per column c of K x ncol arrays: dW[c] = sum_k Y[k,c] * S[k,c] (when Y and dW
 // are given), then S[:, c] *= w[c] (when w is given).
 cudaError_t launch_column_dot_scale(const float *Y, float *S, const float *w, float *dW, int64_t K, int64_t ncol,
