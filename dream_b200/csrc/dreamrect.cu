@@ -430,8 +430,8 @@ __global__ void __launch_bounds__(RECT_WARPS * 32, MINB) rect_kernel(const RectP
   double *stage = rect_dyn + warp * 32;
   double *win_sm = rect_dyn + (blockDim.x >> 5) * 32 + (int64_t)warp * P.win;
   int64_t n = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
-  if (n >= (P.n_rest > 0 ? P.n_rest : P.No)) return;  // whole warps only: no block-wide barrier below
-  if (P.n_rest > 0) n = P.rest[n];
+  if (n >= (!ARR && P.n_rest > 0 ? P.n_rest : P.No)) return;  // whole warps only: no block-wide barrier below
+  if (!ARR && P.n_rest > 0) n = P.rest[n];
   double *out = P.H + n * P.nt;
   ElemView V;
   // union of the live elements' windows
