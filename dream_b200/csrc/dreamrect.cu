@@ -152,7 +152,7 @@ __device__ __forceinline__ bool elem_window(const RectParams &P, const ElemView 
 // residual (P. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", 1990; "IA-64 and Elementary Functions", 2000). They
 // differed from the IEEE operations in none of 1.2e10 samples, half of them next
-// to rounding boundaries; the tests repeat 4.9e6 such samples through SIRs of a
+// to rounding boundaries; the tests repeat 2.4e6 of them through SIRs of a
 // single amplitude. term_plain tells where they hold.
 // ---------------------------------------------------------------------------
 
